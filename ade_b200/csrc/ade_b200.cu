@@ -8,6 +8,7 @@
 #include "compress.cuh"
 #include "decode_ops.cuh"
 #include "factored.cuh"
+#include "linear_tc.cuh"
 #include "recon.cuh"
 #include "recon_strip.cuh"
 
@@ -79,6 +80,7 @@ int device_info(const DeviceInfo** out) {
             if (!cuda_ok(cudaFuncSetAttribute(ade::compress_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               static_cast<int>(ade::compress_smem_bytes(ade::CQ_MAX_RANK, true)))))
                 return ADE_ERR_CUDA;
+            if (!cuda_ok(cudaFuncSetAttribute(ade::linear_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) return ADE_ERR_CUDA;
             if (!optin_factored<1>() || !optin_factored<2>() || !optin_factored<4>() || !optin_factored<8>() ||
                 !optin_factored<16>())
                 return ADE_ERR_CUDA;
@@ -174,8 +176,8 @@ void set_row_split(ade::FactoredParams& p, int grid) {
 // The factored kernel's CTAs wait for one another (grid-wide counters), so the whole grid has to be resident at
 // once.  A cooperative launch makes the driver guarantee that: the grid starts only when every CTA has an SM, also
 // when other kernels occupy part of the device, and a grid that can never fit is refused at launch.
-template <class Kernel>
-int launch_grid(Kernel kernel, int grid, int threads, size_t smem, cudaStream_t st, const ade::FactoredParams& p) {
+template <class Kernel, class... Args>
+int launch_grid(Kernel kernel, int grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(grid));
     cfg.blockDim = dim3(static_cast<unsigned>(threads));
@@ -186,7 +188,7 @@ int launch_grid(Kernel kernel, int grid, int threads, size_t smem, cudaStream_t 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_cooperative ? 1 : 0;
-    return cuda_ok(cudaLaunchKernelEx(&cfg, kernel, p)) ? ADE_OK : ADE_ERR_CUDA;
+    return cuda_ok(cudaLaunchKernelEx(&cfg, kernel, args...)) ? ADE_OK : ADE_ERR_CUDA;
 }
 
 // Launch of one of the small decode-step kernels.
@@ -254,7 +256,8 @@ bool optin_factored() {
 }
 
 // block-diagonal hint of the delta -> kernel parameters (validated: ascending, covering [0, M) x [0, ng))
-int set_blocks(ade::FactoredParams& p, const ade_delta_t* d) {
+template <class Params>
+int set_blocks(Params& p, const ade_delta_t* d) {
     p.n_blocks = 0;
     if (d->n_blocks == 0) return ADE_OK;
     if (d->n_blocks < 0 || d->n_blocks > ADE_B200_MAX_BLOCKS) return ADE_ERR_SHAPE;
@@ -403,6 +406,76 @@ int ade_b200_factored(const ade_delta_t* d, const void* x, const void* y_dense, 
     if (T <= 32) return launch_factored<4>(p, grid, st);
     if (T <= 64) return launch_factored<8>(p, grid, st);
     return launch_factored<16>(p, grid, st);
+}
+
+size_t ade_b200_linear_workspace_bytes(int T, int M, int r) {
+    const DeviceInfo* di = nullptr;
+    if (T < 1 || M < 1 || r < 1 || device_info(&di)) return 0;
+    return ade::linear_workspace_bytes(T, di->sms);
+}
+
+int ade_b200_linear(const ade_delta_t* d, const void* x, const void* w_b, void* out, void* scratch, size_t scratch_bytes,
+                    void* workspace, size_t workspace_bytes, int T, void* stream) {
+    int rc = check_delta(d);
+    if (rc) return rc;
+    if (!d->vt || !x || !w_b || !out || !scratch || !workspace) return ADE_ERR_NULL;
+    if (T < 1 || T > ADE_B200_MAX_TOKENS) return ADE_ERR_SHAPE;
+    if (!aligned16(d->vt) || !aligned16(x) || !aligned16(w_b) || !aligned16(out) || !aligned16(scratch) || !aligned16(workspace))
+        return ADE_ERR_ALIGN;
+    if (scratch_bytes < factored_scratch_min(T, d->r)) return ADE_ERR_SCRATCH;
+    const DeviceInfo* di = nullptr;
+    rc = device_info(&di);
+    if (rc) return rc;
+    const int grid = di->sms;                                   // one persistent CTA per SM, all co-resident
+    if (workspace_bytes < ade::linear_workspace_bytes(T, grid)) return ADE_ERR_SCRATCH;
+    ade::LinearParams p = {};
+    p.tpad = (T + 15) / 16 * 16;
+    ade::LinearSplit split;
+    if (!ade::linear_split(d->M, d->N, T, p.tpad, grid, split)) return ADE_ERR_SHAPE;
+    p.slices = split.slices;
+    p.segs = split.segs;
+    p.ksplit = split.ksplit;
+    p.rows = split.rows;
+    p.stages = split.stages;
+    p.ring_bytes = split.ring_bytes;
+    p.uq = d->uq;
+    p.vt = d->vt;
+    p.us = d->us;
+    p.uz = d->uz;
+    p.vs = d->vs;
+    p.vz = d->vz;
+    p.h = static_cast<__nv_bfloat16*>(scratch);
+    p.sync = reinterpret_cast<unsigned int*>(static_cast<char*>(scratch) + ade_b200_factored_sync_offset(T, d->r));
+    p.status = p.sync + 2;
+    p.part = static_cast<float*>(workspace);
+    p.slice_count = reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + ade::linear_part_bytes(T, grid));
+    p.out = static_cast<__nv_bfloat16*>(out);
+    p.T = T;
+    p.M = d->M;
+    p.N = d->N;
+    p.r = d->r;
+    const int ng = d->r / ADE_B200_GROUP, kbs = d->N / ade::LT_KB;
+    p.hparts = grid / ng < kbs ? grid / ng : kbs;
+    if (p.hparts < 1) return ADE_ERR_SHAPE;
+    // D = F32 (bits 4-5 = 1), A = B = bf16 (bits 7-9, 10-12 = 1), both K-major, N >> 3 (bits 17-22), M >> 4 = 8 (bits 24-28)
+    p.idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.tpad >> 3) << 17) | (8u << 24);
+    p.tmem_cols = 32;
+    while (static_cast<int>(p.tmem_cols) < p.tpad * (1 + p.segs)) p.tmem_cols *= 2;
+    rc = set_blocks(p, d);
+    if (rc) return rc;
+    p.spin_limit = g_wait_limit;
+    p.drop_arrivals = g_drop_signals;
+#ifdef ADE_TRACE
+    p.trace = g_trace;
+#endif
+    if (!load_encode_tiled()) return ADE_ERR_CUDA;
+    ade::LinearMaps maps;
+    const uint64_t N = static_cast<uint64_t>(d->N);
+    if (!make_map_2d(&maps.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_b, N, d->M, ade::LT_KB, p.rows, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_map_2d(&maps.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, N, T, ade::LT_KB, p.tpad, CU_TENSOR_MAP_SWIZZLE_128B))
+        return ADE_ERR_CUDA;
+    return launch_grid(ade::linear_tc_kernel, grid, ade::LT_THREADS, static_cast<size_t>(p.ring_bytes) + ade::LT_SMEM_FIXED,
+                       static_cast<cudaStream_t>(stream), p, maps);
 }
 
 int ade_b200_factored_static(const ade_delta_t* d, const void* x, const void* y_dense, const void* w_b, void* out,

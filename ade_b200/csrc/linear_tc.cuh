@@ -1,0 +1,678 @@
+// One delta linear module  out = x W_b^T + U^ (V^T x)  for up to 128 token rows, one launch, every contraction on the
+// 5th-generation tensor cores.
+//
+// Replaces, per call, the library GEMM of the base term and the reference's kernels A and B behind it
+// (src/kernels.py:486-886, src/serving.py:106-111).  The weights are the 128-row operand of tcgen05.mma (K-major, bf16), the
+// token rows the N operand (padded to a multiple of 16), the accumulators stay in tensor memory for the whole launch.
+//
+// What bounds it: the stream of W_b from HBM, and for short streams the two grid-wide hand-overs of h.  Rows are cut into
+// equal slices, so every SM streams the same number of bytes.  With one slice per SM (ksplit = 1) nothing has to be combined
+// afterwards, but every SM reads all of x (from L2); when x would cost more than the weights do, slices are ksplit times as
+// tall and ksplit SMs share one, each taking a part of the columns and exchanging float32 partial sums through global scratch
+// in a fixed order (the rule is linear_split below).
+//
+// Everything a CTA multiplies goes through ONE ring of shared-memory stages (A part: up to 128 rows x 64 columns, B
+// part: the token rows of the same columns), in this order:
+//   A items   h = V^T x: the (rank group, 64-column block) pairs are dealt to all CTAs.  A = (code - zero) * scale, one bf16
+//             rounding, written by the eight unpack warps; B = x by TMA.  The float32 partial sums of h go to scratch; when
+//             all have arrived every CTA adds its share of the T x r elements, rounds to bf16 once and publishes it.
+//   W items   the CTA's part of W_b: A and B by TMA.  While the tensor core works through them, the unpack warps do the h
+//             exchange above: the hand-overs are hidden under the stream as far as it is long enough.
+//   U items   U^ h on top of the same accumulators, one 64-rank block per warp or group of warps.  The scale of a (row, group) belongs to
+//             the row, so it is multiplied into the A operand; scale (8 significant bits) times code - zero (4) is 12 bits,
+//             which is exactly the sum of two bf16 values hi + lo: two MMA passes share one B tile of h and the product is
+//             exact, as when the scale was applied to the float32 sums.
+#pragma once
+#include <cuda.h>
+
+#include "factored.cuh"
+#include "recon.cuh"
+
+namespace ade {
+
+constexpr int LT_UNPACK_WARPS = 8;
+constexpr int LT_LOAD_WARP = LT_UNPACK_WARPS;
+constexpr int LT_MMA_WARP = LT_UNPACK_WARPS + 1;
+constexpr int LT_THREADS = 32 * (LT_UNPACK_WARPS + 2);
+constexpr int LT_UNPACK_THREADS = 32 * LT_UNPACK_WARPS;
+constexpr int LT_TILE = 128;                       // rows of the MMA: ranks of a group, or up to 128 rows of a slice
+constexpr int LT_KB = 64;                          // contraction block: 64 bf16 = one 128-byte swizzled row
+constexpr int LT_A_BYTES = LT_TILE * 128;
+constexpr int LT_MAX_STAGES = 12;
+constexpr int LT_MAX_SEG = 3;                      // slices per CTA (accumulators in tensor memory beside that of h)
+constexpr int LT_SMEM_FIXED = 1024 /* alignment */ + 8 * (2 * LT_MAX_STAGES + 5) + 32;
+
+struct LinearParams {
+    const uint8_t* uq;             // [M][r/2]
+    const uint8_t* vt;             // [r][N/2]
+    const uint16_t* us;            // [M][ng]
+    const uint8_t* uz;             // [M][ng]
+    const uint16_t* vs;            // [ng][N]
+    const uint8_t* vz;             // [ng][N]
+    __nv_bfloat16* h;              // scratch: bf16 [T][r]
+    unsigned int* sync;            // scratch: [0] partial sums of h written, [1] CTAs past their waits, [3] shares of h published
+    unsigned int* status;          // an expired wait records 1
+    float* part;                   // workspace: [CTA][T][128] partial sums of h, later of the output
+    unsigned int* slice_count;     // workspace: arrivals per slice (zeroed by the kernel before use)
+    __nv_bfloat16* out;            // [T][M]
+    int T, tpad, M, N, r;
+    int slices, segs, ksplit;      // row slices; slices per CTA (ksplit = 1), or CTAs per slice (segs = 1)
+    int rows;                      // tallest slice
+    int hparts;                    // CTAs per rank group in the computation of h
+    int stages;                    // even
+    uint32_t ring_bytes;           // the ring's area; reused for the exchange of partial sums once it has drained
+    uint32_t idesc;
+    uint32_t tmem_cols;
+    int n_blocks;                  // block-diagonal U^ as in FactoredParams
+    int block_rows[5];
+    int block_groups[5];
+    long long spin_limit;
+    int drop_arrivals;
+    unsigned long long* trace;     // development builds (ADE_TRACE) only
+};
+#ifdef ADE_TRACE
+#define LT_STAMP(i) do { if (p.trace && (threadIdx.x & 31) == 0) p.trace[(blockIdx.x * 10 + (threadIdx.x >> 5)) * 16 + (i)] = clock64(); } while (0)
+#else
+#define LT_STAMP(i) do { } while (0)
+#endif
+
+struct LinearMaps {
+    CUtensorMap w;                 // (M, N) bf16, box `rows` rows x 64, 128-byte swizzle
+    CUtensorMap x;                 // (T, N) bf16, box tpad rows x 64, 128-byte swizzle
+};
+
+// D[tmem] (+)= A[smem desc] * B[smem desc], bf16 operands, float32 accumulate, K = 16
+__device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t n) {
+    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar), "r"(n) : "memory");
+}
+__device__ __forceinline__ uint32_t bf2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ void unpack_sync() { asm volatile("bar.sync 1, %0;" ::"n"(LT_UNPACK_THREADS) : "memory"); }
+// other CTAs' generic-proxy writes (made visible by an acquire) -> this thread's bulk copies
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// Grid-wide wait of one thread for a counter (bounded; an expired wait is recorded and the launch carries on to its end).
+__device__ __forceinline__ void lt_wait_count(const unsigned int* c, unsigned int want, const LinearParams& p, volatile int* abort_flag) {
+    const long long t0 = clock64();
+    while (ld_acquire_gpu(c) < want) {
+        if (*abort_flag) return;
+        if (clock64() - t0 > p.spin_limit) {
+            *abort_flag = 1;
+            atomicExch(p.status, 1u);
+            return;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearParams p, const __grid_constant__ LinearMaps maps) {
+    extern __shared__ uint8_t lt_smem[];
+    const uint32_t raw0 = smem_u32(lt_smem);
+    const uint32_t ring = (raw0 + 1023u) & ~1023u;
+    const int S = p.stages;
+    const uint32_t x_bytes = static_cast<uint32_t>(p.tpad) * 128u;               // one B block
+    const uint32_t stage_bytes = LT_A_BYTES + x_bytes;
+    const uint32_t bars = ring + p.ring_bytes;
+    const uint32_t bar_full = bars, bar_empty = bars + 8 * S, bar_h = bars + 16 * S, bar_done = bar_h + 8, bar_gate = bar_h + 16,
+                   bar_pass = bar_h + 24, bar_fix = bar_h + 32;
+    uint8_t* gen = lt_smem + (bar_fix + 8 - raw0);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 4);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const int G = gridDim.x, c = blockIdx.x;
+    LT_STAMP(0);
+    const int T = p.T, N = p.N, M = p.M, r = p.r, ng = r >> 7;
+    const int kbs = N / LT_KB;                                   // column blocks
+    // A items: CTA c computes part c % hparts of rank group c / hparts
+    const int hg = c / p.hparts, hp = c - hg * p.hparts;
+    const bool has_h = hg < ng;
+    const int a0 = has_h ? hp * kbs / p.hparts : 0;
+    const int a1 = has_h ? (hp + 1) * kbs / p.hparts : 0;
+
+    // The operands of the first two A items are requested before anything else: their round trip runs under the set-up.
+    struct AOp {
+        uint4 q, s[4], z[2];
+    } acur, anxt;
+    const int row = tid >> 1, half = tid & 1;                    // rank and 32-column half an unpack thread writes
+    auto fetch_a = [&](AOp& o, int kb) {
+        o.q = ldg16_stream(p.vt + static_cast<size_t>(hg * 128 + row) * (N >> 1) + half * 16 + kb * 32);
+        const uint16_t* srow = p.vs + static_cast<size_t>(hg) * N + half * 32 + kb * LT_KB;
+        const uint8_t* zrow = p.vz + static_cast<size_t>(hg) * N + half * 32 + kb * LT_KB;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o.s[j] = ldg16(srow + 8 * j);
+        o.z[0] = ldg16(zrow);
+        o.z[1] = ldg16(zrow + 16);
+    };
+    if (warp < LT_UNPACK_WARPS) {
+        if (a0 < a1) fetch_a(acur, a0);
+        if (a0 + 1 < a1) fetch_a(anxt, a0 + 1);
+    }
+
+    if (tid == LT_LOAD_WARP * 32) {
+        for (int i = 0; i < S; ++i) {
+            mbar_init(bar_full + 8 * i, 1 + LT_UNPACK_WARPS);
+            mbar_init(bar_empty + 8 * i, 1);
+        }
+        mbar_init(bar_h, 1);
+        mbar_init(bar_done, 1);
+        mbar_init(bar_gate, 1);
+        mbar_init(bar_pass, 1);
+        mbar_init(bar_fix, 1);
+        *abort_flag = 0;
+        fence_mbar_init();
+        prefetch_tensormap(&maps.w);
+        prefetch_tensormap(&maps.x);
+    }
+    if (warp == LT_MMA_WARP) {
+        tmem_alloc(smem_u32(tmem_slot), p.tmem_cols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    LT_STAMP(1);
+    const WaitCtx wctx{abort_flag, reinterpret_cast<int*>(p.status), p.spin_limit};
+
+    // W items: slices [slice0, slice0 + nseg), columns [k0, k1) in blocks
+    const int kpart = p.ksplit > 1 ? c % p.ksplit : 0;
+    const int slice0 = p.ksplit > 1 ? c / p.ksplit : c * p.segs;
+    const int nseg = max(0, min(p.segs, p.slices - slice0));
+    const int k0 = kpart * kbs / p.ksplit, k1 = (kpart + 1) * kbs / p.ksplit;
+    auto slice_row = [&](int s) { return static_cast<int>(static_cast<long long>(s) * M / p.slices); };
+    // U items of segment s: this CTA's share of the 64-rank blocks the slice's rows can touch
+    auto u_range = [&](int s, int& u0, int& u1) {
+        int lo = 0, hi = ng;
+        if (p.n_blocks > 0) {
+            const int m0 = slice_row(slice0 + s), m1 = slice_row(slice0 + s + 1);
+            int l = ng, h = 0;
+            for (int i = 0; i < p.n_blocks; ++i)
+                if (p.block_rows[i] < m1 && p.block_rows[i + 1] > m0) {
+                    l = min(l, p.block_groups[i]);
+                    h = max(h, p.block_groups[i + 1]);
+                }
+            if (h > l) {
+                lo = l;
+                hi = h;
+            }
+        }
+        const int nu = 2 * (hi - lo);
+        u0 = 2 * lo + kpart * nu / p.ksplit;
+        u1 = 2 * lo + (kpart + 1) * nu / p.ksplit;
+    };
+    const int items = (a1 - a0) + nseg * (k1 - k0);                 // ring items before the first U item
+    const int gate = items - S;                                  // the item whose stage the first U item takes (none: negative)
+
+    if (warp == LT_LOAD_WARP) {
+        // ------------------------------------------------------------------ TMA producer
+        if (lane == 0) {
+            int st = 0;
+            uint32_t ph = 1;                                     // parity of the "empty" wait: the first round passes at once
+            auto next = [&]() {
+                if (++st == S) {
+                    st = 0;
+                    ph ^= 1;
+                }
+            };
+            for (int kb = a0; kb < a1; ++kb, next()) {
+                wait_bounded(bar_empty + 8 * st, ph, wctx, 1);
+                mbar_arrive_expect_tx(bar_full + 8 * st, x_bytes);
+                tma_load_2d(ring + st * stage_bytes + LT_A_BYTES, &maps.x, kb * LT_KB, 0, bar_full + 8 * st);
+            }
+            const uint32_t w_bytes = static_cast<uint32_t>(p.rows) * 128u;
+            for (int s = 0; s < nseg; ++s) {
+                const int m0 = slice_row(slice0 + s);
+                for (int kb = k0; kb < k1; ++kb, next()) {
+                    const uint32_t sa = ring + st * stage_bytes, full = bar_full + 8 * st;
+                    wait_bounded(bar_empty + 8 * st, ph, wctx, 1);
+                    mbar_arrive_n(full, LT_UNPACK_WARPS);        // the unpack warps have no part in a W item
+                    mbar_arrive_expect_tx(full, w_bytes + x_bytes);
+                    tma_load_2d(sa, &maps.w, kb * LT_KB, m0, full);
+                    tma_load_2d(sa + LT_A_BYTES, &maps.x, kb * LT_KB, 0, full);
+                }
+            }
+            for (int s = 0; s < nseg; ++s) {
+                int u0, u1;
+                u_range(s, u0, u1);
+                for (int j = 2 * u0; j < 2 * u1; ++j, next()) {
+                    wait_bounded(bar_empty + 8 * st, ph, wctx, 1);
+                    mbar_arrive(bar_full + 8 * st);              // everything of a U item is written by an unpack warp
+                }
+            }
+            // Every CTA checks out once it is past its grid-wide waits; the last one re-arms the counters for the next call.  This
+            // thread does it because nothing waits for it any more.
+            wait_bounded(bar_pass, 0, wctx, 1);
+            if (atomicAdd(p.sync + 1, 1u) == static_cast<unsigned int>(G - 1)) {
+                atomicExch(p.sync, 0u);
+                atomicExch(p.sync + 1, 0u);
+                atomicExch(p.sync + 3, 0u);
+            }
+        }
+        __syncwarp();
+    } else if (warp == LT_MMA_WARP) {
+        // ------------------------------------------------------------------ MMA issuer (warp-uniform loop, one elected lane)
+        int st = 0;
+        uint32_t ph = 0;
+        auto next = [&]() {
+            if (++st == S) {
+                st = 0;
+                ph ^= 1;
+            }
+        };
+        auto mma4 = [&](uint32_t d, uint32_t a, uint32_t b, bool fresh) {
+            const uint64_t ad = smem_desc_k_sw128(a), bd = smem_desc_k_sw128(b);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) tc_mma_bf16(d, ad + 2 * k, bd + 2 * k, p.idesc, fresh && k == 0 ? 0u : 1u);
+        };
+        int it = 0;
+        for (int kb = a0; kb < a1; ++kb, ++it, next()) {
+            wait_bounded(bar_full + 8 * st, ph, wctx, 1);
+            tc_fence_after();
+            if (elect_one()) {
+                mma4(tmem_base, ring + st * stage_bytes, ring + st * stage_bytes + LT_A_BYTES, kb == a0);
+                tc_commit(bar_empty + 8 * st);
+                if (it == gate) tc_commit(bar_gate);
+                if (kb == a1 - 1) tc_commit(bar_h);
+            }
+            __syncwarp();
+        }
+        LT_STAMP(2);
+        for (int s = 0; s < nseg; ++s) {
+            const uint32_t d = tmem_base + static_cast<uint32_t>(p.tpad) * (1 + s);
+            for (int kb = k0; kb < k1; ++kb, ++it, next()) {
+                const uint32_t sa = ring + st * stage_bytes;
+                wait_bounded(bar_full + 8 * st, ph, wctx, 1);
+                tc_fence_after();
+                if (elect_one()) {
+                    mma4(d, sa, sa + LT_A_BYTES, kb == k0);
+                    tc_commit(bar_empty + 8 * st);
+                    if (it == gate) tc_commit(bar_gate);
+                }
+                __syncwarp();
+            }
+        }
+        LT_STAMP(3);
+        for (int s = 0; s < nseg; ++s) {
+            int u0, u1;
+            u_range(s, u0, u1);
+            const uint32_t d = tmem_base + static_cast<uint32_t>(p.tpad) * (1 + s);
+            for (int j = u0; j < u1; ++j) {                      // two stages per 64-rank block: hi, then lo with hi's B tile
+                const int s_hi = st;
+                wait_bounded(bar_full + 8 * st, ph, wctx, 1);
+                next();
+                wait_bounded(bar_full + 8 * st, ph, wctx, 1);
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint32_t b = ring + s_hi * stage_bytes + LT_A_BYTES;
+                    mma4(d, ring + s_hi * stage_bytes, b, false);
+                    mma4(d, ring + st * stage_bytes, b, false);
+                    tc_commit(bar_empty + 8 * s_hi);
+                    tc_commit(bar_empty + 8 * st);
+                }
+                __syncwarp();
+                next();
+            }
+        }
+        LT_STAMP(4);
+        if (elect_one()) tc_commit(bar_done);
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------------ unpack, h exchange, epilogue
+        // counters of the slices, used after the second hand-over only
+        if (p.ksplit > 1)
+            for (int t = c * LT_UNPACK_THREADS + tid; t < p.slices; t += G * LT_UNPACK_THREADS) p.slice_count[t] = 0u;
+
+        {
+            int st = 0;
+            uint32_t ph = 1;
+            for (int kb = a0; kb < a1; ++kb) {
+                wait_bounded(bar_empty + 8 * st, ph, wctx, 1);
+                const uint32_t cw[4] = {acur.q.x, acur.q.y, acur.q.z, acur.q.w};
+                const uint32_t zw[8] = {acur.z[0].x, acur.z[0].y, acur.z[0].z, acur.z[0].w, acur.z[1].x, acur.z[1].y, acur.z[1].z, acur.z[1].w};
+                const uint32_t dst = ring + st * stage_bytes + static_cast<uint32_t>(row) * 128u;
+#pragma unroll
+                for (int wi = 0; wi < 4; ++wi) {                 // (code - zero) is exact; one rounding in the product
+                    uint32_t e[4];
+                    unpack8_bf16(cw[wi], e);
+                    const uint32_t sw[4] = {acur.s[wi].x, acur.s[wi].y, acur.s[wi].z, acur.s[wi].w};
+                    uint32_t o[4];
+                    o[0] = bf2_mul(bf2_sub(e[0], __byte_perm(zw[2 * wi], 0x43434343u, 0x4140)), sw[0]);
+                    o[1] = bf2_mul(bf2_sub(e[1], __byte_perm(zw[2 * wi], 0x43434343u, 0x4342)), sw[1]);
+                    o[2] = bf2_mul(bf2_sub(e[2], __byte_perm(zw[2 * wi + 1], 0x43434343u, 0x4140)), sw[2]);
+                    o[3] = bf2_mul(bf2_sub(e[3], __byte_perm(zw[2 * wi + 1], 0x43434343u, 0x4342)), sw[3]);
+                    sts16(dst + (((half * 4 + wi) ^ (row & 7)) << 4), make_uint4(o[0], o[1], o[2], o[3]));
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full + 8 * st);
+                acur = anxt;
+                if (kb + 2 < a1) fetch_a(anxt, kb + 2);
+                if (++st == S) {
+                    st = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+        LT_STAMP(2);
+
+        // ---- partial sums of h: tensor memory -> scratch, [part][token][rank]
+        const int q = warp & 3, hcol = warp >> 2;                // tensor-memory lane quarter, column half
+        const int rr = q * 32 + lane;                            // accumulator row of this thread
+        const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+        float* const part = p.part + static_cast<size_t>(c) * T * 128 + rr;
+        if (a0 < a1) {
+            wait_bounded(bar_h, 0, wctx, 1);
+            tc_fence_after();
+            for (int c0 = hcol * 16; c0 < p.tpad; c0 += 32) {
+                uint32_t v[16];
+                tmem_ld16_sync(lane_addr + c0, v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (c0 + i < T) __stcg(part + static_cast<size_t>(c0 + i) * 128, __uint_as_float(v[i]));
+            }
+        }
+        LT_STAMP(3);
+
+        // U blocks of this CTA, over its slices, in rounds of up to S / 2; in a round of few blocks several warps share one.  The
+        // codes of the first round do not depend on h and are requested before the waits.
+        int ucount = 0;
+        for (int s = 0; s < nseg; ++s) {
+            int u0, u1;
+            u_range(s, u0, u1);
+            ucount += u1 - u0;
+        }
+        struct UOp {
+            uint4 q[8];            // 32 codes of rows (lane >> 1) + 16 (usub + wpb i)
+            uint32_t s[8], z[8];
+        } u;
+        int ukb = 0;               // 64-rank block the operands belong to
+        const int urow = lane >> 1, uhalf = lane & 1;
+        auto warps_per_block = [](int count) { return count <= 1 ? 8 : (count <= 2 ? 4 : (count <= 4 ? 2 : 1)); };
+        auto fetch_u = [&](int i, int wpb) {
+            int s = 0, u0 = 0, u1 = 0;
+            for (; s < nseg; ++s) {
+                u_range(s, u0, u1);
+                if (i < u1 - u0) break;
+                i -= u1 - u0;
+            }
+            ukb = u0 + i;
+            const int m0 = slice_row(slice0 + s), m1 = slice_row(slice0 + s + 1), usub = warp & (wpb - 1);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int rk = 16 * (usub + wpb * k);
+                if (rk < p.rows) {
+                    const int m = min(m0 + urow + rk, m1 - 1);               // rows past the slice: any values, never stored
+                    u.q[k] = ldg16_stream(p.uq + static_cast<size_t>(m) * (r >> 1) + uhalf * 16 + ukb * 32);
+                    u.s[k] = p.us[static_cast<size_t>(m) * ng + (ukb >> 1)];
+                    u.z[k] = p.uz[static_cast<size_t>(m) * ng + (ukb >> 1)];
+                }
+            }
+        };
+
+        unpack_sync();
+        if (tid == 0 && a0 < a1 && !p.drop_arrivals) red_release_gpu_add(p.sync, 1u);
+        {
+            // after the release: the fence in it would wait for these loads too
+            const int count = min(ucount, S >> 1), wpb = warps_per_block(count);
+            if (warp / wpb < count) fetch_u(warp / wpb, wpb);
+        }
+        if (tid == 0) lt_wait_count(p.sync, static_cast<unsigned int>(ng * p.hparts), p, abort_flag);
+        unpack_sync();
+        LT_STAMP(4);
+        // ---- this CTA's share of h: four lanes per four ranks, each adds every fourth part, fixed order
+        {
+            const int quads = (T * r) >> 2;
+            const int q0 = static_cast<int>(static_cast<long long>(c) * quads / G), q1 = static_cast<int>(static_cast<long long>(c + 1) * quads / G);
+            const int sub = tid & 3;
+            const size_t stride = static_cast<size_t>(T) * 128;
+            for (int base = q0; base < q1; base += LT_UNPACK_THREADS / 4) {
+                const int i = base + (tid >> 2);
+                const bool live = i < q1;
+                const int e = 4 * i, t = e / r, k = e - t * r;
+                const float* src = p.part + (static_cast<size_t>(k >> 7) * p.hparts * T + t) * 128 + (k & 127);
+                float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+                for (int j = sub; live && j < p.hparts; j += 40) {
+                    uint4 a[10];
+#pragma unroll
+                    for (int k2 = 0; k2 < 10; ++k2) a[k2] = j + 4 * k2 < p.hparts ? ldcg16(src + (j + 4 * k2) * stride) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+                    for (int k2 = 0; k2 < 10; ++k2) {
+                        s0 += __uint_as_float(a[k2].x);
+                        s1 += __uint_as_float(a[k2].y);
+                        s2 += __uint_as_float(a[k2].z);
+                        s3 += __uint_as_float(a[k2].w);
+                    }
+                }
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    s0 += __shfl_xor_sync(0xFFFFFFFFu, s0, o);
+                    s1 += __shfl_xor_sync(0xFFFFFFFFu, s1, o);
+                    s2 += __shfl_xor_sync(0xFFFFFFFFu, s2, o);
+                    s3 += __shfl_xor_sync(0xFFFFFFFFu, s3, o);
+                }
+                if (live && sub == 0) {
+                    const __nv_bfloat162 lo = __floats2bfloat162_rn(s0, s1), hi = __floats2bfloat162_rn(s2, s3);
+                    uint2 v;
+                    v.x = *reinterpret_cast<const uint32_t*>(&lo);
+                    v.y = *reinterpret_cast<const uint32_t*>(&hi);
+                    *reinterpret_cast<uint2*>(p.h + e) = v;
+                }
+            }
+        }
+        LT_STAMP(5);
+        unpack_sync();
+        if (tid == 0) {
+            red_release_gpu_add(p.sync + 3, 1u);
+            lt_wait_count(p.sync + 3, static_cast<unsigned int>(G), p, abort_flag);
+            mbar_arrive(bar_pass);                               // the load warp checks out for this CTA
+        }
+        unpack_sync();
+        LT_STAMP(6);
+
+        // ---- U items.  The W items in between were not this role's business; a wait tells the phases of a barrier apart by their
+        // parity only, so before it joins the ring again it waits until the item that used the first U stage before has retired
+        // (items retire in order: every stage is then at most one phase behind).  For the same reason blocks go in rounds of
+        // S / 2, one use of every stage each, with a barrier of the role between rounds.
+        if (ucount > 0 && gate >= 0) wait_bounded(bar_gate, 0, wctx, 1);
+        LT_STAMP(7);
+        for (int first = 0; first < ucount; first += S >> 1) {
+            if (first > 0) unpack_sync();
+            const int count = min(ucount - first, S >> 1), wpb = warps_per_block(count);
+            const int i = first + warp / wpb;
+            if (i < first + count) {
+                const int usub = warp & (wpb - 1);
+                if (first > 0) fetch_u(i, wpb);
+                const int idx = items + 2 * i, use = idx / S, st = idx - use * S, idx2 = idx + 1, use2 = idx2 / S, st2 = idx2 - use2 * S;
+                wait_bounded(bar_empty + 8 * st, (use & 1) ^ 1, wctx, 1);
+                wait_bounded(bar_empty + 8 * st2, (use2 & 1) ^ 1, wctx, 1);
+                // B tile: h of 64 ranks, 16-byte pieces, eight round trips in flight per lane
+                const uint32_t hb = ring + st * stage_bytes + LT_A_BYTES;
+                for (int tb = 4 * usub; tb < T; tb += 32 * wpb) {
+                    uint4 hv[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int t = tb + (lane >> 3) + 4 * wpb * k;
+                        if (t < T) hv[k] = ldcg16(p.h + static_cast<size_t>(t) * r + ukb * 64 + (lane & 7) * 8);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int t = tb + (lane >> 3) + 4 * wpb * k;
+                        if (t < T) sts16(hb + t * 128 + (((lane & 7) ^ (t & 7)) << 4), hv[k]);
+                    }
+                }
+                const uint32_t d_hi = ring + st * stage_bytes, d_lo = ring + st2 * stage_bytes;
+#pragma unroll
+                for (int k8 = 0; k8 < 8; ++k8) {
+                    const int rk = 16 * (usub + wpb * k8);
+                    if (rk >= p.rows) break;
+                    const int ur = urow + rk;
+                    const uint32_t zz = kBf2_128 | u.z[k8] | (u.z[k8] << 16), s2 = u.s[k8] | (u.s[k8] << 16);
+                    const uint32_t cw[4] = {u.q[k8].x, u.q[k8].y, u.q[k8].z, u.q[k8].w};
+#pragma unroll
+                    for (int wi = 0; wi < 4; ++wi) {
+                        uint32_t e[4], hi[4], lo[4];
+                        unpack8_bf16(cw[wi], e);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t dz = bf2_sub(e[k], zz);           // exact
+                            hi[k] = bf2_mul(dz, s2);                         // the product's upper 8 bits
+                            lo[k] = bf2_fma(dz, s2, hi[k] ^ 0x80008000u);    // the rest of its 12, exact
+                        }
+                        const uint32_t off = ur * 128 + (((uhalf * 4 + wi) ^ (ur & 7)) << 4);
+                        sts16(d_hi + off, make_uint4(hi[0], hi[1], hi[2], hi[3]));
+                        sts16(d_lo + off, make_uint4(lo[0], lo[1], lo[2], lo[3]));
+                    }
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {                                 // the wpb warps of an item arrive for all eight
+                    mbar_arrive_n(bar_full + 8 * st, LT_UNPACK_WARPS / wpb);
+                    mbar_arrive_n(bar_full + 8 * st2, LT_UNPACK_WARPS / wpb);
+                }
+            }
+        }
+        LT_STAMP(8);
+
+        // ---- epilogue
+        if (nseg > 0) {
+            wait_bounded(bar_done, 0, wctx, 1);
+            tc_fence_after();
+        }
+        LT_STAMP(9);
+        if (p.ksplit == 1) {
+            for (int s = 0; s < nseg; ++s) {
+                const int m = slice_row(slice0 + s) + rr;
+                if (q * 32 >= p.rows) break;                     // uniform in the warp
+                const bool live = m < slice_row(slice0 + s + 1);
+                for (int c0 = hcol * 16; c0 < p.tpad; c0 += 32) {
+                    uint32_t v[16];
+                    tmem_ld16_sync(lane_addr + static_cast<uint32_t>(p.tpad) * (1 + s) + c0, v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (live && c0 + i < T) p.out[static_cast<size_t>(c0 + i) * M + m] = __float2bfloat16_rn(__uint_as_float(v[i]));
+                }
+            }
+        } else if (nseg > 0) {
+            // ksplit CTAs hold partial sums of the slice: each finishes an equal share of the tokens, [t0, t1)
+            const int n = p.ksplit, t0 = kpart * T / n, t1 = (kpart + 1) * T / n;
+            const uint32_t piece = static_cast<uint32_t>(t1 - t0) * 512u, acc = lane_addr + p.tpad;
+            for (int c0 = hcol * 16; c0 < p.tpad; c0 += 32) {
+                uint32_t v[16];
+                tmem_ld16_sync(acc + c0, v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int t = c0 + i;
+                    if (t < T) {
+                        if (t < t0 || t >= t1) __stcg(part + static_cast<size_t>(t) * 128, __uint_as_float(v[i]));
+                        else sts4(ring + kpart * piece + (t - t0) * 512 + rr * 4, v[i]);
+                    }
+                }
+            }
+            fence_proxy_async_all();
+            unpack_sync();
+            LT_STAMP(10);
+            if (tid == 0) {
+                red_release_gpu_add(p.slice_count + slice0, 1u);
+                if (piece > 0) {
+                    // the others' sums of this CTA's tokens are one contiguous piece each: all in flight together
+                    lt_wait_count(p.slice_count + slice0, static_cast<unsigned int>(n), p, abort_flag);
+                    fence_proxy_async_all();
+                    mbar_arrive_expect_tx(bar_fix, piece * static_cast<uint32_t>(n - 1));
+                    for (int j = 0; j < n; ++j)
+                        if (j != kpart) bulk_g2s(ring + j * piece, p.part + (static_cast<size_t>(c - kpart + j) * T + t0) * 128, piece, bar_fix);
+                }
+            }
+            __syncwarp();
+            LT_STAMP(11);
+            if (piece > 0) {
+                wait_bounded(bar_fix, 0, wctx, 1);
+                // a warp per token, consecutive rows per lane: contributors added in their order, one rounding
+                const int m0 = slice_row(slice0), rows = slice_row(slice0 + 1) - m0;
+                for (int t = t0 + warp; t < t1; t += LT_UNPACK_WARPS) {
+                    const uint32_t src = ring + static_cast<uint32_t>(t - t0) * 512u + lane * 4;
+                    float v[4] = {0.f, 0.f, 0.f, 0.f};
+                    for (int j = 0; j < n; ++j) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) v[k] += __uint_as_float(lds4(src + j * piece + k * 128));
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (lane + 32 * k < rows) p.out[static_cast<size_t>(t) * M + m0 + lane + 32 * k] = __float2bfloat16_rn(v[k]);
+                }
+            }
+        }
+        LT_STAMP(12);
+    }
+
+    drain_after_abort(abort_flag);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == LT_MMA_WARP) tmem_dealloc(tmem_base, p.tmem_cols);
+}
+
+// How a launch is cut: see the note at the top.
+struct LinearSplit {
+    int slices, segs, ksplit, rows, stages;
+    uint32_t ring_bytes;
+};
+constexpr int kLtRingMax = 232448 - LT_SMEM_FIXED;
+
+// Cost in microseconds of `ksplit` CTAs per slice, as far as the choice depends on it: the bytes an SM takes in (its weights
+// once, x for its columns; 83 GB/s per SM measured with all SMs streaming), the MMAs (a 64-column block takes about 0.2 us
+// whatever the height of the slice: the tensor core reads 128 rows) and the exchange of partial sums.
+inline double linear_split_cost(int M, int N, int T, int grid, int ksplit) {
+    const int slices = grid / ksplit;
+    const double rows = (M + slices - 1) / slices;
+    const double ingest = (rows + T) * 2.0 * N / ksplit / 83e3;
+    const double mma = 0.2 * N / LT_KB / ksplit;
+    return (ingest > mma ? ingest : mma) + (ksplit > 1 ? 3.0 + 2.0 * T * rows * 4.0 / 83e3 : 0.0);
+}
+inline bool linear_split(int M, int N, int T, int tpad, int grid, LinearSplit& out) {
+    const int kbs = N / LT_KB;
+    LinearSplit s = {};
+    s.ksplit = 1;
+    s.segs = (M + LT_TILE * grid - 1) / (LT_TILE * grid);
+    if (s.segs > LT_MAX_SEG) return false;
+    if (s.segs == 1) {
+        double best = linear_split_cost(M, N, T, grid, 1);
+        for (int k = 2; k <= kbs && k <= grid; ++k) {
+            const int slices = grid / k;
+            if ((M + slices - 1) / slices > LT_TILE) break;
+            const double cost = linear_split_cost(M, N, T, grid, k);
+            if (cost < best) {
+                best = cost;
+                s.ksplit = k;
+            }
+        }
+    }
+    s.slices = grid / s.ksplit * s.segs;
+    if (s.slices > M) s.slices = M;
+    s.rows = (M + s.slices - 1) / s.slices;
+    const int stage = LT_A_BYTES + tpad * 128;
+    s.stages = kLtRingMax / stage;
+    if (s.stages > LT_MAX_STAGES) s.stages = LT_MAX_STAGES;
+    s.stages &= ~1;
+    int ring = s.stages * stage;
+    const int fix = s.ksplit > 1 ? 512 * (T + s.ksplit) : 0;      // n pieces of ceil(T / n) token rows at most
+    if (ring < fix) ring = (fix + 1023) & ~1023;
+    s.ring_bytes = static_cast<uint32_t>(ring);
+    if (s.stages < 2 || ring > kLtRingMax) return false;
+    out = s;
+    return true;
+}
+
+// Workspace: partial sums (of h, then of the output) and the slice counters behind them.
+inline size_t linear_part_bytes(int T, int grid) { return static_cast<size_t>(grid) * T * 128 * sizeof(float); }
+inline size_t linear_workspace_bytes(int T, int grid) { return linear_part_bytes(T, grid) + static_cast<size_t>(grid) * sizeof(unsigned int); }
+
+}  // namespace ade

@@ -278,6 +278,37 @@ def factored_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor | None = No
             raise _kernel_error(e) from None
 
 
+def linear_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor) -> torch.Tensor:
+    """out = x W_b^T + U^(V^T x) for T <= 128 tokens with every contraction on the tensor cores, one call of
+    ``ade_b200_linear`` (replaces the library GEMM + kernels A and B of src/serving.py:106-111)."""
+    lib = _lib.load()
+    M, N, r = int(p4["M"]), int(p4["N"]), int(p4["r"])
+    _check_x(x, N, "x")
+    T = x.shape[0]
+    if not (weight.dtype == torch.bfloat16 and weight.is_contiguous() and tuple(weight.shape) == (M, N) and weight.device == x.device):
+        raise ValueError("weight must be a contiguous bfloat16 (d_o, d_i) tensor on x's device")
+    with _on_device(x.device):
+        stream = torch.cuda.current_stream().cuda_stream
+        scratch = _scratch_for(x.device, stream, T, r, lib.ade_b200_factored_scratch_bytes(T, r))
+        try:
+            return _lib.ops().linear(x, weight, p4["uq"], p4["vq"], p4["vt"], p4["us"], p4["uz"], p4["vs"], p4["vz"],
+                                     M, N, r, _flat_blocks(p4), scratch)
+        except RuntimeError as e:
+            raise _kernel_error(e) from None
+
+
+# Up to this many tokens the warp-MMA kernel of `factored_forward` serves a module, above it the tensor-core kernel of
+# `linear_forward`.  Per call on B200, in a graph over rotated weights, factored / linear: 4096 x 4096 r = 512 T = 8 11.7 / 17,
+# T = 16 13.8 / 17.6; 11008 x 4096 T = 8 21.9 / 27, T = 16 28.5 / 28; above 16 tokens the former used a library GEMM for the base
+# term: 4096 x 4096 T = 40 27.7 / 18.8, 4096 x 11008 T = 100 63.8 / 30.3, 5000 x 5120 r = 896 T = 40 45.9 / 25.0 us.
+FACTORED_MAX_TOKENS = 16
+
+
+def module_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor) -> torch.Tensor:
+    """x W_b^T + U^(V^T x) of one module for T <= 128 tokens, by the kernel that is faster at T."""
+    return factored_forward(x, p4, weight=weight) if x.shape[0] <= FACTORED_MAX_TOKENS else linear_forward(x, p4, weight)
+
+
 def _kernel_error(e: RuntimeError) -> Exception:
     """A status the C ABI returned comes back from the binding as a RuntimeError; give it the library's own type."""
     msg = str(e).split("\n")[0]

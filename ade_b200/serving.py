@@ -5,7 +5,7 @@ decode_max_tokens, use_decode, use_recon, split_k)`` with ``forward(x)`` and the
 ``out_features / in_features / weight``, and ``build_kernel_model`` -- on top of the B200 kernels.
 Differences: tensors are bfloat16 (the reference module is float16), there is no float
 fallback (``use_decode`` / ``use_recon`` = False raise), and for T <= decode_max_tokens the base
-GEMM x W_b^T runs inside the factored kernel instead of a separate ``F.linear`` up to 16 tokens.
+GEMM x W_b^T runs in the same launch as the delta instead of a separate ``F.linear``.
 """
 from __future__ import annotations
 
@@ -13,15 +13,9 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .kernels import (GROUP, STORED_KEYS, decode_forward_packed, decode_kernel_status, expand_codes, factored_forward,
-                      pack_int4, recon_int4, recon_kernel_status)
+from .kernels import (GROUP, STORED_KEYS, decode_kernel_status, expand_codes, module_forward, pack_int4, recon_int4,
+                      recon_kernel_status)
 
-# Up to this many tokens the base GEMM x W_b^T runs inside the factored kernel (one launch, W_b streamed once by
-# a kernel built for skinny operands, h computed by side warps under the stream).  Above it cuBLAS is faster at the
-# base term, so the module falls back to the reference's split: F.linear for the base, the kernel for the delta
-# only (measured on B200 per call, fused / split: 4096 x 4096 T = 16 14.5 / 21.0 us, T = 32 22.4 / 23.7, T = 64
-# 46.3 / 29.2; 11008 x 4096 T = 16 30.1 / 34.0, T = 24 40.6 / 39.2, T = 64 117.6 / 55.9).
-FUSED_BASE_MAX_TOKENS = 16
 # Modules keep int8 operands for the reconstructed path once they have served a long input (see ADEKernelLinear._expanded).
 EXPAND_FOR_RECON = True
 
@@ -102,13 +96,10 @@ class ADEKernelLinear(nn.Module):
         T = x2.shape[0]
         if T == 0:
             return x2.new_empty(*shape[:-1], self.out_features)
-        if T <= FUSED_BASE_MAX_TOKENS and T <= self.decode_max_tokens:
+        if T <= self.decode_max_tokens:
             y = self._group[0].apply(self._group[1], x, x2) if self._group is not None else None
             if y is None:
-                y = factored_forward(x2, self._stored_form(), weight=self.weight)
-        elif T <= self.decode_max_tokens:
-            # the reference's own split (src/serving.py:106-111): library GEMM for the base term, kernel for the delta
-            y = decode_forward_packed(x2, F.linear(x2, self.weight), self._stored_form())
+                y = module_forward(x2, self._stored_form(), self.weight)
         else:
             y = F.linear(x2, self.merged_weight())
         return y.reshape(*shape[:-1], self.out_features)
@@ -191,7 +182,7 @@ class FusedADEGroup:
             self.release()
             return None
         if self._y is None or x is not self._x or x._version != self._ver or index in self._used:
-            self._y = factored_forward(x2, self.p4, weight=self.weight)
+            self._y = module_forward(x2, self.p4, self.weight)
             self._x, self._ver = x, x._version
             self._used = set()
         self._used.add(index)

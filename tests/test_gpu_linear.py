@@ -1,0 +1,90 @@
+"""The tensor-core module kernel (`ade_b200_linear`: base GEMM and delta in one launch, up to 128 token rows) against the CPU oracle."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from ade_b200 import _lib, kernels, serving, synth
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _case(M, N, r, T):
+    tp = synth.random_packed(M, N, r, M + N + T)
+    W, x = synth.base_weight(M, N, M + 1), synth.activations(T, N, T + 2)
+    return tp, W, x
+
+
+# one row, one slice per SM and fewer rows than SMs; ragged token counts around the multiples of 16; ksplit > 1 with ragged slices
+# (4096 x 2048 at 100 tokens, 1000 x 4096); the highest rank; two and three slices per SM (19000 and 38000 rows); the widest token range
+@pytest.mark.parametrize("M,N,r,T", [(1, 128, 128, 1), (100, 256, 512, 17), (129, 128, 256, 128), (500, 1024, 128, 33), (1000, 4096, 384, 20),
+                                     (4096, 2048, 640, 100), (301, 4096, 1024, 64), (256, 384, 2048, 47), (19000, 128, 256, 40),
+                                     (38000, 128, 128, 128), (2050, 1152, 896, 16)])
+def test_linear_matches_oracle(M, N, r, T):
+    tp, W, x = _case(M, N, r, T)
+    p4 = kernels.pack_int4(tp, device=DEV)
+    y = kernels.linear_forward(x.to(DEV), p4, W.to(DEV))
+    y2 = kernels.linear_forward(x.to(DEV), p4, W.to(DEV))
+    torch.cuda.synchronize()
+    kernels.check_factored_status(DEV)
+    assert torch.equal(y, y2), "two runs differ"
+    ref = O.factored_apply(x.view(torch.uint16).numpy(), W.view(torch.uint16).numpy(), O.packed_from_torch(tp))
+    err, cos = O.parity(y.float().cpu().numpy(), ref)
+    assert err <= 1e-2 and cos >= 0.9999, (err, cos)
+
+
+@pytest.mark.parametrize("T", [17, 64, 128])
+def test_fused_group_above_16_tokens(T):
+    """A group of three modules of different heights and ranks, one launch, against the members alone: the same products; the
+    contraction is cut differently, so up to the last bf16 bit (2^-8 of the value, and of the row's terms where they cancel)."""
+    N = 1024
+    mods, packs = [], []
+    for M, r in ((700, 256), (300, 384), (1300, 128)):
+        tp, W, x = _case(M, N, r, T)
+        mods.append(serving.ADEKernelLinear(W, tp).to(DEV))
+    xd = x.to(DEV)
+    alone = [m(xd) for m in mods]
+    group = serving.FusedADEGroup(mods)
+    assert group.p4["blocks"] is not None
+    for a, m in zip(alone, mods):
+        y = m(xd)
+        assert torch.all((y.float() - a.float()).abs() <= 2.0 ** -7 * (a.float().abs() + a.float().abs().mean()))
+    torch.cuda.synchronize()
+    kernels.check_factored_status(DEV)
+
+
+def test_linear_wait_expires_and_recovers():
+    """Nobody reports h: every CTA's wait runs out, the launch still ends, the status word says so, the next call is right."""
+    M, N, r, T = 512, 1024, 256, 40
+    tp, W, x = _case(M, N, r, T)
+    p4, W, x = kernels.pack_int4(tp, device=DEV), W.to(DEV), x.to(DEV)
+    good = kernels.linear_forward(x, p4, W)
+    torch.cuda.synchronize()
+    _lib.set_option(_lib.OPT_WAIT_LIMIT_CYCLES, 400_000)
+    _lib.set_option(_lib.OPT_DROP_SIGNALS, 1)
+    try:
+        kernels.linear_forward(x, p4, W)
+        torch.cuda.synchronize()
+        assert kernels.factored_status(DEV, T, r) == 1
+        with pytest.raises(_lib.AdeKernelError):
+            kernels.check_factored_status(DEV)
+    finally:
+        _lib.set_option(_lib.OPT_DROP_SIGNALS, 0)
+        _lib.set_option(_lib.OPT_WAIT_LIMIT_CYCLES, 0)
+        kernels.reset_factored_scratch(DEV)
+    again = kernels.linear_forward(x, p4, W)
+    torch.cuda.synchronize()
+    assert kernels.factored_status(DEV, T, r) == 0 and torch.equal(again, good)
+
+
+def test_linear_argument_checks():
+    tp, W, x = _case(256, 256, 128, 20)
+    p4 = kernels.pack_int4(tp, device=DEV)
+    with pytest.raises(ValueError):
+        kernels.linear_forward(x.to(DEV), p4, W.to(DEV).t())
+    with pytest.raises(ValueError):
+        kernels.linear_forward(x.float().to(DEV), p4, W.to(DEV))
+    with pytest.raises(_lib.AdeKernelError):
+        kernels.linear_forward(torch.zeros(129, 256, dtype=torch.bfloat16, device=DEV), p4, W.to(DEV))
