@@ -50,6 +50,7 @@ unsigned long long* g_trace = nullptr;         // development builds: device buf
 
 template <int NT>
 bool optin_factored();
+bool optin_compress();
 
 // per-device set-up: architecture check, SM count, dynamic shared-memory opt-in
 int device_info(const DeviceInfo** out) {
@@ -77,9 +78,7 @@ int device_info(const DeviceInfo** out) {
                 !cuda_ok(cudaFuncSetAttribute(ade::recon_strip_kernel<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
                 !cuda_ok(cudaFuncSetAttribute(ade::recon_strip_kernel<false, false, true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
                 return ADE_ERR_CUDA;
-            if (!cuda_ok(cudaFuncSetAttribute(ade::compress_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              static_cast<int>(ade::compress_smem_bytes(ade::CQ_MAX_RANK, true)))))
-                return ADE_ERR_CUDA;
+            if (!optin_compress()) return ADE_ERR_CUDA;
             if (!cuda_ok(cudaFuncSetAttribute(ade::linear_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) return ADE_ERR_CUDA;
             if (!optin_factored<1>() || !optin_factored<2>() || !optin_factored<4>() || !optin_factored<8>() ||
                 !optin_factored<16>())
@@ -255,6 +254,35 @@ bool optin_factored() {
            cuda_ok(cudaFuncSetAttribute(ade::factored_kernel<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
 }
 
+// Instantiations of the producer kernel: rotated rows of 128 NJ elements (NJ a power of two), or groups one by one; 16-byte loads
+// where the pointers allow them.
+using CompressKernel = void (*)(const float*, const float*, uint8_t*, __nv_bfloat16*, __nv_bfloat16*, int, int);
+template <bool TRANSPOSED, bool VEC>
+CompressKernel compress_kernel_for(int ng, bool rotate) {
+    if (!rotate) return ade::compress_rows_kernel<1, false, TRANSPOSED, VEC>;
+    switch (ng) {
+        case 1: return ade::compress_rows_kernel<1, true, TRANSPOSED, VEC>;
+        case 2: return ade::compress_rows_kernel<2, true, TRANSPOSED, VEC>;
+        case 4: return ade::compress_rows_kernel<4, true, TRANSPOSED, VEC>;
+        case 8: return ade::compress_rows_kernel<8, true, TRANSPOSED, VEC>;
+        default: return ade::compress_rows_kernel<16, true, TRANSPOSED, VEC>;
+    }
+}
+CompressKernel compress_kernel(int ng, bool rotate, bool transposed, bool vec) {
+    if (transposed) return vec ? compress_kernel_for<true, true>(ng, rotate) : compress_kernel_for<true, false>(ng, rotate);
+    return vec ? compress_kernel_for<false, true>(ng, rotate) : compress_kernel_for<false, false>(ng, rotate);
+}
+bool optin_compress() {
+    const int smem = static_cast<int>(ade::compress_smem_bytes(ade::CQ_MAX_RANK, true));
+    for (int vec = 0; vec < 2; ++vec) {
+        if (!cuda_ok(cudaFuncSetAttribute(compress_kernel(1, false, true, vec), cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) return false;
+        for (int ng = 1; ng <= 16; ng *= 2)
+            if (!cuda_ok(cudaFuncSetAttribute(compress_kernel(ng, true, true, vec), cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
+                return false;
+    }
+    return true;
+}
+
 // block-diagonal hint of the delta -> kernel parameters (validated: ascending, covering [0, M) x [0, ng))
 template <class Params>
 int set_blocks(Params& p, const ade_delta_t* d) {
@@ -324,6 +352,36 @@ int ade_b200_pack_zeros(const uint16_t* zeros_bf16, uint8_t* out, size_t count, 
     if (count == 0) return ADE_OK;
     const int blocks = static_cast<int>((count + 255) / 256 < 65535 ? (count + 255) / 256 : 65535);
     pack_zeros_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(zeros_bf16, out, count);
+    return cuda_ok(cudaGetLastError()) ? ADE_OK : ADE_ERR_CUDA;
+}
+
+int ade_b200_pack_delta(const uint8_t* u_codes, const uint8_t* vt_codes, const uint16_t* u_zero_bf16, const uint16_t* vt_zero_bf16, uint8_t* uq,
+                        uint8_t* vq, uint8_t* vt, uint8_t* uz, uint8_t* vz, int M, int N, int r, void* stream) {
+    if (!u_codes || !vt_codes || !u_zero_bf16 || !vt_zero_bf16 || !uq || !vq || !vt || !uz || !vz) return ADE_ERR_NULL;
+    if (M < 1 || N < 8 || N % 8 || r < ADE_B200_GROUP || r % ADE_B200_GROUP) return ADE_ERR_SHAPE;
+    if (!aligned16(uq) || !aligned16(vq) || !aligned16(vt)) return ADE_ERR_ALIGN;
+    ade::PackParams p;
+    p.uc = u_codes;
+    p.vc = vt_codes;
+    p.uzb = u_zero_bf16;
+    p.vzb = vt_zero_bf16;
+    p.uq = reinterpret_cast<uint32_t*>(uq);
+    p.vq = reinterpret_cast<uint32_t*>(vq);
+    p.vt = reinterpret_cast<uint32_t*>(vt);
+    p.uz = uz;
+    p.vz = vz;
+    p.M = M;
+    p.N = N;
+    p.r = r;
+    p.vec = aligned16(u_codes) && aligned16(vt_codes);
+    const long long u_words = static_cast<long long>(M) * (r >> 3), zeros = (static_cast<long long>(M) + N) * (r >> 7);
+    const long long v_tiles = static_cast<long long>(r / ade::PK_K) * ((N + ade::PK_N - 1) / ade::PK_N);
+    const long long ub = (u_words + 4 * ade::PK_THREADS - 1) / (4 * ade::PK_THREADS), zb = (zeros + 4 * ade::PK_THREADS - 1) / (4 * ade::PK_THREADS);
+    p.u_blocks = static_cast<int>(ub < 1 << 20 ? ub : 1 << 20);
+    p.z_blocks = static_cast<int>(zb < 1 << 20 ? zb : 1 << 20);
+    if (v_tiles > 1 << 30) return ADE_ERR_SHAPE;
+    p.v_blocks = static_cast<int>(v_tiles);
+    ade::pack_delta_kernel<<<p.u_blocks + p.v_blocks + p.z_blocks, ade::PK_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(p);
     return cuda_ok(cudaGetLastError()) ? ADE_OK : ADE_ERR_CUDA;
 }
 
@@ -546,14 +604,11 @@ int ade_b200_compress_rows(const float* x, const float* sqrt_s, uint8_t* codes, 
     const DeviceInfo* di = nullptr;
     const int rc = device_info(&di);
     if (rc) return rc;
-    const int blocks_wanted = (rows + ade::CQ_ROWS - 1) / ade::CQ_ROWS;
-    const int grid = blocks_wanted < 8 * di->sms ? blocks_wanted : 8 * di->sms;
-    const size_t smem = ade::compress_smem_bytes(r, transposed != 0);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    __nv_bfloat16* sc = reinterpret_cast<__nv_bfloat16*>(scale);
-    __nv_bfloat16* zp = reinterpret_cast<__nv_bfloat16*>(zero);
-    if (transposed) ade::compress_rows_kernel<true><<<grid, ade::CQ_THREADS, smem, st>>>(x, sqrt_s, codes, sc, zp, rows, r, rotate);
-    else ade::compress_rows_kernel<false><<<grid, ade::CQ_THREADS, smem, st>>>(x, sqrt_s, codes, sc, zp, rows, r, rotate);
+    const int grid = (rows + ade::CQ_ROWS - 1) / ade::CQ_ROWS;
+    const bool vec = aligned16(x) && (!sqrt_s || aligned16(sqrt_s)) && (reinterpret_cast<uintptr_t>(codes) & 3u) == 0;
+    compress_kernel(r / ADE_B200_GROUP, rotate != 0, transposed != 0, vec)<<<grid, ade::CQ_THREADS, ade::compress_smem_bytes(r, transposed != 0),
+                                                                             static_cast<cudaStream_t>(stream)>>>(
+        x, sqrt_s, codes, reinterpret_cast<__nv_bfloat16*>(scale), reinterpret_cast<__nv_bfloat16*>(zero), rows, r);
     return cuda_ok(cudaGetLastError()) ? ADE_OK : ADE_ERR_CUDA;
 }
 

@@ -155,11 +155,8 @@ def _pack_int4_cuda(packed: dict, dev: torch.device) -> dict:
     }
     with _on_device(dev):
         sp = torch.cuda.current_stream().cuda_stream
-        _lib.check(lib.ade_b200_pack_codes(uc.data_ptr(), out["uq"].data_ptr(), M, r, 0, sp), "ade_b200_pack_codes(U)")
-        _lib.check(lib.ade_b200_pack_codes(vc.data_ptr(), out["vt"].data_ptr(), r, N, 0, sp), "ade_b200_pack_codes(Vt)")
-        _lib.check(lib.ade_b200_pack_codes(vc.data_ptr(), out["vq"].data_ptr(), N, r, 1, sp), "ade_b200_pack_codes(V)")
-        _lib.check(lib.ade_b200_pack_zeros(uzb.data_ptr(), out["uz"].data_ptr(), M * ng, sp), "ade_b200_pack_zeros(U)")
-        _lib.check(lib.ade_b200_pack_zeros(vzb.data_ptr(), out["vz"].data_ptr(), ng * N, sp), "ade_b200_pack_zeros(Vt)")
+        _lib.check(lib.ade_b200_pack_delta(uc.data_ptr(), vc.data_ptr(), uzb.data_ptr(), vzb.data_ptr(), out["uq"].data_ptr(), out["vq"].data_ptr(),
+                                           out["vt"].data_ptr(), out["uz"].data_ptr(), out["vz"].data_ptr(), M, N, r, sp), "ade_b200_pack_delta")
     return out
 
 

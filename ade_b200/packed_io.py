@@ -111,8 +111,7 @@ class DeviceDeltaLoader:
     """Builds device stored forms (the dict ``kernels.pack_int4`` returns) from packed modules in one pass.
 
     Per module: the six fields are copied into one pinned staging block (two blocks alternate), sent to the GPU
-    with one asynchronous copy on a side stream, and packed there by ``ade_b200_pack_codes`` (uq, vt, and vq
-    with the transposing read) and ``ade_b200_pack_zeros``; scales are already in their final form.  The staging
+    with one asynchronous copy on a side stream, and packed there by one launch of ``ade_b200_pack_delta``; scales are already in their final form.  The staging
     blocks are sized for the largest module seen and reused.  ``finish()`` joins the side stream.
     """
 
@@ -183,11 +182,8 @@ class DeviceDeltaLoader:
             staged[:total].copy_(pinned[:total], non_blocking=True)
             base = staged.data_ptr()
             at = lambda k: base + off[k][0]
-            check(lib.ade_b200_pack_codes(at("U_codes"), out["uq"].data_ptr(), M, r, 0, sp), "ade_b200_pack_codes(U)")
-            check(lib.ade_b200_pack_codes(at("Vt_codes"), out["vt"].data_ptr(), r, N, 0, sp), "ade_b200_pack_codes(Vt)")
-            check(lib.ade_b200_pack_codes(at("Vt_codes"), out["vq"].data_ptr(), N, r, 1, sp), "ade_b200_pack_codes(V)")
-            check(lib.ade_b200_pack_zeros(at("U_zero"), out["uz"].data_ptr(), M * ng, sp), "ade_b200_pack_zeros(U)")
-            check(lib.ade_b200_pack_zeros(at("Vt_zero"), out["vz"].data_ptr(), ng * N, sp), "ade_b200_pack_zeros(Vt)")
+            check(lib.ade_b200_pack_delta(at("U_codes"), at("Vt_codes"), at("U_zero"), at("Vt_zero"), out["uq"].data_ptr(), out["vq"].data_ptr(),
+                                          out["vt"].data_ptr(), out["uz"].data_ptr(), out["vz"].data_ptr(), M, N, r, sp), "ade_b200_pack_delta")
             out["us"].view(torch.uint8).reshape(-1).copy_(staged[off["U_scale"][0]:off["U_scale"][0] + off["U_scale"][1]])
             out["vs"].view(torch.uint8).reshape(-1).copy_(staged[off["Vt_scale"][0]:off["Vt_scale"][0] + off["Vt_scale"][1]])
             ev = torch.cuda.Event()

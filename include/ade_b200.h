@@ -110,6 +110,14 @@ int ade_b200_pack_codes(const uint8_t* codes, uint8_t* out, int rows, int K, int
 int ade_b200_pack_zeros(const uint16_t* zeros_bf16, uint8_t* out, size_t count, void* stream);
 
 /*
+ * Both of the above for a whole module in one launch: U codes (M, r) and V^T codes (r, N), one code per byte, and the
+ * bfloat16 zero-points (M, r/128) / (r/128, N) -> uq, vq, vt, uz, vz of struct ade_delta.  uq, vq and vt 16-byte aligned;
+ * the inputs may have any alignment.
+ */
+int ade_b200_pack_delta(const uint8_t* u_codes, const uint8_t* vt_codes, const uint16_t* u_zero_bf16, const uint16_t* vt_zero_bf16, uint8_t* uq,
+                        uint8_t* vq, uint8_t* vt, uint8_t* uz, uint8_t* vz, int M, int N, int r, void* stream);
+
+/*
  * Producer side of the format on the device: one factor of a truncated SVD to codes, scales and zero-points in one
  * pass (replaces, per factor, the chain of src/quantization.py:244-285: scaling by sqrt(S) :266-268, the shared
  * rotation H :270-272, and quantize_rowwise / quantize_colwise :134-199 with _pin_zero_in_range :109-131).

@@ -5,7 +5,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from ade_b200 import _lib, quantization as Q
+from ade_b200 import _lib, kernels, quantization as Q, synth
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -83,3 +83,43 @@ def test_compress_module_on_the_gpu(d_o, d_i, r):
     assert torch.equal(folded["U_scale"], (cpu["U_scale"].float() * gamma.unsqueeze(1)).to(torch.bfloat16))
     assert torch.equal(folded["Vt_scale"], (cpu["Vt_scale"].float() * rho.unsqueeze(0)).to(torch.bfloat16))
     assert folded["U_codes"] is cpu["U_codes"]
+
+
+def _hadamard_rows(X):
+    """Fast Walsh-Hadamard transform in float32, strides 1, 2, 4, ... as the kernel takes them."""
+    rows, r = X.shape
+    h = 1
+    while h < r:
+        v = X.reshape(rows, r // (2 * h), 2, h)
+        X = torch.stack([v[:, :, 0] + v[:, :, 1], v[:, :, 0] - v[:, :, 1]], 2).reshape(rows, r)
+        h *= 2
+    return X * (1.0 / r ** 0.5)
+
+
+@pytest.mark.parametrize("rows,r,shift", [(1, 256, 0), (33, 1024, 0), (70, 256, 1), (31, 1024, 3), (4097, 256, 0)])
+def test_rotated_rows_bit_exact(rows, r, shift):
+    """Ranks that are powers of four (their normalisation is exact): the butterflies round one by one in a fixed order, so the
+    codes equal those of the same transform done with torch.  `shift`: an input that is not 16-byte aligned."""
+    g = torch.Generator().manual_seed(rows + r)
+    X, root = torch.randn(rows, r, generator=g) * 0.05, torch.rand(r, generator=g) + 0.1
+    buf = torch.zeros(rows * r + 4, device=DEV)
+    Xd = buf[shift:shift + rows * r].view(rows, r).copy_(X)
+    rot = _hadamard_rows(X * root)
+    for transposed in (False, True):
+        c, s, z = _kernel(Xd, root.to(DEV), True, transposed)
+        rc, rs, rz = Q.quantize_colwise(rot.t().contiguous(), 4, 128) if transposed else Q.quantize_rowwise(rot, 4, 128)
+        assert torch.equal(c.cpu(), rc) and torch.equal(s.cpu(), rs) and torch.equal(z.cpu(), rz)
+
+
+@pytest.mark.parametrize("M,N,r,shift", [(1, 8, 128, 0), (129, 136, 256, 0), (300, 1000, 384, 1), (64, 4096, 2048, 8)])
+def test_pack_delta_matches_host_packing(M, N, r, shift):
+    """One launch for the whole stored form: ragged d_i (multiples of 8), unaligned code arrays."""
+    tp = synth.random_packed(M, N, r, M + N + r)
+    host = kernels.pack_int4(tp)
+    dev = {k: v.to(DEV) for k, v in tp.items()}
+    for k in ("U_codes", "Vt_codes"):
+        buf = torch.zeros(tp[k].numel() + 16, dtype=torch.uint8, device=DEV)
+        dev[k] = buf[shift:shift + tp[k].numel()].view(tp[k].shape).copy_(tp[k])
+    out = kernels.pack_int4(dev)
+    for k in kernels.STORED_KEYS:
+        assert torch.equal(out[k].cpu(), host[k]), k
