@@ -633,7 +633,8 @@ int ade_b200_rope(const void* q, const void* k, const void* cos_t, const void* s
                   int k_heads, int head_dim, long long q_row_stride, long long k_row_stride, long long cs_batch_stride, void* stream) {
     if (!q || !k || !cos_t || !sin_t || !q_out || !k_out) return ADE_ERR_NULL;
     if (B < 1 || T < 1 || q_heads < 1 || k_heads < 1 || head_dim < 2 || (head_dim & 1)) return ADE_ERR_SHAPE;
-    const long long total = static_cast<long long>(B) * T * (q_heads + k_heads) * head_dim;
+    // sixteen elements per thread in the usual case; an input the kernel takes element by element makes more rounds
+    const long long total = static_cast<long long>(B) * T * (q_heads + k_heads) * ((head_dim + 15) / 16);
     const int blocks = static_cast<int>((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
     return launch_small(ade::rope_kernel, blocks, 256, 0, stream, static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
                         static_cast<const __nv_bfloat16*>(cos_t), static_cast<const __nv_bfloat16*>(sin_t), static_cast<__nv_bfloat16*>(q_out),
@@ -644,7 +645,7 @@ int ade_b200_silu_mul(const void* gate, const void* up, void* out, int rows, int
                       void* stream) {
     if (!gate || !up || !out) return ADE_ERR_NULL;
     if (rows < 1 || cols < 1 || gate_row_stride < cols || up_row_stride < cols) return ADE_ERR_SHAPE;
-    const long long total = static_cast<long long>(rows) * cols;
+    const long long total = static_cast<long long>(rows) * ((cols + 7) / 8);
     const int blocks = static_cast<int>((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
     return launch_small(ade::silu_mul_kernel, blocks, 256, 0, stream, static_cast<const __nv_bfloat16*>(gate), static_cast<const __nv_bfloat16*>(up),
                         static_cast<__nv_bfloat16*>(out), rows, cols, gate_row_stride, up_row_stride);
