@@ -76,6 +76,9 @@ int device_info(const DeviceInfo** out) {
                 !cuda_ok(cudaFuncSetAttribute(ade::recon_strip_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
                 !cuda_ok(cudaFuncSetAttribute(ade::recon_strip_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
                 !cuda_ok(cudaFuncSetAttribute(ade::recon_strip_kernel<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
+                !cuda_ok(cudaFuncSetAttribute(ade::recon_strip_kernel<false, false, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
+                !cuda_ok(cudaFuncSetAttribute(ade::recon_strip_kernel<false, true, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
+                !cuda_ok(cudaFuncSetAttribute(ade::recon_strip_kernel<false, false, true, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
                 !cuda_ok(cudaFuncSetAttribute(ade::recon_strip_kernel<false, false, true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
                 return ADE_ERR_CUDA;
             if (!optin_compress()) return ADE_ERR_CUDA;
@@ -720,7 +723,7 @@ int ade_b200_set_option(int option, long long value) {
     }
 }
 
-int ade_b200_expand_codes(const ade_delta_t* d, void* u8, void* v8, void* stream) {
+static int expand_impl(const ade_delta_t* d, void* u8, void* v8, bool f8, void* stream) {
     int rc = check_delta(d);
     if (rc) return rc;
     if (!d->vq || !u8 || !v8) return ADE_ERR_NULL;
@@ -732,27 +735,40 @@ int ade_b200_expand_codes(const ade_delta_t* d, void* u8, void* v8, void* stream
     const long long chunks = (static_cast<long long>(d->M) + d->N) * ng * 4;
     const long long want = (chunks + 255) / 256;
     const int grid = static_cast<int>(want < 8ll * di->sms ? want : 8ll * di->sms);
-    ade::expand_codes_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(d->uq, d->uz, d->vq, d->vz, static_cast<uint8_t*>(u8),
-                                                                                 static_cast<uint8_t*>(v8), d->M, d->N, ng);
+    const auto kernel = f8 ? ade::expand_codes_kernel<true> : ade::expand_codes_kernel<false>;
+    kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(d->uq, d->uz, d->vq, d->vz, static_cast<uint8_t*>(u8), static_cast<uint8_t*>(v8), d->M,
+                                                                d->N, ng);
     return cuda_ok(cudaGetLastError()) ? ADE_OK : ADE_ERR_CUDA;
 }
 
-static int recon_impl(const ade_delta_t* d, const void* u8, const void* v8, const void* w_b, void* w_out, int32_t* dbg_acc,
+int ade_b200_expand_codes(const ade_delta_t* d, void* u8, void* v8, void* stream) { return expand_impl(d, u8, v8, false, stream); }
+
+int ade_b200_expand_codes_f8(const ade_delta_t* d, void* u8, void* v8, void* stream) { return expand_impl(d, u8, v8, true, stream); }
+
+static int recon_impl(const ade_delta_t* d, const void* u8, const void* v8, bool f8, const void* w_b, void* w_out, int32_t* dbg_acc,
                       int* status_dev, void* stream);
 
 int ade_b200_recon(const ade_delta_t* d, const void* w_b, void* w_out, int32_t* dbg_acc, int* status_dev,
                    void* stream) {
-    return recon_impl(d, nullptr, nullptr, w_b, w_out, dbg_acc, status_dev, stream);
+    return recon_impl(d, nullptr, nullptr, false, w_b, w_out, dbg_acc, status_dev, stream);
 }
 
 int ade_b200_recon_expanded(const ade_delta_t* d, const void* u8, const void* v8, const void* w_b, void* w_out,
                             int32_t* dbg_acc, int* status_dev, void* stream) {
     if (!u8 || !v8) return ADE_ERR_NULL;
     if (!aligned16(u8) || !aligned16(v8)) return ADE_ERR_ALIGN;
-    return recon_impl(d, u8, v8, w_b, w_out, dbg_acc, status_dev, stream);
+    return recon_impl(d, u8, v8, false, w_b, w_out, dbg_acc, status_dev, stream);
 }
 
-static int recon_impl(const ade_delta_t* d, const void* u8, const void* v8, const void* w_b, void* w_out, int32_t* dbg_acc,
+int ade_b200_recon_expanded_f8(const ade_delta_t* d, const void* u8, const void* v8, const void* w_b, void* w_out, int* status_dev,
+                               void* stream) {
+    if (!u8 || !v8) return ADE_ERR_NULL;
+    if (!aligned16(u8) || !aligned16(v8)) return ADE_ERR_ALIGN;
+    if (d && d->r > ade::RS_MAX_GROUPS * ADE_B200_GROUP) return ADE_ERR_SHAPE;
+    return recon_impl(d, u8, v8, true, w_b, w_out, nullptr, status_dev, stream);
+}
+
+static int recon_impl(const ade_delta_t* d, const void* u8, const void* v8, bool f8, const void* w_b, void* w_out, int32_t* dbg_acc,
                       int* status_dev, void* stream) {
     int rc = check_delta(d);
     if (rc) return rc;
@@ -804,7 +820,11 @@ static int recon_impl(const ade_delta_t* d, const void* u8, const void* v8, cons
             if (!make_map_2d(&maps.u8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, u8, r, M, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
                 !make_map_2d(&maps.v8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, v8, r, N, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B))
                 return ADE_ERR_CUDA;
-            if (ng > 4) {
+            if (f8) {
+                if (ng > 4) ade::recon_strip_kernel<false, true, true, 0, true><<<grid, ade::RS_THREADS_EXP, smem, st>>>(p, maps);
+                else if (ng == 4) ade::recon_strip_kernel<false, false, true, 4, true><<<grid, ade::RS_THREADS_EXP, smem, st>>>(p, maps);
+                else ade::recon_strip_kernel<false, false, true, 0, true><<<grid, ade::RS_THREADS_EXP, smem, st>>>(p, maps);
+            } else if (ng > 4) {
                 if (dbg_acc) ade::recon_strip_kernel<true, true, true><<<grid, ade::RS_THREADS_EXP, smem, st>>>(p, maps);
                 else ade::recon_strip_kernel<false, true, true><<<grid, ade::RS_THREADS_EXP, smem, st>>>(p, maps);
             } else {

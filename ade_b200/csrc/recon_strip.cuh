@@ -17,7 +17,7 @@
 //               128-byte-swizzled operand tiles; U items go to the resident strip, V items to a ring.
 //   warp  20    one thread issues tcgen05.mma.kind::i8 and the commits.
 //   warp  21    one thread issues the TMA copies of packed codes and V zero-points (raw ring).
-//   warp  22    scales: bf16 us / vs of the next tile -> float32 tables in shared memory (two buffers).
+//   warp  22    scales: bf16 us of a strip and vs of the next tile -> float32 tables in shared memory (two buffers each).
 // Every mbarrier wait is bounded as in recon.cuh (abort flag, status word, normal exit).
 //
 // Expanded operands (template parameter EXP): when the caller has run expand_codes_kernel once (int8 code minus
@@ -47,8 +47,11 @@ constexpr int RS_RAW_SLOT = RS_RAW_CODES + 256;          // + 128 zero-points, p
 constexpr int RS_ACC_STAGES = 4;                        // 128-column accumulators in tensor memory (all 512 columns)
 constexpr int RS_TMEM_COLS = RS_ACC_STAGES * RC_TILE;
 constexpr int RS_BOX_BYTES = 32 * 64;                    // a warp's 32 x 32 bf16 box
-// scale tables of one tile, per group: us of the 128 rows, then vs of the 128 columns, as float32
+// scale tables, per group: us of a strip's 128 rows and vs of a tile's 128 columns, as float32
 constexpr int RS_SC_BYTES = 512 + 512;
+
+// D = F32 (bits 4-5 = 1), A = B = e4m3 (bits 7-9, 10-12 = 0), both K-major, N >> 3 = 16 (bits 17-22), M >> 4 = 8 (bits 24-28)
+constexpr uint32_t RS_IDESC_F8 = (1u << 4) | (16u << 17) | (8u << 24);
 
 struct ReconMaps {
     CUtensorMap wb;     // (M, N) bf16, box 32 x 32, 64-byte swizzle
@@ -65,7 +68,7 @@ struct ReconMaps {
 template <bool BIG, bool EXP = false>
 struct RsCfg {
     static constexpr int GROUPS = BIG ? 8 : 4;           // resident groups at most
-    static constexpr int B_STAGES = EXP ? (BIG ? 3 : 5) : (BIG ? 2 : 3);   // int8 V tiles in flight
+    static constexpr int B_STAGES = EXP ? (BIG ? 3 : 5) : (BIG ? 2 : 3);   // 8-bit V tiles in flight (more were measured: no gain)
     static constexpr int RAW_DEPTH = EXP ? 1 : (BIG ? 2 : 4);                // packed items in flight (no ring when EXP)
     static constexpr int RAW_BYTES = EXP ? 0 : RAW_DEPTH * RS_RAW_SLOT;
     static constexpr int WB_BUFS = BIG ? 1 : 2;          // box buffers per epilogue warp
@@ -120,6 +123,18 @@ __device__ __forceinline__ void unpack_store_s(uint32_t tile, int row, int c, ui
 // Packed codes -> int8 operands (code minus zero-point) in the byte order the unpack role of recon_strip_kernel
 // produces: thread t turns the t-th 16-byte chunk of a (rows, r/2) code array into the t-th 32-byte chunk of the
 // (rows, r) int8 array.  U zero-points are (M, ng) bytes, V zero-points (ng, N).
+// F8: the same values as e4m3 bytes (integers up to 16 are exact in it) in natural rank order, for the float8 kernel.
+__device__ __forceinline__ uint32_t cvt_e4m3x2(uint32_t h2) {
+    uint16_t r;
+    asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(r) : "r"(h2));
+    return r;
+}
+__device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+template <bool F8>
 __global__ void __launch_bounds__(256) expand_codes_kernel(const uint8_t* __restrict__ uq, const uint8_t* __restrict__ uz,
                                                            const uint8_t* __restrict__ vq, const uint8_t* __restrict__ vz,
                                                            uint8_t* __restrict__ u8, uint8_t* __restrict__ v8, int M, int N, int ng) {
@@ -141,8 +156,17 @@ __global__ void __launch_bounds__(256) expand_codes_kernel(const uint8_t* __rest
         uint32_t o[8];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            o[2 * i] = ((w[i] & 0x0F0F0F0Fu) + zk) ^ 0x80808080u;
-            o[2 * i + 1] = (((w[i] >> 4) & 0x0F0F0F0Fu) + zk) ^ 0x80808080u;
+            if (F8) {
+                const uint32_t zz = 0x64006400u | z | (z << 16);            // half2 (1024 + zero): code - zero is exact
+                uint32_t e[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) e[j] = cvt_e4m3x2(h2_sub(((w[i] >> (4 * j)) & 0x000F000Fu) | 0x64006400u, zz));
+                o[2 * i] = e[0] | (e[1] << 16);
+                o[2 * i + 1] = e[2] | (e[3] << 16);
+            } else {
+                o[2 * i] = ((w[i] & 0x0F0F0F0Fu) + zk) ^ 0x80808080u;
+                o[2 * i + 1] = (((w[i] >> 4) & 0x0F0F0F0Fu) + zk) ^ 0x80808080u;
+            }
         }
         uint4* dst = reinterpret_cast<uint4*>((is_u ? u8 : v8) + e * 32);
         dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
@@ -152,7 +176,11 @@ __global__ void __launch_bounds__(256) expand_codes_kernel(const uint8_t* __rest
 
 // NG > 0: the number of groups is fixed at compile time (4: rank 512), so the epilogue's group loop unrolls with
 // constant stage, table and tensor-memory offsets; 0: read from the delta.
-template <bool DBG, bool BIG, bool EXP = false, int NG = 0>
+// F8: expanded operands as e4m3 bytes and float32 accumulators.  Every product (at most 225) and every partial sum (at most
+// 28 800) is an integer the accumulator holds exactly, so the group products are the INT32 ones, already as floats: the
+// accumulator needs no re-arming with the conversion constant, and the epilogue is three packed operations per pair on what
+// it loads.
+template <bool DBG, bool BIG, bool EXP = false, int NG = 0, bool F8 = false>
 __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_strip_kernel(const ReconParams p, const __grid_constant__ ReconMaps maps) {
     using C = RsCfg<BIG, EXP>;
     constexpr int MMA_WARP = EXP ? RS_EPI_WARPS : RS_MMA_WARP;
@@ -166,7 +194,7 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
     const uint32_t b_st = a_res + ng * RS_OPER_BYTES;                     // [C::B_STAGES][128][128] int8
     const uint32_t wbuf = b_st + C::B_STAGES * RS_OPER_BYTES;             // [16 warps][2][32][64 B]
     const uint32_t rawr = wbuf + C::WB_BYTES;                             // [C::RAW_DEPTH][RS_RAW_SLOT]
-    const uint32_t scf = rawr + C::RAW_BYTES;                             // [2][ng][RS_SC_BYTES] scale tables
+    const uint32_t scf = rawr + C::RAW_BYTES;                             // scale tables: F8 us [2 strips][ng][128], then vs [2 tiles][ng][128]; else [2 tiles][ng][us 128, vs 128]
     const uint32_t bars = scf + ng * RS_SC_BYTES * 2;
     uint8_t* gen = smem_raw + (bars - raw0);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + C::BAR_COUNT * 8);
@@ -224,11 +252,13 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
         uint32_t magic4[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) asm volatile("mov.u32 %0, %1;" : "=r"(magic4[i]) : "n"(RC_MAGIC));
+        if (!F8) {
 #pragma unroll
-        for (int st = 0; st < RS_ACC_STAGES; ++st)
+            for (int st = 0; st < RS_ACC_STAGES; ++st)
 #pragma unroll
-            for (int ch = 0; ch < 2; ++ch) tmem_st16_fill(lane_addr + st * RC_TILE + ch * 16, magic4);
-        tmem_st_wait();
+                for (int ch = 0; ch < 2; ++ch) tmem_st16_fill(lane_addr + st * RC_TILE + ch * 16, magic4);
+            tmem_st_wait();
+        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
@@ -241,6 +271,7 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
         uint32_t it = 0;
         bool tf_ready = false;                            // per-group barriers: the coming group's accumulator was seen complete
         int j = 0, sm = strip0, nt = nt0;
+        uint32_t sct_u = scf;                             // us table of the current strip
 #ifdef ADE_TRACE
         int tcn = 0;
         const int ttrack = warp == 0 ? 0 : 1;
@@ -280,7 +311,7 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
             }
             if (C::PER_TILE) tc_fence_after();
             EPI_STAMP(0x0200 | (j & 255));
-            const uint32_t sct = scf + b * (ng * RS_SC_BYTES);          // this tile's tables
+            const uint32_t sct = F8 ? scf + (2 + b) * (ng * 512) : scf + b * (ng * RS_SC_BYTES);     // the tile's vs, or both its tables
 
             uint64_t acc[16];
 #pragma unroll
@@ -299,13 +330,12 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                     tc_fence_after();
                 }
                 EPI_STAMP(0x0300 | g);
-                const uint32_t scg = sct + g * RS_SC_BYTES;
-                const float u = __uint_as_float(lds4(scg + row * 4));
+                const float u = __uint_as_float(lds4((F8 ? sct_u + g * 512 : sct + g * RS_SC_BYTES) + row * 4));
                 const uint64_t uu = f2_pack(u, u);
                 const float um = __fmul_rn(u, -12582912.0f);            // -m us, exact (m = 1.5 * 2^23)
                 const uint64_t cc = f2_pack(um, um);
                 const uint32_t tbase = lane_addr + a * RC_TILE;
-                const uint32_t svg = scg + 512 + hh * 128;               // vs of this warp's 32 columns
+                const uint32_t svg = (F8 ? sct + g * 512 : sct + g * RS_SC_BYTES + 512) + hh * 128;      // vs of this warp's 32 columns
                 // The accumulator started at RC_MAGIC, so its bits are the float m + P, exactly.
                 // x = fma(m + P, us, -m us) = P us exactly (|P| < 2^15, us has 8 significant bits);
                 // t = x * vs is P * (us * vs) rounded once, as the reference rounds it; acc + t rounded once.
@@ -318,7 +348,8 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {
                             const int k = h4 * 4 + kk;
-                            const uint64_t x2 = f2_fma(f2_pack(__uint_as_float(vc[2 * k]), __uint_as_float(vc[2 * k + 1])), uu, cc);
+                            const uint64_t pp = f2_pack(__uint_as_float(vc[2 * k]), __uint_as_float(vc[2 * k + 1]));
+                            const uint64_t x2 = f2_fma(pp, uu, cc);
                             acc[ch * 8 + k] = f2_fma(f2_mul(x2, vs2[kk]), one2, acc[ch * 8 + k]);
                         }
                     }
@@ -330,6 +361,34 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                                                                         vc[i + 3] - RC_MAGIC);
                     }
                 };
+                if constexpr (F8) {
+                    // The scales of the chunk are requested before its accumulators: their latency runs under that of tensor memory.
+                    auto rescale_f8 = [&](const uint32_t* vc, const uint64_t (&vs2)[8], const int ch) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            const uint64_t x2 = f2_mul(f2_pack(__uint_as_float(vc[2 * k]), __uint_as_float(vc[2 * k + 1])), uu);   // exact
+                            acc[ch * 8 + k] = f2_fma(f2_mul(x2, vs2[k]), one2, acc[ch * 8 + k]);
+                        }
+                    };
+                    if (!C::PER_TILE) {                  // is the next group's accumulator (next stage) there yet?  Used a group later.
+                        const uint32_t a1 = (it + 1) % RS_ACC_STAGES, ph1 = ((it + 1) / RS_ACC_STAGES) & 1;
+                        tf_ready = mbar_test(bar(C::BAR_TFULL + a1), ph1);
+                    }
+                    uint64_t vs2[8];
+#pragma unroll
+                    for (int ch = 0; ch < 2; ++ch) {
+                        uint32_t vc[16];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) lds_f2x2(svg + (ch * 4 + i) * 16, vs2[2 * i], vs2[2 * i + 1]);
+                        tmem_ld16_sync(tbase + ch * 16, vc);
+                        if (ch == 1) {                   // both chunks are in registers: hand the stage back
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(bar(C::BAR_TEMPTY + a));
+                        }
+                        rescale_f8(vc, vs2, ch);
+                    }
+                } else {
 #pragma unroll
                 for (int ch = 0; ch < 2; ++ch) {
                     uint32_t vc[16];                     // 16 columns at a time: 32 would not fit the register budget
@@ -339,14 +398,17 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                     }
                     tmem_ld16_sync(tbase + ch * 16, vc);
                     EPI_STAMP(0x0400 | (g << 1) | ch);
-                    tmem_st16_fill(tbase + ch * 16, magic4);             // re-arm, completes under the arithmetic
+                    tmem_st16_fill(tbase + ch * 16, magic4);    // re-arm, completes under the arithmetic
                     rescale16(vc, ch);
                 }
+                }
                 EPI_STAMP(0x0500 | g);
-                tmem_st_wait();                          // accumulator stage re-armed: hand it back
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(C::BAR_TEMPTY + a));
+                if (!F8) {
+                    tmem_st_wait();                      // accumulator stage re-armed: hand it back
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(C::BAR_TEMPTY + a));
+                }
                 EPI_STAMP(0x0600 | g);
                 if (C::WB_BUFS == 2 && g == 0 && lane == 0 && tile + 1 < t_end) {
                     // base box of the next tile into the other buffer; the store that last read it was issued a tile ago
@@ -390,6 +452,7 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
             if (++nt == tiles_n) {
                 nt = 0;
                 ++sm;
+                sct_u = 2 * scf + ng * 512 - sct_u;
             }
         }
         if (lane == 0) bulk_wait_group_read<0>();    // shared memory may go once the last store has read it
@@ -507,8 +570,10 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                     const uint64_t bd = smem_desc_k_sw128(b_st + s * RS_OPER_BYTES);
                     if (!EXP || elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            tc_mma_i8(tmem_base + a * RC_TILE, ad + 2 * kk, bd + 2 * kk, RC_IDESC, 1u);
+                        for (int kk = 0; kk < 4; ++kk) {
+                            if (F8) tc_mma_f8(tmem_base + a * RC_TILE, ad + 2 * kk, bd + 2 * kk, RS_IDESC_F8, kk > 0);
+                            else tc_mma_i8(tmem_base + a * RC_TILE, ad + 2 * kk, bd + 2 * kk, RC_IDESC, 1u);
+                        }
                         tc_commit(bar(C::BAR_B_EMPTY + s));
                         if (!C::PER_TILE) tc_commit(bar(C::BAR_TFULL + a));
                         else if (g == ng - 1) tc_commit(bar(C::BAR_TFULL + (jt & (C::TFULL_BARS - 1))));
@@ -597,54 +662,52 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
         __syncwarp();
     } else if (warp == SCALE_WARP) {
         // ------------------------------------------------------------------ scale tables, one tile ahead
-        int j = 0, sm = strip0, nt = nt0;
+        // vs of the tile's columns per tile; us of the strip's rows per tile too, or (F8) once per strip (two buffers each).  Strip
+        // k + 2 overwrites the us table of strip k after the wait for the tile two before its first one, which is not before
+        // strip k's last tile.  (13824 x 5120, r = 1024: 127 -> 121 us against a warp that rebuilt both tables for every tile with an
+        // integer division per us value.)
+        int j = 0, sm = strip0, nt = nt0, sk = -1, cur_strip = -1;
         for (int tile = t_begin; tile < t_end; ++tile, ++j) {
-            const int m0 = sm << 7, n0 = nt << 7;
+            const int strip = sm, n0 = nt << 7;
             if (++nt == tiles_n) {
                 nt = 0;
                 ++sm;
             }
+            const bool fresh = !F8 || strip != cur_strip;
+            if (fresh) {
+                cur_strip = strip;
+                ++sk;
+            }
             const uint32_t b = j & 1, jph = (j >> 1) & 1;
-            const uint32_t sct = scf + b * (ng * RS_SC_BYTES);
-            // us: rows m0.. of a (M, ng) array = 128 * ng consecutive bf16; vs: 128 consecutive bf16 per group
-            constexpr int NV = C::GROUPS / 2;           // 16-byte vectors per lane: 16 * ng of each kind over 32 lanes
-            uint4 vu[NV], vv[NV];
-            const long long u_first = static_cast<long long>(m0) * ng, u_total = static_cast<long long>(p.M) * ng;
+            constexpr int NV = C::GROUPS / 2;            // 16-byte vectors of vs per lane: 16 * ng over 32 lanes
+            uint4 vv[NV];
 #pragma unroll
             for (int t = 0; t < NV; ++t) {
-                const int vi = lane + 32 * t;             // 16-byte vector index, 16 * ng of each kind
-                vu[t] = make_uint4(0, 0, 0, 0);
-                vv[t] = make_uint4(0, 0, 0, 0);
-                if (vi < 16 * ng) {
-                    const long long e0 = u_first + 8 * vi;
-                    if (e0 + 8 <= u_total) {
-                        vu[t] = ldg16(p.us + e0);
-                    } else {
-                        uint32_t w[4] = {0, 0, 0, 0};
-                        for (int e = 0; e < 8; ++e)
-                            if (e0 + e < u_total) w[e >> 1] |= static_cast<uint32_t>(p.us[e0 + e]) << (16 * (e & 1));
-                        vu[t] = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                    vv[t] = ldg16(p.vs + static_cast<size_t>(vi >> 4) * p.N + n0 + (vi & 15) * 8);
-                }
+                const int vi = lane + 32 * t;             // 16-byte vector index: group vi / 16, columns 8 (vi % 16) ..
+                vv[t] = vi < 16 * ng ? ldg16(p.vs + static_cast<size_t>(vi >> 4) * p.N + n0 + (vi & 15) * 8) : make_uint4(0, 0, 0, 0);
             }
             wait_bounded(bar(C::BAR_SC_EMPTY + b), jph ^ 1, wctx, 11);
+            if (fresh) {
+                const uint32_t ut = F8 ? scf + (sk & 1) * (ng * 512) : scf + b * (ng * RS_SC_BYTES);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int m = (strip << 7) + lane + 32 * i;
+                    uint32_t hu[C::GROUPS];
+#pragma unroll
+                    for (int g = 0; g < C::GROUPS; ++g) hu[g] = m < p.M && g < ng ? p.us[static_cast<size_t>(m) * ng + g] : 0u;
+#pragma unroll
+                    for (int g = 0; g < C::GROUPS; ++g)
+                        if (g < ng) sts4(ut + g * (F8 ? 512 : RS_SC_BYTES) + (lane + 32 * i) * 4, hu[g] << 16);
+                }
+            }
+            const uint32_t vt = F8 ? scf + (2 + b) * (ng * 512) : scf + b * (ng * RS_SC_BYTES) + 512;
 #pragma unroll
             for (int t = 0; t < NV; ++t) {
                 const int vi = lane + 32 * t;
                 if (vi < 16 * ng) {
-                    const uint32_t wu[4] = {vu[t].x, vu[t].y, vu[t].z, vu[t].w};
-                    const uint32_t wv[4] = {vv[t].x, vv[t].y, vv[t].z, vv[t].w};
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const int eu = 8 * vi + e;        // element of the strip: row * ng + group
-                        const int r_ = eu / ng, g_ = eu - r_ * ng;
-                        const uint32_t hu = (e & 1) ? (wu[e >> 1] & 0xFFFF0000u) : (wu[e >> 1] << 16);
-                        sts4(sct + g_ * RS_SC_BYTES + r_ * 4, hu);
-                    }
-                    const uint32_t dst = sct + (vi >> 4) * RS_SC_BYTES + 512 + (vi & 15) * 32;   // 8 columns of group vi / 16
-                    sts16(dst, make_uint4(wv[0] << 16, wv[0] & 0xFFFF0000u, wv[1] << 16, wv[1] & 0xFFFF0000u));
-                    sts16(dst + 16, make_uint4(wv[2] << 16, wv[2] & 0xFFFF0000u, wv[3] << 16, wv[3] & 0xFFFF0000u));
+                    const uint32_t dst = F8 ? vt + vi * 32 : vt + (vi >> 4) * RS_SC_BYTES + (vi & 15) * 32;
+                    sts16(dst, make_uint4(vv[t].x << 16, vv[t].x & 0xFFFF0000u, vv[t].y << 16, vv[t].y & 0xFFFF0000u));
+                    sts16(dst + 16, make_uint4(vv[t].z << 16, vv[t].z & 0xFFFF0000u, vv[t].w << 16, vv[t].w & 0xFFFF0000u));
                 }
             }
             __syncwarp();

@@ -6,7 +6,7 @@
 //   torch.ops.ade_b200.factored(x, weight?, y_dense?, uq, vq, vt, us, uz, vs, vz, M, N, r, blocks, scratch) -> out
 //   torch.ops.ade_b200.linear(x, weight, uq, vq, vt, us, uz, vs, vz, M, N, r, blocks, scratch) -> out
 //   torch.ops.ade_b200.recon(base, uq, vq, vt, us, uz, vs, vz, M, N, r, dbg_acc?, status?, u8?, v8?) -> merged
-//   torch.ops.ade_b200.expand(uq, vq, vt, us, uz, vs, vz, M, N, r) -> (u8, v8)
+//   torch.ops.ade_b200.expand / expand_f8(uq, vq, vt, us, uz, vs, vz, M, N, r) -> (u8, v8)
 //
 // Built with the host compiler only (no nvcc): `python -m ade_b200.build`.
 #include <ATen/ATen.h>
@@ -122,16 +122,23 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const at::Tenso
     return out;
 }
 
+// A merge without kept operands expands the codes into a work buffer first and takes the float8 kernel: two launches, but the kernel
+// that unpacks codes inside is slower by more than the expansion from rank 384 up (4096 x 4096 r = 256 22.5 / 22.2 us;
+// 11008 x 4096 r = 512 72 / 50 us; 13824 x 5120 r = 1024 189 / 126 us; unpacking inside / both launches).
+constexpr int kExpandFirst = 384;
+
 at::Tensor recon(const at::Tensor& base, const at::Tensor& uq, const at::Tensor& vq, const at::Tensor& vt, const at::Tensor& us,
                  const at::Tensor& uz, const at::Tensor& vs, const at::Tensor& vz, int64_t M, int64_t N, int64_t r,
                  const c10::optional<at::Tensor>& dbg_acc, const c10::optional<at::Tensor>& status,
                  const c10::optional<at::Tensor>& u8, const c10::optional<at::Tensor>& v8) {
     TORCH_CHECK(u8.has_value() == v8.has_value(), "u8 and v8 come together");
+    const bool f8 = u8.has_value() && u8->scalar_type() == at::kFloat8_e4m3fn;
     if (u8.has_value())
-        TORCH_CHECK(u8->scalar_type() == at::kChar && v8->scalar_type() == at::kChar && u8->is_contiguous() && v8->is_contiguous() &&
+        TORCH_CHECK((u8->scalar_type() == at::kChar || f8) && v8->scalar_type() == u8->scalar_type() && u8->is_contiguous() && v8->is_contiguous() &&
                         u8->dim() == 2 && v8->dim() == 2 && u8->size(0) == M && u8->size(1) == r && v8->size(0) == N && v8->size(1) == r &&
                         u8->device() == base.device() && v8->device() == base.device(),
-                    "expanded operands must be contiguous int8 (d_o, r) and (d_i, r) tensors on the device of base");
+                    "expanded operands must be contiguous int8 or float8_e4m3fn (d_o, r) and (d_i, r) tensors on the device of base");
+    TORCH_CHECK(!(f8 && dbg_acc.has_value()), "the INT32 accumulators are dumped by the int8 kernels only");
     TORCH_CHECK(base.is_cuda() && base.scalar_type() == at::kBFloat16 && base.dim() == 2 && base.size(0) == M && base.size(1) == N,
                 "base must be a CUDA bfloat16 (", M, ", ", N, ") tensor");
     const at::Tensor b = base.contiguous();
@@ -148,22 +155,35 @@ at::Tensor recon(const at::Tensor& base, const at::Tensor& uq, const at::Tensor&
     int32_t* dbg = dbg_acc.has_value() ? static_cast<int32_t*>(dbg_acc->data_ptr()) : nullptr;
     int* st = status.has_value() ? static_cast<int*>(status->data_ptr()) : nullptr;
     void* stream = c10::cuda::getCurrentCUDAStream(base.get_device()).stream();
-    const int rc = u8.has_value() ? ade_b200_recon_expanded(&d, u8->data_ptr(), v8->data_ptr(), b.data_ptr(), out.data_ptr(), dbg, st, stream)
-                                  : ade_b200_recon(&d, b.data_ptr(), out.data_ptr(), dbg, st, stream);
+    int rc;
+    if (u8.has_value()) {
+        rc = f8 ? ade_b200_recon_expanded_f8(&d, u8->data_ptr(), v8->data_ptr(), b.data_ptr(), out.data_ptr(), st, stream)
+                : ade_b200_recon_expanded(&d, u8->data_ptr(), v8->data_ptr(), b.data_ptr(), out.data_ptr(), dbg, st, stream);
+    } else if (!dbg && d.r >= kExpandFirst && d.r <= 1024) {
+        const at::Tensor work = at::empty({(M + N) * r}, b.options().dtype(at::kByte));
+        uint8_t* u = static_cast<uint8_t*>(work.data_ptr());
+        rc = ade_b200_expand_codes_f8(&d, u, u + M * r, stream);
+        if (rc == ADE_OK) rc = ade_b200_recon_expanded_f8(&d, u, u + M * r, b.data_ptr(), out.data_ptr(), st, stream);
+    } else {
+        rc = ade_b200_recon(&d, b.data_ptr(), out.data_ptr(), dbg, st, stream);
+    }
     TORCH_CHECK(rc == ADE_OK, "ade_b200_recon: ", err_name(rc), rc == ADE_ERR_CUDA ? " (cudaError " : "",
                 rc == ADE_ERR_CUDA ? std::to_string(ade_b200_last_cuda_error()) + ")" : std::string());
     return out;
 }
 
-// int8 operands (code minus zero-point) of a stored form, for recon(..., u8, v8)
+// int8 or e4m3 operands (code minus zero-point) of a stored form, for recon(..., u8, v8)
+template <bool F8>
 std::tuple<at::Tensor, at::Tensor> expand(const at::Tensor& uq, const at::Tensor& vq, const at::Tensor& vt, const at::Tensor& us,
                                           const at::Tensor& uz, const at::Tensor& vs, const at::Tensor& vz, int64_t M, int64_t N, int64_t r) {
     TORCH_CHECK(uq.is_cuda(), "stored form must be on a CUDA device");
     const c10::cuda::CUDAGuard guard(uq.device());
     const ade_delta_t d = make_delta(uq, vq, vt, us, uz, vs, vz, M, N, r, {}, uq);
-    at::Tensor u8 = at::empty({M, r}, uq.options().dtype(at::kChar));
-    at::Tensor v8 = at::empty({N, r}, uq.options().dtype(at::kChar));
-    const int rc = ade_b200_expand_codes(&d, u8.data_ptr(), v8.data_ptr(), c10::cuda::getCurrentCUDAStream(uq.get_device()).stream());
+    at::Tensor u8 = at::empty({M, r}, uq.options().dtype(F8 ? at::kFloat8_e4m3fn : at::kChar));
+    at::Tensor v8 = at::empty({N, r}, uq.options().dtype(F8 ? at::kFloat8_e4m3fn : at::kChar));
+    void* stream = c10::cuda::getCurrentCUDAStream(uq.get_device()).stream();
+    const int rc = F8 ? ade_b200_expand_codes_f8(&d, u8.data_ptr(), v8.data_ptr(), stream)
+                      : ade_b200_expand_codes(&d, u8.data_ptr(), v8.data_ptr(), stream);
     TORCH_CHECK(rc == ADE_OK, "ade_b200_expand_codes: ", err_name(rc), rc == ADE_ERR_CUDA ? " (cudaError " : "",
                 rc == ADE_ERR_CUDA ? std::to_string(ade_b200_last_cuda_error()) + ")" : std::string());
     return {u8, v8};
@@ -179,11 +199,13 @@ TORCH_LIBRARY(ade_b200, m) {
     m.def("recon(Tensor base, Tensor uq, Tensor vq, Tensor vt, Tensor us, Tensor uz, Tensor vs, Tensor vz, int M, int N, int r, "
           "Tensor? dbg_acc, Tensor? status, Tensor? u8, Tensor? v8) -> Tensor");
     m.def("expand(Tensor uq, Tensor vq, Tensor vt, Tensor us, Tensor uz, Tensor vs, Tensor vz, int M, int N, int r) -> (Tensor, Tensor)");
+    m.def("expand_f8(Tensor uq, Tensor vq, Tensor vt, Tensor us, Tensor uz, Tensor vs, Tensor vz, int M, int N, int r) -> (Tensor, Tensor)");
 }
 
 TORCH_LIBRARY_IMPL(ade_b200, CUDA, m) {
     m.impl("factored", &factored);
     m.impl("linear", &linear);
     m.impl("recon", &recon);
-    m.impl("expand", &expand);
+    m.impl("expand", &expand<false>);
+    m.impl("expand_f8", &expand<true>);
 }

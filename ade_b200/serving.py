@@ -13,10 +13,10 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .kernels import (GROUP, STORED_KEYS, decode_kernel_status, expand_codes, module_forward, pack_int4, recon_int4,
+from .kernels import (GROUP, STORED_KEYS, decode_kernel_status, expand_codes_f8, module_forward, pack_int4, recon_int4,
                       recon_kernel_status)
 
-# Modules keep int8 operands for the reconstructed path once they have served a long input (see ADEKernelLinear._expanded).
+# Modules keep 8-bit operands for the reconstructed path once they have served a long input (see ADEKernelLinear._expanded).
 EXPAND_FOR_RECON = True
 
 # the seven linear modules of a LLaMA decoder layer (same list as src/adaptation.py:39-42)
@@ -76,11 +76,11 @@ class ADEKernelLinear(nn.Module):
         return self._p4
 
     def _expanded(self):
-        """int8 operands of the reconstruction kernel, built on the first long input and kept ((d_o + d_i) * r bytes;
+        """8-bit operands of the reconstruction kernel, built on the first long input and kept ((d_o + d_i) * r bytes;
         EXPAND_FOR_RECON = False keeps the packed codes only and unpacks inside the kernel on every call)."""
         p4 = self._stored_form()
         if self._x8 is None or self._x8[0] != p4["uq"].data_ptr():
-            self._x8 = (p4["uq"].data_ptr(), expand_codes(p4))
+            self._x8 = (p4["uq"].data_ptr(), expand_codes_f8(p4))
         return self._x8[1]
 
     def merged_weight(self) -> torch.Tensor:

@@ -251,8 +251,14 @@ int ade_b200_recon(const ade_delta_t* d, const void* w_b, void* w_out,
  * ade_b200_recon (the arrays are then ignored).
  */
 int ade_b200_expand_codes(const ade_delta_t* d, void* u8, void* v8, void* stream);
+/* The same operands as e4m3 bytes in rank order, for ade_b200_recon_expanded_f8. */
+int ade_b200_expand_codes_f8(const ade_delta_t* d, void* u8, void* v8, void* stream);
 int ade_b200_recon_expanded(const ade_delta_t* d, const void* u8, const void* v8, const void* w_b, void* w_out,
                             int32_t* dbg_acc, int* status_dev, void* stream);
+/* ade_b200_recon_expanded on operands of ade_b200_expand_codes_f8 (ranks up to 1024): the group products are formed in
+ * float32 accumulators, which hold them exactly, so the result is the same bit for bit. */
+int ade_b200_recon_expanded_f8(const ade_delta_t* d, const void* u8, const void* v8, const void* w_b, void* w_out, int* status_dev,
+                               void* stream);
 
 /*
  * Elementwise pieces of a LLaMA decoder layer at decode sizes, one launch each.  No counterpart in the reference, which
