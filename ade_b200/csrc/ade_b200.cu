@@ -309,7 +309,11 @@ int set_blocks(Params& p, const ade_delta_t* d) {
 // the status word, which only ade_b200_factored_static_status clears), always at the same place whatever T and
 // r, then h = V^T x and, above 16 tokens, the partial sums of sliced phase-A units in what is left.  In host
 // code this name is only a handle for cudaGetSymbolAddress.
-__device__ __align__(256) unsigned char g_static_scratch[ADE_B200_STATIC_SCRATCH_BYTES];
+// Behind it the workspace of the tensor-core kernel, which serves the calls with y_dense that it is preferred for.
+constexpr int kStaticGrid = 160;
+constexpr size_t kStaticWorkspace = static_cast<size_t>(kStaticGrid) * (ADE_B200_MAX_TOKENS * 128 * sizeof(float) + sizeof(unsigned int));
+static_assert(ADE_B200_STATIC_SCRATCH_BYTES % 256 == 0, "the workspace behind the scratch array keeps its alignment");
+__device__ __align__(256) unsigned char g_static_scratch[ADE_B200_STATIC_SCRATCH_BYTES + kStaticWorkspace];
 void* g_static_scratch_addr[kMaxDevices] = {};
 
 // Device address of the array on the current device; looked up on the first use per device.
@@ -469,35 +473,38 @@ int ade_b200_factored(const ade_delta_t* d, const void* x, const void* y_dense, 
     return launch_factored<16>(p, grid, st);
 }
 
+// With y_dense, the tensor-core kernel against the warp-MMA kernel, per call with the library GEMM of the base term in front, in us:
+// 4096 x 4096 r = 512 T = 32 27.6 / 23.3, T = 40 29.5 / 27.3, T = 65 32.8 / 36.5, T = 128 37.5 / 40.1; 5000 x 5120 r = 896 T = 32 38.0 / 35.4,
+// T = 40 38.7 / 45.9, T = 128 49.5 / 109; 11008 x 4096 r = 512 T = 32 39.5 / 38.7, T = 40 42.7 / 48.7, T = 128 46.8 / 73.1; 4096 x 11008 T = 40
+// 43.6 / 41.8, T = 100 50.6 / 63.9.  The warp-MMA kernel slows down with M r (its U^ h) whenever the tokens pass a power of two.
+int ade_b200_linear_preferred(int T, int M, int r) {
+    return T > 64 || (T > 32 && static_cast<long long>(M) * r >= 4000000);
+}
+
 size_t ade_b200_linear_workspace_bytes(int T, int M, int r) {
     const DeviceInfo* di = nullptr;
     if (T < 1 || M < 1 || r < 1 || device_info(&di)) return 0;
     return ade::linear_workspace_bytes(T, di->sms);
 }
 
-int ade_b200_linear(const ade_delta_t* d, const void* x, const void* w_b, void* out, void* scratch, size_t scratch_bytes,
-                    void* workspace, size_t workspace_bytes, int T, void* stream) {
-    int rc = check_delta(d);
-    if (rc) return rc;
-    if (!d->vt || !x || !w_b || !out || !scratch || !workspace) return ADE_ERR_NULL;
-    if (T < 1 || T > ADE_B200_MAX_TOKENS) return ADE_ERR_SHAPE;
-    if (!aligned16(d->vt) || !aligned16(x) || !aligned16(w_b) || !aligned16(out) || !aligned16(scratch) || !aligned16(workspace))
-        return ADE_ERR_ALIGN;
-    if (scratch_bytes < factored_scratch_min(T, d->r)) return ADE_ERR_SCRATCH;
+// Launch of the tensor-core module kernel; the arguments have been checked except for what depends on the device.
+static int launch_linear(const ade_delta_t* d, const void* x, const void* y_dense, const void* w_b, void* out, __nv_bfloat16* h,
+                         unsigned int* sync, unsigned int* status, void* workspace, size_t workspace_bytes, int T, void* stream) {
     const DeviceInfo* di = nullptr;
-    rc = device_info(&di);
+    int rc = device_info(&di);
     if (rc) return rc;
     const int grid = di->sms;                                   // one persistent CTA per SM, all co-resident
     if (workspace_bytes < ade::linear_workspace_bytes(T, grid)) return ADE_ERR_SCRATCH;
     ade::LinearParams p = {};
     p.tpad = (T + 15) / 16 * 16;
     ade::LinearSplit split;
-    if (!ade::linear_split(d->M, d->N, T, p.tpad, grid, split)) return ADE_ERR_SHAPE;
+    if (!ade::linear_split(d->M, d->N, T, p.tpad, grid, w_b != nullptr, split)) return ADE_ERR_SHAPE;
     p.slices = split.slices;
     p.segs = split.segs;
     p.ksplit = split.ksplit;
     p.rows = split.rows;
     p.stages = split.stages;
+    p.u_start = split.u_start;
     p.ring_bytes = split.ring_bytes;
     p.uq = d->uq;
     p.vt = d->vt;
@@ -505,9 +512,10 @@ int ade_b200_linear(const ade_delta_t* d, const void* x, const void* w_b, void* 
     p.uz = d->uz;
     p.vs = d->vs;
     p.vz = d->vz;
-    p.h = static_cast<__nv_bfloat16*>(scratch);
-    p.sync = reinterpret_cast<unsigned int*>(static_cast<char*>(scratch) + ade_b200_factored_sync_offset(T, d->r));
-    p.status = p.sync + 2;
+    p.h = h;
+    p.sync = sync;
+    p.status = status;
+    p.y_dense = static_cast<const __nv_bfloat16*>(y_dense);
     p.part = static_cast<float*>(workspace);
     p.slice_count = reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + ade::linear_part_bytes(T, grid));
     p.out = static_cast<__nv_bfloat16*>(out);
@@ -515,7 +523,7 @@ int ade_b200_linear(const ade_delta_t* d, const void* x, const void* w_b, void* 
     p.M = d->M;
     p.N = d->N;
     p.r = d->r;
-    const int ng = d->r / ADE_B200_GROUP, kbs = d->N / ade::LT_KB;
+    const int ng = d->r / ADE_B200_GROUP, kbs = d->N / ade::LT_ITEM;
     p.hparts = grid / ng < kbs ? grid / ng : kbs;
     if (p.hparts < 1) return ADE_ERR_SHAPE;
     // D = F32 (bits 4-5 = 1), A = B = bf16 (bits 7-9, 10-12 = 1), both K-major, N >> 3 (bits 17-22), M >> 4 = 8 (bits 24-28)
@@ -532,11 +540,27 @@ int ade_b200_linear(const ade_delta_t* d, const void* x, const void* w_b, void* 
     if (!load_encode_tiled()) return ADE_ERR_CUDA;
     ade::LinearMaps maps;
     const uint64_t N = static_cast<uint64_t>(d->N);
-    if (!make_map_2d(&maps.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_b, N, d->M, ade::LT_KB, p.rows, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !make_map_2d(&maps.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, N, T, ade::LT_KB, p.tpad, CU_TENSOR_MAP_SWIZZLE_128B))
+    if (!make_map_2d(&maps.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, N, T, ade::LT_KB, p.tpad, CU_TENSOR_MAP_SWIZZLE_128B)) return ADE_ERR_CUDA;
+    maps.w = maps.x;                                             // not read without W_b
+    if (w_b && !make_map_2d(&maps.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_b, N, d->M, ade::LT_KB, p.rows, CU_TENSOR_MAP_SWIZZLE_128B))
         return ADE_ERR_CUDA;
     return launch_grid(ade::linear_tc_kernel, grid, ade::LT_THREADS, static_cast<size_t>(p.ring_bytes) + ade::LT_SMEM_FIXED,
                        static_cast<cudaStream_t>(stream), p, maps);
+}
+
+int ade_b200_linear(const ade_delta_t* d, const void* x, const void* y_dense, const void* w_b, void* out, void* scratch, size_t scratch_bytes,
+                    void* workspace, size_t workspace_bytes, int T, void* stream) {
+    const int rc = check_delta(d);
+    if (rc) return rc;
+    if (!d->vt || !x || !out || !scratch || !workspace) return ADE_ERR_NULL;
+    if ((y_dense == nullptr) == (w_b == nullptr)) return ADE_ERR_NULL;      // exactly one base term
+    if (T < 1 || T > ADE_B200_MAX_TOKENS) return ADE_ERR_SHAPE;
+    if (!aligned16(d->vt) || !aligned16(x) || !aligned16(out) || !aligned16(scratch) || !aligned16(workspace) || (y_dense && !aligned16(y_dense)) ||
+        (w_b && !aligned16(w_b)))
+        return ADE_ERR_ALIGN;
+    if (scratch_bytes < factored_scratch_min(T, d->r)) return ADE_ERR_SCRATCH;
+    unsigned int* sync = reinterpret_cast<unsigned int*>(static_cast<char*>(scratch) + ade_b200_factored_sync_offset(T, d->r));
+    return launch_linear(d, x, y_dense, w_b, out, static_cast<__nv_bfloat16*>(scratch), sync, sync + 2, workspace, workspace_bytes, T, stream);
 }
 
 int ade_b200_factored_static(const ade_delta_t* d, const void* x, const void* y_dense, const void* w_b, void* out,
@@ -561,6 +585,11 @@ int ade_b200_factored_static(const ade_delta_t* d, const void* x, const void* y_
     // the array keeps whatever the previous call left: the four sync words must start at zero (the status word
     // behind them is sticky until ade_b200_factored_static_status clears it)
     if (!cuda_ok(cudaMemsetAsync(base, 0, 16, st))) return ADE_ERR_CUDA;
+    if (y_dense && ade_b200_linear_preferred(T, d->M, d->r) && di->sms <= kStaticGrid) {
+        unsigned int* sync = reinterpret_cast<unsigned int*>(base);
+        return launch_linear(d, x, y_dense, nullptr, out, reinterpret_cast<__nv_bfloat16*>(base + 256), sync, sync + 4,
+                             base + ADE_B200_STATIC_SCRATCH_BYTES, kStaticWorkspace, T, stream);
+    }
     ade::FactoredParams p;
     p.w_b = static_cast<const __nv_bfloat16*>(w_b);
     p.x = static_cast<const __nv_bfloat16*>(x);

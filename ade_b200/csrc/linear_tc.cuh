@@ -11,17 +11,22 @@
 // tall and ksplit SMs share one, each taking a part of the columns and exchanging float32 partial sums through global scratch
 // in a fixed order (the rule is linear_split below).
 //
-// Everything a CTA multiplies goes through ONE ring of shared-memory stages (A part: up to 128 rows x 64 columns, B
-// part: the token rows of the same columns), in this order:
-//   A items   h = V^T x: the (rank group, 64-column block) pairs are dealt to all CTAs.  A = (code - zero) * scale, one bf16
+// Everything a CTA multiplies goes through ONE ring of shared-memory stages (A part: up to 128 rows x 128 columns,
+// B part: the token rows of the same columns), in this order:
+//   A items   h = V^T x: the (rank group, 128-column block) pairs are dealt to all CTAs.  A = (code - zero) * scale, one bf16
 //             rounding, written by the eight unpack warps; B = x by TMA.  The float32 partial sums of h go to scratch; when
 //             all have arrived every CTA adds its share of the T x r elements, rounds to bf16 once and publishes it.
 //   W items   the CTA's part of W_b: A and B by TMA.  While the tensor core works through them, the unpack warps do the h
 //             exchange above: the hand-overs are hidden under the stream as far as it is long enough.
-//   U items   U^ h on top of the same accumulators, one 64-rank block per warp or group of warps.  The scale of a (row, group) belongs to
+//             (With a base term from the caller there are no W items; its values are added at the end.)
+//   U items   U^ h on top of the same accumulators, 64 ranks at a time, spread over the end of the stream.  The scale of a (row, group) belongs to
 //             the row, so it is multiplied into the A operand; scale (8 significant bits) times code - zero (4) is 12 bits,
 //             which is exactly the sum of two bf16 values hi + lo: two MMA passes share one B tile of h and the product is
 //             exact, as when the scale was applied to the float32 sums.
+// Measured (us per call in a graph over rotated weights, library GEMM + warp-MMA delta launch before): 4096 x 4096 r = 512 T = 40 27.8 -> 19.4
+// (its bytes take 5.4; the stream has ended after 9, h is there after 11.5, U^ h after 14, the exchange of partial sums takes 4);
+// 4096 x 11008 T = 100 63.6 -> 28.9; 11008 x 4096 T = 128 73.3 -> 35.5; 5000 x 5120 r = 896 T = 40 45.3 -> 25.8; 22016 x 4096 (a fused
+// group) T = 32 49.8.  One 64-column block per ring item took 36 and 70 us on the two tall ones: the issuing warp bound them.
 #pragma once
 #include <cuda.h>
 
@@ -36,11 +41,15 @@ constexpr int LT_MMA_WARP = LT_UNPACK_WARPS + 1;
 constexpr int LT_THREADS = 32 * (LT_UNPACK_WARPS + 2);
 constexpr int LT_UNPACK_THREADS = 32 * LT_UNPACK_WARPS;
 constexpr int LT_TILE = 128;                       // rows of the MMA: ranks of a group, or up to 128 rows of a slice
-constexpr int LT_KB = 64;                          // contraction block: 64 bf16 = one 128-byte swizzled row
-constexpr int LT_A_BYTES = LT_TILE * 128;
+constexpr int LT_KB = 64;                          // column block: 64 bf16 = one 128-byte swizzled row
+constexpr int LT_ITEM = 2 * LT_KB;                 // columns of a ring item: one wait, one commit per two blocks (the issuing warp needs some
+                                                   // 400 cycles per item, as long as the eight MMAs of a short slice take)
+constexpr int LT_A_BLOCK = LT_TILE * 128;
+constexpr int LT_A_BYTES = 2 * LT_A_BLOCK;
 constexpr int LT_MAX_STAGES = 12;
 constexpr int LT_MAX_SEG = 3;                      // slices per CTA (accumulators in tensor memory beside that of h)
-constexpr int LT_SMEM_FIXED = 1024 /* alignment */ + 8 * (2 * LT_MAX_STAGES + 5) + 32;
+constexpr int LT_MAX_BLOCKS = LT_MAX_SEG * 2 * 16;  // 64-rank blocks of a CTA at the highest rank
+constexpr int LT_SMEM_FIXED = 1024 /* alignment */ + 8 * (2 * LT_MAX_STAGES + LT_MAX_BLOCKS + 4) + 32;
 
 struct LinearParams {
     const uint8_t* uq;             // [M][r/2]
@@ -54,12 +63,14 @@ struct LinearParams {
     unsigned int* status;          // an expired wait records 1
     float* part;                   // workspace: [CTA][T][128] partial sums of h, later of the output
     unsigned int* slice_count;     // workspace: arrivals per slice (zeroed by the kernel before use)
+    const __nv_bfloat16* y_dense;  // [T][M]: base term supplied by the caller, nothing of W_b is streamed; or nullptr
     __nv_bfloat16* out;            // [T][M]
     int T, tpad, M, N, r;
     int slices, segs, ksplit;      // row slices; slices per CTA (ksplit = 1), or CTAs per slice (segs = 1)
     int rows;                      // tallest slice
     int hparts;                    // CTAs per rank group in the computation of h
-    int stages;                    // even
+    int stages;
+    int u_start;                   // W items a CTA streams before its first U item (h is there by then)
     uint32_t ring_bytes;           // the ring's area; reused for the exchange of partial sums once it has drained
     uint32_t idesc;
     uint32_t tmem_cols;
@@ -120,10 +131,10 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
     const uint32_t ring = (raw0 + 1023u) & ~1023u;
     const int S = p.stages;
     const uint32_t x_bytes = static_cast<uint32_t>(p.tpad) * 128u;               // one B block
-    const uint32_t stage_bytes = LT_A_BYTES + x_bytes;
+    const uint32_t stage_bytes = LT_A_BYTES + 2 * x_bytes;
     const uint32_t bars = ring + p.ring_bytes;
-    const uint32_t bar_full = bars, bar_empty = bars + 8 * S, bar_h = bars + 16 * S, bar_done = bar_h + 8, bar_gate = bar_h + 16,
-                   bar_pass = bar_h + 24, bar_fix = bar_h + 32;
+    const uint32_t bar_full = bars, bar_empty = bars + 8 * S, bar_slot = bars + 16 * S, bar_h = bar_slot + 8 * LT_MAX_BLOCKS, bar_done = bar_h + 8,
+                   bar_pass = bar_h + 16, bar_fix = bar_h + 24;
     uint8_t* gen = lt_smem + (bar_fix + 8 - raw0);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 4);
@@ -132,30 +143,31 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
     const int G = gridDim.x, c = blockIdx.x;
     LT_STAMP(0);
     const int T = p.T, N = p.N, M = p.M, r = p.r, ng = r >> 7;
-    const int kbs = N / LT_KB;                                   // column blocks
+    const int kbs = N / LT_ITEM;                                 // items along the columns
     // A items: CTA c computes part c % hparts of rank group c / hparts
     const int hg = c / p.hparts, hp = c - hg * p.hparts;
     const bool has_h = hg < ng;
     const int a0 = has_h ? hp * kbs / p.hparts : 0;
     const int a1 = has_h ? (hp + 1) * kbs / p.hparts : 0;
 
-    // The operands of the first two A items are requested before anything else: their round trip runs under the set-up.
+    // The operands of the first A item are requested before anything else: their round trip runs under the set-up.
     struct AOp {
-        uint4 q, s[4], z[2];
-    } acur, anxt;
-    const int row = tid >> 1, half = tid & 1;                    // rank and 32-column half an unpack thread writes
+        uint4 q[2], s[8], z[4];
+    } acur;
+    const int row = tid >> 1, half = tid & 1;                    // operand row and half of the item an unpack thread writes
     auto fetch_a = [&](AOp& o, int kb) {
-        o.q = ldg16_stream(p.vt + static_cast<size_t>(hg * 128 + row) * (N >> 1) + half * 16 + kb * 32);
-        const uint16_t* srow = p.vs + static_cast<size_t>(hg) * N + half * 32 + kb * LT_KB;
-        const uint8_t* zrow = p.vz + static_cast<size_t>(hg) * N + half * 32 + kb * LT_KB;
+        const uint8_t* qrow = p.vt + static_cast<size_t>(hg * 128 + row) * (N >> 1) + half * 32 + kb * 64;
+        const uint16_t* srow = p.vs + static_cast<size_t>(hg) * N + half * LT_KB + kb * LT_ITEM;
+        const uint8_t* zrow = p.vz + static_cast<size_t>(hg) * N + half * LT_KB + kb * LT_ITEM;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o.s[j] = ldg16(srow + 8 * j);
-        o.z[0] = ldg16(zrow);
-        o.z[1] = ldg16(zrow + 16);
+        for (int j = 0; j < 2; ++j) o.q[j] = ldg16_stream(qrow + 16 * j);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o.s[j] = ldg16(srow + 8 * j);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o.z[j] = ldg16(zrow + 16 * j);
     };
     if (warp < LT_UNPACK_WARPS) {
         if (a0 < a1) fetch_a(acur, a0);
-        if (a0 + 1 < a1) fetch_a(anxt, a0 + 1);
     }
 
     if (tid == LT_LOAD_WARP * 32) {
@@ -163,9 +175,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
             mbar_init(bar_full + 8 * i, 1 + LT_UNPACK_WARPS);
             mbar_init(bar_empty + 8 * i, 1);
         }
+        for (int i = 0; i < LT_MAX_BLOCKS; ++i) mbar_init(bar_slot + 8 * i, 1);
         mbar_init(bar_h, 1);
         mbar_init(bar_done, 1);
-        mbar_init(bar_gate, 1);
         mbar_init(bar_pass, 1);
         mbar_init(bar_fix, 1);
         *abort_flag = 0;
@@ -210,8 +222,23 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
         u0 = 2 * lo + kpart * nu / p.ksplit;
         u1 = 2 * lo + (kpart + 1) * nu / p.ksplit;
     };
-    const int items = (a1 - a0) + nseg * (k1 - k0);                 // ring items before the first U item
-    const int gate = items - S;                                  // the item whose stage the first U item takes (none: negative)
+    // The U items (one per 64-rank block) are spread evenly over the part of the W items that comes after u_start, so that their
+    // preparation runs under the stream; a block of segment s comes after the segment's first W item, which starts the
+    // accumulator.  Every role walks the same order: `u_before(j)` W items come before U block j.
+    const int wtotal = p.y_dense ? 0 : nseg * (k1 - k0);
+    int ucum[LT_MAX_SEG + 1] = {0, 0, 0, 0}, ufirst[LT_MAX_SEG] = {0, 0, 0};
+#pragma unroll
+    for (int s = 0; s < LT_MAX_SEG; ++s) {
+        int u0 = 0, u1 = 0;
+        if (s < nseg) u_range(s, u0, u1);
+        ufirst[s] = u0;
+        ucum[s + 1] = ucum[s] + u1 - u0;
+    }
+    const int ucount = ucum[LT_MAX_SEG];
+    const int u_start = min(p.u_start, wtotal);
+    auto u_seg = [&](int j) { return (j >= ucum[1]) + (j >= ucum[2]); };
+    auto u_block = [&](int j) { return j < ucum[1] ? ufirst[0] + j : (j < ucum[2] ? ufirst[1] + j - ucum[1] : ufirst[2] + j - ucum[2]); };
+    auto u_before = [&](int j) { return min(max(u_start + (j + 1) * (wtotal - u_start) / ucount, u_seg(j) * (k1 - k0) + 1), wtotal); };
 
     if (warp == LT_LOAD_WARP) {
         // ------------------------------------------------------------------ TMA producer
@@ -224,29 +251,37 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                     ph ^= 1;
                 }
             };
+            auto load_x = [&](int kb, uint32_t full) {
+                tma_load_2d(ring + st * stage_bytes + LT_A_BYTES, &maps.x, kb * LT_ITEM, 0, full);
+                tma_load_2d(ring + st * stage_bytes + LT_A_BYTES + x_bytes, &maps.x, kb * LT_ITEM + LT_KB, 0, full);
+            };
             for (int kb = a0; kb < a1; ++kb, next()) {
                 wait_bounded(bar_empty + 8 * st, ph, wctx, 1);
-                mbar_arrive_expect_tx(bar_full + 8 * st, x_bytes);
-                tma_load_2d(ring + st * stage_bytes + LT_A_BYTES, &maps.x, kb * LT_KB, 0, bar_full + 8 * st);
+                mbar_arrive_expect_tx(bar_full + 8 * st, 2 * x_bytes);
+                load_x(kb, bar_full + 8 * st);
             }
             const uint32_t w_bytes = static_cast<uint32_t>(p.rows) * 128u;
-            for (int s = 0; s < nseg; ++s) {
-                const int m0 = slice_row(slice0 + s);
-                for (int kb = k0; kb < k1; ++kb, next()) {
+            int s = 0, kb = k0, m0 = slice_row(slice0), i = 0;
+            for (int j = 0; j <= ucount; ++j) {
+                const int stop = j < ucount ? u_before(j) : wtotal;
+                for (; i < stop; ++i, next()) {
                     const uint32_t sa = ring + st * stage_bytes, full = bar_full + 8 * st;
                     wait_bounded(bar_empty + 8 * st, ph, wctx, 1);
                     mbar_arrive_n(full, LT_UNPACK_WARPS);        // the unpack warps have no part in a W item
-                    mbar_arrive_expect_tx(full, w_bytes + x_bytes);
-                    tma_load_2d(sa, &maps.w, kb * LT_KB, m0, full);
-                    tma_load_2d(sa + LT_A_BYTES, &maps.x, kb * LT_KB, 0, full);
+                    mbar_arrive_expect_tx(full, 2 * (w_bytes + x_bytes));
+                    tma_load_2d(sa, &maps.w, kb * LT_ITEM, m0, full);
+                    tma_load_2d(sa + LT_A_BLOCK, &maps.w, kb * LT_ITEM + LT_KB, m0, full);
+                    load_x(kb, full);
+                    if (++kb == k1) {
+                        kb = k0;
+                        m0 = slice_row(slice0 + ++s);
+                    }
                 }
-            }
-            for (int s = 0; s < nseg; ++s) {
-                int u0, u1;
-                u_range(s, u0, u1);
-                for (int j = 2 * u0; j < 2 * u1; ++j, next()) {
+                if (j < ucount) {                                // everything of a U item is written by the unpack warps, once its stage is free
                     wait_bounded(bar_empty + 8 * st, ph, wctx, 1);
-                    mbar_arrive(bar_full + 8 * st);              // everything of a U item is written by an unpack warp
+                    mbar_arrive(bar_full + 8 * st);
+                    mbar_arrive(bar_slot + 8 * j);
+                    next();
                 }
             }
             // Every CTA checks out once it is past its grid-wide waits; the last one re-arms the counters for the next call.  This
@@ -274,53 +309,47 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
 #pragma unroll
             for (int k = 0; k < 4; ++k) tc_mma_bf16(d, ad + 2 * k, bd + 2 * k, p.idesc, fresh && k == 0 ? 0u : 1u);
         };
-        int it = 0;
-        for (int kb = a0; kb < a1; ++kb, ++it, next()) {
+        // a stage: both blocks of the columns, or (U item) the hi and lo parts of one 64-rank block against the same tile of h
+        auto item = [&](uint32_t d, uint32_t b2, bool fresh) {
+            const uint32_t sa = ring + st * stage_bytes, sb = sa + LT_A_BYTES;
+            mma4(d, sa, sb, fresh);
+            mma4(d, sa + LT_A_BLOCK, sb + b2, false);
+            tc_commit(bar_empty + 8 * st);
+        };
+        for (int kb = a0; kb < a1; ++kb, next()) {
             wait_bounded(bar_full + 8 * st, ph, wctx, 1);
             tc_fence_after();
             if (elect_one()) {
-                mma4(tmem_base, ring + st * stage_bytes, ring + st * stage_bytes + LT_A_BYTES, kb == a0);
-                tc_commit(bar_empty + 8 * st);
-                if (it == gate) tc_commit(bar_gate);
+                item(tmem_base, x_bytes, kb == a0);
                 if (kb == a1 - 1) tc_commit(bar_h);
             }
             __syncwarp();
         }
         LT_STAMP(2);
-        for (int s = 0; s < nseg; ++s) {
-            const uint32_t d = tmem_base + static_cast<uint32_t>(p.tpad) * (1 + s);
-            for (int kb = k0; kb < k1; ++kb, ++it, next()) {
-                const uint32_t sa = ring + st * stage_bytes;
-                wait_bounded(bar_full + 8 * st, ph, wctx, 1);
-                tc_fence_after();
-                if (elect_one()) {
-                    mma4(d, sa, sa + LT_A_BYTES, kb == k0);
-                    tc_commit(bar_empty + 8 * st);
-                    if (it == gate) tc_commit(bar_gate);
+        {
+            uint32_t d = tmem_base + p.tpad;
+            int kb = k0, i = 0;
+            for (int j = 0; j <= ucount; ++j) {
+                const int stop = j < ucount ? u_before(j) : wtotal;
+                for (; i < stop; ++i, next()) {
+                    wait_bounded(bar_full + 8 * st, ph, wctx, 1);
+                    tc_fence_after();
+                    if (elect_one()) item(d, x_bytes, kb == k0);
+                    __syncwarp();
+                    if (++kb == k1) {
+                        kb = k0;
+                        d += p.tpad;
+                    }
                 }
-                __syncwarp();
-            }
-        }
-        LT_STAMP(3);
-        for (int s = 0; s < nseg; ++s) {
-            int u0, u1;
-            u_range(s, u0, u1);
-            const uint32_t d = tmem_base + static_cast<uint32_t>(p.tpad) * (1 + s);
-            for (int j = u0; j < u1; ++j) {                      // two stages per 64-rank block: hi, then lo with hi's B tile
-                const int s_hi = st;
-                wait_bounded(bar_full + 8 * st, ph, wctx, 1);
-                next();
-                wait_bounded(bar_full + 8 * st, ph, wctx, 1);
-                tc_fence_after();
-                if (elect_one()) {
-                    const uint32_t b = ring + s_hi * stage_bytes + LT_A_BYTES;
-                    mma4(d, ring + s_hi * stage_bytes, b, false);
-                    mma4(d, ring + st * stage_bytes, b, false);
-                    tc_commit(bar_empty + 8 * s_hi);
-                    tc_commit(bar_empty + 8 * st);
+                if (i == wtotal && j == 0) LT_STAMP(3);
+                if (j < ucount) {
+                    wait_bounded(bar_full + 8 * st, ph, wctx, 1);
+                    tc_fence_after();
+                    const int us = u_seg(j);
+                    if (elect_one()) item(tmem_base + static_cast<uint32_t>(p.tpad) * (1 + us), 0u, wtotal == 0 && j == ucum[us]);
+                    __syncwarp();
+                    next();
                 }
-                __syncwarp();
-                next();
             }
         }
         LT_STAMP(4);
@@ -337,26 +366,25 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
             uint32_t ph = 1;
             for (int kb = a0; kb < a1; ++kb) {
                 wait_bounded(bar_empty + 8 * st, ph, wctx, 1);
-                const uint32_t cw[4] = {acur.q.x, acur.q.y, acur.q.z, acur.q.w};
-                const uint32_t zw[8] = {acur.z[0].x, acur.z[0].y, acur.z[0].z, acur.z[0].w, acur.z[1].x, acur.z[1].y, acur.z[1].z, acur.z[1].w};
-                const uint32_t dst = ring + st * stage_bytes + static_cast<uint32_t>(row) * 128u;
+                const uint32_t cw[8] = {acur.q[0].x, acur.q[0].y, acur.q[0].z, acur.q[0].w, acur.q[1].x, acur.q[1].y, acur.q[1].z, acur.q[1].w};
+                const uint32_t dst = ring + st * stage_bytes + half * LT_A_BLOCK + static_cast<uint32_t>(row) * 128u;
 #pragma unroll
-                for (int wi = 0; wi < 4; ++wi) {                 // (code - zero) is exact; one rounding in the product
+                for (int wi = 0; wi < 8; ++wi) {                 // (code - zero) is exact; one rounding in the product
                     uint32_t e[4];
                     unpack8_bf16(cw[wi], e);
-                    const uint32_t sw[4] = {acur.s[wi].x, acur.s[wi].y, acur.s[wi].z, acur.s[wi].w};
+                    const uint4 zq = acur.z[wi >> 1];
+                    const uint32_t z0 = (wi & 1) ? zq.z : zq.x, z1 = (wi & 1) ? zq.w : zq.y;
                     uint32_t o[4];
-                    o[0] = bf2_mul(bf2_sub(e[0], __byte_perm(zw[2 * wi], 0x43434343u, 0x4140)), sw[0]);
-                    o[1] = bf2_mul(bf2_sub(e[1], __byte_perm(zw[2 * wi], 0x43434343u, 0x4342)), sw[1]);
-                    o[2] = bf2_mul(bf2_sub(e[2], __byte_perm(zw[2 * wi + 1], 0x43434343u, 0x4140)), sw[2]);
-                    o[3] = bf2_mul(bf2_sub(e[3], __byte_perm(zw[2 * wi + 1], 0x43434343u, 0x4342)), sw[3]);
-                    sts16(dst + (((half * 4 + wi) ^ (row & 7)) << 4), make_uint4(o[0], o[1], o[2], o[3]));
+                    o[0] = bf2_mul(bf2_sub(e[0], __byte_perm(z0, 0x43434343u, 0x4140)), acur.s[wi].x);
+                    o[1] = bf2_mul(bf2_sub(e[1], __byte_perm(z0, 0x43434343u, 0x4342)), acur.s[wi].y);
+                    o[2] = bf2_mul(bf2_sub(e[2], __byte_perm(z1, 0x43434343u, 0x4140)), acur.s[wi].z);
+                    o[3] = bf2_mul(bf2_sub(e[3], __byte_perm(z1, 0x43434343u, 0x4342)), acur.s[wi].w);
+                    sts16(dst + ((wi ^ (row & 7)) << 4), make_uint4(o[0], o[1], o[2], o[3]));
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_full + 8 * st);
-                acur = anxt;
-                if (kb + 2 < a1) fetch_a(anxt, kb + 2);
+                if (kb + 1 < a1) fetch_a(acur, kb + 1);
                 if (++st == S) {
                     st = 0;
                     ph ^= 1;
@@ -383,49 +411,29 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
         }
         LT_STAMP(3);
 
-        // U blocks of this CTA, over its slices, in rounds of up to S / 2; in a round of few blocks several warps share one.  The
-        // codes of the first round do not depend on h and are requested before the waits.
-        int ucount = 0;
-        for (int s = 0; s < nseg; ++s) {
-            int u0, u1;
-            u_range(s, u0, u1);
-            ucount += u1 - u0;
-        }
+        // Operands of the U blocks, one block ahead of their use: 32 codes of one row per thread, and 16-byte pieces of h.
         struct UOp {
-            uint4 q[8];            // 32 codes of rows (lane >> 1) + 16 (usub + wpb i)
-            uint32_t s[8], z[8];
-        } u;
-        int ukb = 0;               // 64-rank block the operands belong to
-        const int urow = lane >> 1, uhalf = lane & 1;
-        auto warps_per_block = [](int count) { return count <= 1 ? 8 : (count <= 2 ? 4 : (count <= 4 ? 2 : 1)); };
-        auto fetch_u = [&](int i, int wpb) {
-            int s = 0, u0 = 0, u1 = 0;
-            for (; s < nseg; ++s) {
-                u_range(s, u0, u1);
-                if (i < u1 - u0) break;
-                i -= u1 - u0;
-            }
-            ukb = u0 + i;
-            const int m0 = slice_row(slice0 + s), m1 = slice_row(slice0 + s + 1), usub = warp & (wpb - 1);
+            uint4 q;
+            uint32_t s, z;
+        } u, un;
+        auto fetch_u = [&](UOp& o, int j) {
+            const int s = slice0 + u_seg(j), kb = u_block(j);
+            const int m = min(slice_row(s) + row, slice_row(s + 1) - 1);              // rows past the slice: any values, never stored
+            o.q = ldg16_stream(p.uq + static_cast<size_t>(m) * (r >> 1) + half * 16 + kb * 32);
+            o.s = p.us[static_cast<size_t>(m) * ng + (kb >> 1)];
+            o.z = p.uz[static_cast<size_t>(m) * ng + (kb >> 1)];
+        };
+        auto fetch_h = [&](uint4 (&o)[4], int j) {
+            const __nv_bfloat16* src = p.h + u_block(j) * 64 + (tid & 7) * 8;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int rk = 16 * (usub + wpb * k);
-                if (rk < p.rows) {
-                    const int m = min(m0 + urow + rk, m1 - 1);               // rows past the slice: any values, never stored
-                    u.q[k] = ldg16_stream(p.uq + static_cast<size_t>(m) * (r >> 1) + uhalf * 16 + ukb * 32);
-                    u.s[k] = p.us[static_cast<size_t>(m) * ng + (ukb >> 1)];
-                    u.z[k] = p.uz[static_cast<size_t>(m) * ng + (ukb >> 1)];
-                }
-            }
+            for (int i = 0; i < 4; ++i)
+                if ((tid >> 3) + 32 * i < T) o[i] = ldcg16(src + static_cast<size_t>((tid >> 3) + 32 * i) * r);
         };
 
         unpack_sync();
         if (tid == 0 && a0 < a1 && !p.drop_arrivals) red_release_gpu_add(p.sync, 1u);
-        {
-            // after the release: the fence in it would wait for these loads too
-            const int count = min(ucount, S >> 1), wpb = warps_per_block(count);
-            if (warp / wpb < count) fetch_u(warp / wpb, wpb);
-        }
+        const bool by_warp = p.y_dense && T <= 64;
+        if (!by_warp && ucount > 0) fetch_u(u, 0);                           // after the release: the fence in it would wait for these loads too
         if (tid == 0) lt_wait_count(p.sync, static_cast<unsigned int>(ng * p.hparts), p, abort_flag);
         unpack_sync();
         LT_STAMP(4);
@@ -479,45 +487,86 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
         unpack_sync();
         LT_STAMP(6);
 
-        // ---- U items.  The W items in between were not this role's business; a wait tells the phases of a barrier apart by their
-        // parity only, so before it joins the ring again it waits until the item that used the first U stage before has retired
-        // (items retire in order: every stage is then at most one phase behind).  For the same reason blocks go in rounds of
-        // S / 2, one use of every stage each, with a barrier of the role between rounds.
-        if (ucount > 0 && gate >= 0) wait_bounded(bar_gate, 0, wctx, 1);
-        LT_STAMP(7);
-        for (int first = 0; first < ucount; first += S >> 1) {
-            if (first > 0) unpack_sync();
-            const int count = min(ucount - first, S >> 1), wpb = warps_per_block(count);
-            const int i = first + warp / wpb;
-            if (i < first + count) {
-                const int usub = warp & (wpb - 1);
-                if (first > 0) fetch_u(i, wpb);
-                const int idx = items + 2 * i, use = idx / S, st = idx - use * S, idx2 = idx + 1, use2 = idx2 / S, st2 = idx2 - use2 * S;
-                wait_bounded(bar_empty + 8 * st, (use & 1) ^ 1, wctx, 1);
-                wait_bounded(bar_empty + 8 * st2, (use2 & 1) ^ 1, wctx, 1);
-                // B tile: h of 64 ranks, 16-byte pieces, eight round trips in flight per lane
-                const uint32_t hb = ring + st * stage_bytes + LT_A_BYTES;
-                for (int tb = 4 * usub; tb < T; tb += 32 * wpb) {
+        // ---- U items.  The load warp, which follows the ring item by item, says when a block's stage is free (one barrier per block: a
+        // wait of this role's own on bar_empty could take an older phase of the same parity for the right one).
+        if (by_warp) {
+            // Nothing streams beside them, slices are short and h is small: a warp per block, so that the blocks' round trips for h
+            // overlap (4096 x 4096 r = 512, this launch at T = 17 22.0 -> 17.7 us; from 65 tokens up one warp's share of h takes longer
+            // than the round trips, T = 100 26.3 -> 29.4).
+            for (int j = warp; j < ucount; j += LT_UNPACK_WARPS) {
+                const int s = slice0 + u_seg(j), kb = u_block(j), m0 = slice_row(s), m1 = slice_row(s + 1);
+                uint4 q8[8];
+                uint32_t s8[8], z8[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (16 * k < p.rows) {
+                        const int m = min(m0 + (lane >> 1) + 16 * k, m1 - 1);          // rows past the slice: any values, never stored
+                        q8[k] = ldg16_stream(p.uq + static_cast<size_t>(m) * (r >> 1) + (lane & 1) * 16 + kb * 32);
+                        s8[k] = p.us[static_cast<size_t>(m) * ng + (kb >> 1)];
+                        z8[k] = p.uz[static_cast<size_t>(m) * ng + (kb >> 1)];
+                    }
+                const int us = ((a1 - a0) + j) % S;
+                const uint32_t ua = ring + us * stage_bytes, hb = ua + LT_A_BYTES;
+                wait_bounded(bar_slot + 8 * j, 0, wctx, 1);
+                for (int tb = 0; tb < T; tb += 32) {
                     uint4 hv[8];
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
-                        const int t = tb + (lane >> 3) + 4 * wpb * k;
-                        if (t < T) hv[k] = ldcg16(p.h + static_cast<size_t>(t) * r + ukb * 64 + (lane & 7) * 8);
+                        const int t = tb + (lane >> 3) + 4 * k;
+                        if (t < T) hv[k] = ldcg16(p.h + static_cast<size_t>(t) * r + kb * 64 + (lane & 7) * 8);
                     }
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
-                        const int t = tb + (lane >> 3) + 4 * wpb * k;
+                        const int t = tb + (lane >> 3) + 4 * k;
                         if (t < T) sts16(hb + t * 128 + (((lane & 7) ^ (t & 7)) << 4), hv[k]);
                     }
                 }
-                const uint32_t d_hi = ring + st * stage_bytes, d_lo = ring + st2 * stage_bytes;
 #pragma unroll
                 for (int k8 = 0; k8 < 8; ++k8) {
-                    const int rk = 16 * (usub + wpb * k8);
-                    if (rk >= p.rows) break;
-                    const int ur = urow + rk;
-                    const uint32_t zz = kBf2_128 | u.z[k8] | (u.z[k8] << 16), s2 = u.s[k8] | (u.s[k8] << 16);
-                    const uint32_t cw[4] = {u.q[k8].x, u.q[k8].y, u.q[k8].z, u.q[k8].w};
+                    if (16 * k8 >= p.rows) break;
+                    const int ur = (lane >> 1) + 16 * k8;
+                    const uint32_t zz = kBf2_128 | z8[k8] | (z8[k8] << 16), s2 = s8[k8] | (s8[k8] << 16);
+                    const uint32_t cw[4] = {q8[k8].x, q8[k8].y, q8[k8].z, q8[k8].w};
+#pragma unroll
+                    for (int wi = 0; wi < 4; ++wi) {
+                        uint32_t e[4], hi[4], lo[4];
+                        unpack8_bf16(cw[wi], e);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t dz = bf2_sub(e[k], zz);           // as below
+                            hi[k] = bf2_mul(dz, s2);
+                            lo[k] = bf2_fma(dz, s2, hi[k] ^ 0x80008000u);
+                        }
+                        const uint32_t off = ur * 128 + ((((lane & 1) * 4 + wi) ^ (ur & 7)) << 4);
+                        sts16(ua + off, make_uint4(hi[0], hi[1], hi[2], hi[3]));
+                        sts16(ua + LT_A_BLOCK + off, make_uint4(lo[0], lo[1], lo[2], lo[3]));
+                    }
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_n(bar_full + 8 * us, LT_UNPACK_WARPS);          // one warp for all eight
+            }
+        } else {
+            // All eight warps on each block, operands one block ahead.
+            uint4 hc[4], hn[4];
+            if (ucount > 0) fetch_h(hc, 0);
+            LT_STAMP(7);
+            for (int j = 0; j < ucount; ++j) {
+                if (j + 1 < ucount) {
+                    fetch_u(un, j + 1);
+                    fetch_h(hn, j + 1);
+                }
+                const int us = ((a1 - a0) + u_before(j) + j) % S;      // the block's stage
+                wait_bounded(bar_slot + 8 * j, 0, wctx, 1);
+                const uint32_t ua = ring + us * stage_bytes, hb = ua + LT_A_BYTES;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {                    // B tile: h of 64 ranks
+                    const int t = (tid >> 3) + 32 * i, k8 = tid & 7;
+                    if (t < T) sts16(hb + t * 128 + ((k8 ^ (t & 7)) << 4), hc[i]);
+                }
+                if (row < p.rows) {
+                    const uint32_t zz = kBf2_128 | u.z | (u.z << 16), s2 = u.s | (u.s << 16);
+                    const uint32_t cw[4] = {u.q.x, u.q.y, u.q.z, u.q.w};
 #pragma unroll
                     for (int wi = 0; wi < 4; ++wi) {
                         uint32_t e[4], hi[4], lo[4];
@@ -528,42 +577,61 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                             hi[k] = bf2_mul(dz, s2);                         // the product's upper 8 bits
                             lo[k] = bf2_fma(dz, s2, hi[k] ^ 0x80008000u);    // the rest of its 12, exact
                         }
-                        const uint32_t off = ur * 128 + (((uhalf * 4 + wi) ^ (ur & 7)) << 4);
-                        sts16(d_hi + off, make_uint4(hi[0], hi[1], hi[2], hi[3]));
-                        sts16(d_lo + off, make_uint4(lo[0], lo[1], lo[2], lo[3]));
+                        const uint32_t off = row * 128 + (((half * 4 + wi) ^ (row & 7)) << 4);
+                        sts16(ua + off, make_uint4(hi[0], hi[1], hi[2], hi[3]));
+                        sts16(ua + LT_A_BLOCK + off, make_uint4(lo[0], lo[1], lo[2], lo[3]));
                     }
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) {                                 // the wpb warps of an item arrive for all eight
-                    mbar_arrive_n(bar_full + 8 * st, LT_UNPACK_WARPS / wpb);
-                    mbar_arrive_n(bar_full + 8 * st2, LT_UNPACK_WARPS / wpb);
-                }
+                if (lane == 0) mbar_arrive(bar_full + 8 * us);
+                u = un;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) hc[i] = hn[i];
             }
         }
         LT_STAMP(8);
 
         // ---- epilogue
-        if (nseg > 0) {
-            wait_bounded(bar_done, 0, wctx, 1);
-            tc_fence_after();
-        }
-        LT_STAMP(9);
         if (p.ksplit == 1) {
             for (int s = 0; s < nseg; ++s) {
                 const int m = slice_row(slice0 + s) + rr;
-                if (q * 32 >= p.rows) break;                     // uniform in the warp
                 const bool live = m < slice_row(slice0 + s + 1);
-                for (int c0 = hcol * 16; c0 < p.tpad; c0 += 32) {
+                uint32_t y[4][16];                               // base term, requested before the last products are waited for
+                if (p.y_dense) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const int t = hcol * 16 + 32 * k + i;
+                            y[k][i] = live && t < T ? static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(p.y_dense) + static_cast<size_t>(t) * M + m)) : 0u;
+                        }
+                }
+                if (s == 0) {
+                    wait_bounded(bar_done, 0, wctx, 1);
+                    tc_fence_after();
+                    LT_STAMP(9);
+                }
+                if (q * 32 >= p.rows) continue;                  // uniform in the warp
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int c0 = hcol * 16 + 32 * k;
+                    if (c0 >= p.tpad) break;
                     uint32_t v[16];
                     tmem_ld16_sync(lane_addr + static_cast<uint32_t>(p.tpad) * (1 + s) + c0, v);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (live && c0 + i < T) p.out[static_cast<size_t>(c0 + i) * M + m] = __float2bfloat16_rn(__uint_as_float(v[i]));
+                    for (int i = 0; i < 16; ++i) {
+                        float o = __uint_as_float(v[i]);
+                        if (p.y_dense) o += __uint_as_float(y[k][i] << 16);
+                        if (live && c0 + i < T) p.out[static_cast<size_t>(c0 + i) * M + m] = __float2bfloat16_rn(o);
+                    }
                 }
             }
         } else if (nseg > 0) {
             // ksplit CTAs hold partial sums of the slice: each finishes an equal share of the tokens, [t0, t1)
+            wait_bounded(bar_done, 0, wctx, 1);
+            tc_fence_after();
+            LT_STAMP(9);
             const int n = p.ksplit, t0 = kpart * T / n, t1 = (kpart + 1) * T / n;
             const uint32_t piece = static_cast<uint32_t>(t1 - t0) * 512u, acc = lane_addr + p.tpad;
             for (int c0 = hcol * 16; c0 < p.tpad; c0 += 32) {
@@ -622,28 +690,29 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
 
 // How a launch is cut: see the note at the top.
 struct LinearSplit {
-    int slices, segs, ksplit, rows, stages;
+    int slices, segs, ksplit, rows, stages, u_start;
     uint32_t ring_bytes;
 };
 constexpr int kLtRingMax = 232448 - LT_SMEM_FIXED;
 
 // Cost in microseconds of `ksplit` CTAs per slice, as far as the choice depends on it: the bytes an SM takes in (its weights
-// once, x for its columns; 83 GB/s per SM measured with all SMs streaming), the MMAs (a 64-column block takes about 0.2 us
+// once, x for its columns; 83 GB/s per SM measured with all SMs streaming), the MMAs (a 64-column block takes about 0.17 us
 // whatever the height of the slice: the tensor core reads 128 rows) and the exchange of partial sums.
 inline double linear_split_cost(int M, int N, int T, int grid, int ksplit) {
     const int slices = grid / ksplit;
     const double rows = (M + slices - 1) / slices;
     const double ingest = (rows + T) * 2.0 * N / ksplit / 83e3;
-    const double mma = 0.2 * N / LT_KB / ksplit;
+    const double mma = 0.17 * N / LT_KB / ksplit;
     return (ingest > mma ? ingest : mma) + (ksplit > 1 ? 3.0 + 2.0 * T * rows * 4.0 / 83e3 : 0.0);
 }
-inline bool linear_split(int M, int N, int T, int tpad, int grid, LinearSplit& out) {
-    const int kbs = N / LT_KB;
+// `stream`: W_b is streamed; without it there is nothing to split over the columns.
+inline bool linear_split(int M, int N, int T, int tpad, int grid, bool stream, LinearSplit& out) {
+    const int kbs = N / LT_ITEM;
     LinearSplit s = {};
     s.ksplit = 1;
     s.segs = (M + LT_TILE * grid - 1) / (LT_TILE * grid);
     if (s.segs > LT_MAX_SEG) return false;
-    if (s.segs == 1) {
+    if (s.segs == 1 && stream) {
         double best = linear_split_cost(M, N, T, grid, 1);
         for (int k = 2; k <= kbs && k <= grid; ++k) {
             const int slices = grid / k;
@@ -658,10 +727,13 @@ inline bool linear_split(int M, int N, int T, int tpad, int grid, LinearSplit& o
     s.slices = grid / s.ksplit * s.segs;
     if (s.slices > M) s.slices = M;
     s.rows = (M + s.slices - 1) / s.slices;
-    const int stage = LT_A_BYTES + tpad * 128;
+    const int stage = LT_A_BYTES + 2 * tpad * 128;
     s.stages = kLtRingMax / stage;
     if (s.stages > LT_MAX_STAGES) s.stages = LT_MAX_STAGES;
-    s.stages &= ~1;
+    // h is there after about 10 us (two grid-wide hand-overs; more with more of it to add up); by then an SM has streamed this many items
+    // (its share of 6.4 TB/s, or 0.34 us each).  U items that come up earlier would hold the stream up.
+    const double item = s.rows * 256.0 * grid / 6.4e6 > 0.34 ? s.rows * 256.0 * grid / 6.4e6 : 0.34;
+    s.u_start = static_cast<int>((10.0 + 0.04 * T) / item) + 1;
     int ring = s.stages * stage;
     const int fix = s.ksplit > 1 ? 512 * (T + s.ksplit) : 0;      // n pieces of ceil(T / n) token rows at most
     if (ring < fix) ring = (fix + 1023) & ~1023;

@@ -4,7 +4,7 @@
 // but contains no kernel: everything it does is fill an ade_delta_t and call libade_b200.so.
 //
 //   torch.ops.ade_b200.factored(x, weight?, y_dense?, uq, vq, vt, us, uz, vs, vz, M, N, r, blocks, scratch) -> out
-//   torch.ops.ade_b200.linear(x, weight, uq, vq, vt, us, uz, vs, vz, M, N, r, blocks, scratch) -> out
+//   torch.ops.ade_b200.linear(as factored) -> out
 //   torch.ops.ade_b200.recon(base, uq, vq, vt, us, uz, vs, vz, M, N, r, dbg_acc?, status?, u8?, v8?) -> merged
 //   torch.ops.ade_b200.expand / expand_f8(uq, vq, vt, us, uz, vs, vz, M, N, r) -> (u8, v8)
 //
@@ -69,6 +69,9 @@ ade_delta_t make_delta(const at::Tensor& uq, const at::Tensor& vq, const at::Ten
     return d;
 }
 
+// TC: the tensor-core kernel (ade_b200_linear) in any case, else where it is preferred for a call with y_dense; its workspace comes from torch's caching allocator (stream-ordered, so calls on other
+// streams and graph captures get memory of their own).
+template <bool TC>
 at::Tensor factored(const at::Tensor& x, const c10::optional<at::Tensor>& weight, const c10::optional<at::Tensor>& y_dense,
                     const at::Tensor& uq, const at::Tensor& vq, const at::Tensor& vt, const at::Tensor& us, const at::Tensor& uz,
                     const at::Tensor& vs, const at::Tensor& vz, int64_t M, int64_t N, int64_t r, at::IntArrayRef blocks,
@@ -89,35 +92,20 @@ at::Tensor factored(const at::Tensor& x, const c10::optional<at::Tensor>& weight
     const c10::cuda::CUDAGuard guard(x.device());
     const ade_delta_t d = make_delta(uq, vq, vt, us, uz, vs, vz, M, N, r, blocks, x);
     at::Tensor out = at::empty({T, M}, x.options());
-    const int rc = ade_b200_factored(&d, x.data_ptr(), y_dense.has_value() ? y_dense->data_ptr() : nullptr,
-                                     weight.has_value() ? weight->data_ptr() : nullptr, out.data_ptr(), scratch.data_ptr(),
-                                     static_cast<size_t>(scratch.nbytes()), static_cast<int>(T),
-                                     c10::cuda::getCurrentCUDAStream(x.get_device()).stream());
-    TORCH_CHECK(rc == ADE_OK, "ade_b200_factored: ", err_name(rc), rc == ADE_ERR_CUDA ? " (cudaError " : "",
-                rc == ADE_ERR_CUDA ? std::to_string(ade_b200_last_cuda_error()) + ")" : std::string());
-    return out;
-}
-
-// One delta linear module, base GEMM included, through the tensor-core kernel; the workspace comes from torch's caching allocator
-// (stream-ordered, so calls on other streams and graph captures get memory of their own).
-at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const at::Tensor& uq, const at::Tensor& vq, const at::Tensor& vt,
-                  const at::Tensor& us, const at::Tensor& uz, const at::Tensor& vs, const at::Tensor& vz, int64_t M, int64_t N, int64_t r,
-                  at::IntArrayRef blocks, const at::Tensor& scratch) {
-    TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.is_contiguous() && x.size(1) == N,
-                "x must be a contiguous CUDA bfloat16 tensor of shape (T, ", N, ")");
-    TORCH_CHECK(weight.scalar_type() == at::kBFloat16 && weight.is_contiguous() && weight.dim() == 2 && weight.size(0) == M &&
-                    weight.size(1) == N && weight.device() == x.device(),
-                "weight must be a contiguous bfloat16 (d_o, d_i) tensor on x's device");
-    TORCH_CHECK(scratch.is_cuda() && scratch.device() == x.device() && scratch.is_contiguous(), "scratch must be a CUDA buffer on x's device");
-    const int T = static_cast<int>(x.size(0));
-    const c10::cuda::CUDAGuard guard(x.device());
-    const ade_delta_t d = make_delta(uq, vq, vt, us, uz, vs, vz, M, N, r, blocks, x);
-    at::Tensor out = at::empty({x.size(0), M}, x.options());
-    const size_t wbytes = ade_b200_linear_workspace_bytes(T, d.M, d.r);
-    at::Tensor work = at::empty({static_cast<int64_t>(wbytes)}, x.options().dtype(at::kByte));
-    const int rc = ade_b200_linear(&d, x.data_ptr(), weight.data_ptr(), out.data_ptr(), scratch.data_ptr(), static_cast<size_t>(scratch.nbytes()),
-                                   work.data_ptr(), wbytes, T, c10::cuda::getCurrentCUDAStream(x.get_device()).stream());
-    TORCH_CHECK(rc == ADE_OK, "ade_b200_linear: ", err_name(rc), rc == ADE_ERR_CUDA ? " (cudaError " : "",
+    const void* yd = y_dense.has_value() ? y_dense->data_ptr() : nullptr;
+    const void* wb = weight.has_value() ? weight->data_ptr() : nullptr;
+    void* stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
+    int rc;
+    if (TC || (yd && ade_b200_linear_preferred(static_cast<int>(T), d.M, d.r))) {
+        const size_t wbytes = ade_b200_linear_workspace_bytes(static_cast<int>(T), d.M, d.r);
+        const at::Tensor work = at::empty({static_cast<int64_t>(wbytes)}, x.options().dtype(at::kByte));
+        rc = ade_b200_linear(&d, x.data_ptr(), yd, wb, out.data_ptr(), scratch.data_ptr(), static_cast<size_t>(scratch.nbytes()), work.data_ptr(),
+                             wbytes, static_cast<int>(T), stream);
+    } else {
+        rc = ade_b200_factored(&d, x.data_ptr(), yd, wb, out.data_ptr(), scratch.data_ptr(), static_cast<size_t>(scratch.nbytes()),
+                               static_cast<int>(T), stream);
+    }
+    TORCH_CHECK(rc == ADE_OK, TC ? "ade_b200_linear: " : "ade_b200_factored: ", err_name(rc), rc == ADE_ERR_CUDA ? " (cudaError " : "",
                 rc == ADE_ERR_CUDA ? std::to_string(ade_b200_last_cuda_error()) + ")" : std::string());
     return out;
 }
@@ -194,7 +182,7 @@ std::tuple<at::Tensor, at::Tensor> expand(const at::Tensor& uq, const at::Tensor
 TORCH_LIBRARY(ade_b200, m) {
     m.def("factored(Tensor x, Tensor? weight, Tensor? y_dense, Tensor uq, Tensor vq, Tensor vt, Tensor us, Tensor uz, Tensor vs, Tensor vz, "
           "int M, int N, int r, int[] blocks, Tensor scratch) -> Tensor");
-    m.def("linear(Tensor x, Tensor weight, Tensor uq, Tensor vq, Tensor vt, Tensor us, Tensor uz, Tensor vs, Tensor vz, "
+    m.def("linear(Tensor x, Tensor? weight, Tensor? y_dense, Tensor uq, Tensor vq, Tensor vt, Tensor us, Tensor uz, Tensor vs, Tensor vz, "
           "int M, int N, int r, int[] blocks, Tensor scratch) -> Tensor");
     m.def("recon(Tensor base, Tensor uq, Tensor vq, Tensor vt, Tensor us, Tensor uz, Tensor vs, Tensor vz, int M, int N, int r, "
           "Tensor? dbg_acc, Tensor? status, Tensor? u8, Tensor? v8) -> Tensor");
@@ -203,8 +191,8 @@ TORCH_LIBRARY(ade_b200, m) {
 }
 
 TORCH_LIBRARY_IMPL(ade_b200, CUDA, m) {
-    m.impl("factored", &factored);
-    m.impl("linear", &linear);
+    m.impl("factored", &factored<false>);
+    m.impl("linear", &factored<true>);
     m.impl("recon", &recon);
     m.impl("expand", &expand<false>);
     m.impl("expand_f8", &expand<true>);

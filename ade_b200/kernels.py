@@ -187,7 +187,7 @@ _NULL = contextlib.nullcontext()
 
 def _on_device(dev: torch.device):
     """Device guard for a launch; free when `dev` is already current (the guard costs ~10 us of host time)."""
-    return _NULL if dev.index is None or dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
+    return _NULL if dev.index is None or dev.index == torch._C._cuda_getDevice() else torch.cuda.device(dev)
 
 
 _scratch: dict = {}
@@ -247,14 +247,10 @@ def _check_x(x: torch.Tensor, N: int, what: str):
                          f"{tuple(x.shape)} {x.dtype} on {x.device}")
 
 
-def factored_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor | None = None,
-                     y_dense: torch.Tensor | None = None) -> torch.Tensor:
-    """out = base + U^(V^T x) for T <= 128 tokens; base = x W_b^T computed in-kernel when `weight`
-    is given, else the supplied `y_dense`.  One call of ``ade_b200_factored``."""
-    lib = _lib.load()
-    M, N, r = int(p4["M"]), int(p4["N"]), int(p4["r"])
+def _check_module_args(x, p4, weight, y_dense):
+    """What the two entry points below refuse, with a message of its own for each."""
+    M, N = int(p4["M"]), int(p4["N"])
     _check_x(x, N, "x")
-    T = x.shape[0]
     if (weight is None) == (y_dense is None):
         raise ValueError("give exactly one of weight (fused base GEMM) or y_dense")
     if weight is not None and not (weight.dtype == torch.bfloat16 and weight.is_contiguous()
@@ -262,48 +258,66 @@ def factored_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor | None = No
         raise ValueError("weight must be a contiguous bfloat16 (d_o, d_i) tensor on x's device")
     if y_dense is not None:
         _check_x(y_dense, M, "y_dense")
-        if y_dense.shape[0] != T:
+        if y_dense.shape[0] != x.shape[0]:
             raise ValueError("y_dense and x disagree on T")
-    with _on_device(x.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        scratch = _scratch_for(x.device, stream, T, r, lib.ade_b200_factored_scratch_bytes(T, r))
-        # through the torch binding: it allocates the output, takes torch's current stream and calls ade_b200_factored
+
+
+def _launch(op, x, p4, weight, y_dense):
+    """One launch through the torch binding, which allocates the output, takes torch's current stream and checks dtypes, shapes,
+    strides and devices itself; a refusal is put into words by the checks above (which would cost every call several
+    microseconds of host time here)."""
+    if not x.is_cuda or x.dim() != 2 or (weight is None) == (y_dense is None):
+        _check_module_args(x, p4, weight, y_dense)
+    dev = x.device
+    r, T = p4["r"], x.shape[0]
+    with _on_device(dev):
+        stream = torch._C._cuda_getCurrentRawStream(dev.index)
+        scratch = _scratch.get((dev.index, stream, T, r))
+        if scratch is None:
+            _check_module_args(x, p4, weight, y_dense)
+            scratch = _scratch_for(dev, stream, T, r, _lib.load().ade_b200_factored_scratch_bytes(T, r))
         try:
-            return _lib.ops().factored(x, weight, y_dense, p4["uq"], p4["vq"], p4["vt"], p4["us"], p4["uz"], p4["vs"], p4["vz"],
-                                       M, N, r, _flat_blocks(p4), scratch)
+            return op(x, weight, y_dense, p4["uq"], p4["vq"], p4["vt"], p4["us"], p4["uz"], p4["vs"], p4["vz"], p4["M"], p4["N"], r,
+                      _flat_blocks(p4), scratch)
         except RuntimeError as e:
+            _check_module_args(x, p4, weight, y_dense)
             raise _kernel_error(e) from None
+
+
+def factored_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor | None = None,
+                     y_dense: torch.Tensor | None = None) -> torch.Tensor:
+    """out = base + U^(V^T x) for T <= 128 tokens; base = x W_b^T computed in-kernel when `weight`
+    is given, else the supplied `y_dense`.  One launch: ``ade_b200_factored``, or with `y_dense` ``ade_b200_linear`` where
+    ``ade_b200_linear_preferred`` says so."""
+    return _launch(_lib.ops().factored, x, p4, weight, y_dense)
 
 
 def linear_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor) -> torch.Tensor:
-    """out = x W_b^T + U^(V^T x) for T <= 128 tokens with every contraction on the tensor cores, one call of
-    ``ade_b200_linear`` (replaces the library GEMM + kernels A and B of src/serving.py:106-111)."""
-    lib = _lib.load()
-    M, N, r = int(p4["M"]), int(p4["N"]), int(p4["r"])
-    _check_x(x, N, "x")
-    T = x.shape[0]
-    if not (weight.dtype == torch.bfloat16 and weight.is_contiguous() and tuple(weight.shape) == (M, N) and weight.device == x.device):
-        raise ValueError("weight must be a contiguous bfloat16 (d_o, d_i) tensor on x's device")
-    with _on_device(x.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        scratch = _scratch_for(x.device, stream, T, r, lib.ade_b200_factored_scratch_bytes(T, r))
-        try:
-            return _lib.ops().linear(x, weight, p4["uq"], p4["vq"], p4["vt"], p4["us"], p4["uz"], p4["vs"], p4["vz"],
-                                     M, N, r, _flat_blocks(p4), scratch)
-        except RuntimeError as e:
-            raise _kernel_error(e) from None
+    """out = x W_b^T + U^(V^T x) for T <= 128 tokens with every contraction on the tensor cores in one launch of ``ade_b200_linear``.
+    Modules use it for tall groups at 9-16 tokens only: above 16 their result is defined by the reference's split, whose base
+    term is rounded to bfloat16 by the library GEMM.  This one keeps the base term in float32 and is faster (4096 x 4096 r = 512
+    T = 40 19.9 us against 27.3 for the split, 4096 x 11008 T = 100 29.8 / 50.6)."""
+    return _launch(_lib.ops().linear, x, p4, weight, None)
 
 
-# Up to this many tokens the warp-MMA kernel of `factored_forward` serves a module, above it the tensor-core kernel of
-# `linear_forward`.  Per call on B200, in a graph over rotated weights, factored / linear: 4096 x 4096 r = 512 T = 8 11.7 / 17,
-# T = 16 13.8 / 17.6; 11008 x 4096 T = 8 21.9 / 27, T = 16 28.5 / 28; above 16 tokens the former used a library GEMM for the base
-# term: 4096 x 4096 T = 40 27.7 / 18.8, 4096 x 11008 T = 100 63.8 / 30.3, 5000 x 5120 r = 896 T = 40 45.9 / 25.0 us.
-FACTORED_MAX_TOKENS = 16
+# Up to this many tokens the base GEMM runs in the launch of the delta: the warp-MMA kernel (`ade_b200_factored`), or for modules of
+# TALL_ROWS rows and more (the fused gate/up groups) above 8 tokens the tensor-core kernel (`ade_b200_linear`), because the former no
+# longer hides U^ h under its stream there.  Per call on B200 in a graph over rotated weights, former / latter in us: 22016 x 4096 T = 8
+# 36.9 / 48.3, T = 16 62.5 / 49.1; 27648 x 5120 T = 16 86.2 / 59.9; 12288 x 4096 (q/k/v) T = 16 41.7 / 42.7; 4096 x 4096 T = 16 13.9 / 18.3.
+FUSED_MAX_TOKENS = 16
+TALL_ROWS = 16384
+TALL_FACTORED_MAX_TOKENS = 8
 
 
 def module_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor) -> torch.Tensor:
-    """x W_b^T + U^(V^T x) of one module for T <= 128 tokens, by the kernel that is faster at T."""
-    return factored_forward(x, p4, weight=weight) if x.shape[0] <= FACTORED_MAX_TOKENS else linear_forward(x, p4, weight)
+    """x W_b^T + U^(V^T x) of one module (up to FUSED_MAX_TOKENS tokens also of a fused group) for T <= 128 tokens.  Above that the
+    reference's own split (src/serving.py:106-111): library GEMM for the base term, kernel for the delta."""
+    T = x.shape[0]
+    if T > FUSED_MAX_TOKENS:
+        return decode_forward_packed(x, torch.nn.functional.linear(x, weight), p4)
+    if T > TALL_FACTORED_MAX_TOKENS and weight.shape[0] >= TALL_ROWS:
+        return linear_forward(x, p4, weight)
+    return factored_forward(x, p4, weight=weight)
 
 
 def _kernel_error(e: RuntimeError) -> Exception:

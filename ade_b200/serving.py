@@ -4,8 +4,8 @@ Keeps the API of the reference's ``src/serving.py`` -- ``ADEKernelLinear(W_b, pa
 decode_max_tokens, use_decode, use_recon, split_k)`` with ``forward(x)`` and the attributes
 ``out_features / in_features / weight``, and ``build_kernel_model`` -- on top of the B200 kernels.
 Differences: tensors are bfloat16 (the reference module is float16), there is no float
-fallback (``use_decode`` / ``use_recon`` = False raise), and for T <= decode_max_tokens the base
-GEMM x W_b^T runs in the same launch as the delta instead of a separate ``F.linear``.
+fallback (``use_decode`` / ``use_recon`` = False raise), and up to 16 tokens the base GEMM x W_b^T
+runs in the same launch as the delta instead of a separate ``F.linear``.
 """
 from __future__ import annotations
 
@@ -13,7 +13,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .kernels import (GROUP, STORED_KEYS, decode_kernel_status, expand_codes_f8, module_forward, pack_int4, recon_int4,
+from .kernels import (FUSED_MAX_TOKENS, GROUP, STORED_KEYS, decode_kernel_status, expand_codes_f8, module_forward, pack_int4, recon_int4,
                       recon_kernel_status)
 
 # Modules keep 8-bit operands for the reconstructed path once they have served a long input (see ADEKernelLinear._expanded).
@@ -70,7 +70,7 @@ class ADEKernelLinear(nn.Module):
 
     def _stored_form(self) -> dict:
         """Stored form on the module's device (rebuilt after .to(device))."""
-        if self._p4 is None or self._p4["uq"].data_ptr() != self.p4_uq.data_ptr():
+        if self._p4 is None or self._p4["uq"].data_ptr() != self._buffers["p4_uq"].data_ptr():
             self._p4 = {k: getattr(self, f"p4_{k}") for k in STORED_KEYS}
             self._p4["M"], self._p4["N"], self._p4["r"] = self._dims
         return self._p4
@@ -92,17 +92,18 @@ class ADEKernelLinear(nn.Module):
     def forward(self, x):
         """x (..., d_i) -> (..., d_o) in bfloat16."""
         shape = x.shape
-        x2 = x.reshape(-1, shape[-1]).to(torch.bfloat16).contiguous()
+        plain = len(shape) == 2 and x.dtype is torch.bfloat16 and x.is_contiguous()
+        x2 = x if plain else x.reshape(-1, shape[-1]).to(torch.bfloat16).contiguous()
         T = x2.shape[0]
         if T == 0:
             return x2.new_empty(*shape[:-1], self.out_features)
         if T <= self.decode_max_tokens:
-            y = self._group[0].apply(self._group[1], x, x2) if self._group is not None else None
+            y = self._group[0].apply(self._group[1], x, x2) if self._group is not None and T <= FUSED_MAX_TOKENS else None
             if y is None:
-                y = module_forward(x2, self._stored_form(), self.weight)
+                y = module_forward(x2, self._stored_form(), self._buffers["weight"])
         else:
             y = F.linear(x2, self.merged_weight())
-        return y.reshape(*shape[:-1], self.out_features)
+        return y if plain else y.reshape(*shape[:-1], self.out_features)
 
 
 class FusedADEGroup:

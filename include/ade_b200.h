@@ -172,15 +172,18 @@ int ade_b200_factored(const ade_delta_t* d, const void* x, const void* y_dense, 
                       void* out, void* scratch, size_t scratch_bytes, int T, void* stream);
 
 /*
- * One delta linear module, out = x W_b^T + U^ (V^T x), for 1..128 token rows in one launch with every contraction on the
- * tensor cores (the reference's F.linear + kernels A and B, src/serving.py:106-111).  Arguments as ade_b200_factored
- * with w_b; the same scratch buffer serves both (h, sync words, status word).
+ * One delta linear module for 1..128 token rows in one launch with every contraction on the tensor cores.  Arguments as
+ * ade_b200_factored: out = x W_b^T + U^ (V^T x) with w_b (the reference's F.linear + kernels A and B, src/serving.py:106-111), or
+ * out = y_dense + U^ (V^T x) with y_dense (its kernels A and B); the same scratch buffer serves all (h, sync words, status word).
  *   workspace: device buffer of at least ade_b200_linear_workspace_bytes(T, M, r) bytes for partial sums; its contents need no
  *   preparation and are undefined afterwards.  It must not be in use by another launch at the same time.
- * d->M up to 256 rows per SM of the device (37888 on 148 SMs).  The launch is cooperative, one CTA per SM.
+ * d->M up to 384 rows per SM of the device (56832 on 148 SMs).  The launch is cooperative, one CTA per SM.
  */
 size_t ade_b200_linear_workspace_bytes(int T, int M, int r);
-int ade_b200_linear(const ade_delta_t* d, const void* x, const void* w_b, void* out, void* scratch, size_t scratch_bytes,
+/* 1 where ade_b200_linear is the faster of the two for a call with y_dense (what the torch binding and
+ * ade_b200_factored_static go by), else 0. */
+int ade_b200_linear_preferred(int T, int M, int r);
+int ade_b200_linear(const ade_delta_t* d, const void* x, const void* y_dense, const void* w_b, void* out, void* scratch, size_t scratch_bytes,
                     void* workspace, size_t workspace_bytes, int T, void* stream);
 
 /*

@@ -35,13 +35,13 @@ def test_linear_matches_oracle(M, N, r, T):
     assert err <= 1e-2 and cos >= 0.9999, (err, cos)
 
 
-@pytest.mark.parametrize("T", [17, 64, 128])
-def test_fused_group_above_16_tokens(T):
-    """A group of three modules of different heights and ranks, one launch, against the members alone: the same products; the
-    contraction is cut differently, so up to the last bf16 bit (2^-8 of the value, and of the row's terms where they cancel)."""
-    N = 1024
-    mods, packs = [], []
-    for M, r in ((700, 256), (300, 384), (1300, 128)):
+@pytest.mark.parametrize("T", [8, 9, 16])
+def test_tall_fused_group(T):
+    """A group of 16500 rows, on both sides of the line at 8 tokens, against its members alone: the same float32 sums in another
+    order, so up to the last bf16 bit (2^-8 of the value, and of the row's terms where they cancel)."""
+    N = 128
+    mods = []
+    for M, r in ((7700, 256), (300, 384), (8500, 128)):
         tp, W, x = _case(M, N, r, T)
         mods.append(serving.ADEKernelLinear(W, tp).to(DEV))
     xd = x.to(DEV)
@@ -53,6 +53,23 @@ def test_fused_group_above_16_tokens(T):
         assert torch.all((y.float() - a.float()).abs() <= 2.0 ** -7 * (a.float().abs() + a.float().abs().mean()))
     torch.cuda.synchronize()
     kernels.check_factored_status(DEV)
+
+
+# both ways U^ h is prepared (64 / 65 tokens), one to three slices per SM, ragged rows, the highest rank, fewer rows than SMs
+@pytest.mark.parametrize("M,N,r,T", [(5000, 256, 896, 33), (5000, 256, 896, 64), (129, 128, 256, 65), (300, 1024, 2048, 100), (4097, 384, 1024, 47),
+                                     (19000, 128, 256, 40), (38000, 128, 128, 128), (1, 128, 128, 128)])
+def test_supplied_base_term(M, N, r, T):
+    tp, W, x = _case(M, N, r, T)
+    assert _lib.load().ade_b200_linear_preferred(T, M, r) == 1
+    p4, xd = kernels.pack_int4(tp, device=DEV), x.to(DEV)
+    yd = torch.nn.functional.linear(xd, W.to(DEV))
+    y, y2 = kernels.decode_forward_packed(xd, yd, p4), kernels.decode_forward_packed(xd, yd, p4)
+    torch.cuda.synchronize()
+    kernels.check_factored_status(DEV)
+    assert torch.equal(y, y2), "two runs differ"
+    ref = O.factored_apply(x.view(torch.uint16).numpy(), W.view(torch.uint16).numpy(), O.packed_from_torch(tp))
+    err, cos = O.parity(y.float().cpu().numpy(), ref)
+    assert err <= 1e-2 and cos >= 0.9999, (err, cos)
 
 
 def test_linear_wait_expires_and_recovers():
@@ -88,3 +105,16 @@ def test_linear_argument_checks():
         kernels.linear_forward(x.float().to(DEV), p4, W.to(DEV))
     with pytest.raises(_lib.AdeKernelError):
         kernels.linear_forward(torch.zeros(129, 256, dtype=torch.bfloat16, device=DEV), p4, W.to(DEV))
+
+
+@pytest.mark.parametrize("M,T", [(16384, 8), (16384, 9), (16383, 9), (16384, 17), (300, 16), (300, 17), (300, 64), (300, 65)])
+def test_module_dispatch_edges(M, T):
+    """Both sides of the lines between the two kernels, through the module."""
+    N, r = 128, 128
+    tp, W, x = _case(M, N, r, T)
+    y = serving.ADEKernelLinear(W, tp).to(DEV)(x.to(DEV))
+    torch.cuda.synchronize()
+    kernels.check_factored_status(DEV)
+    ref = O.factored_apply(x.view(torch.uint16).numpy(), W.view(torch.uint16).numpy(), O.packed_from_torch(tp))
+    err, cos = O.parity(y.float().cpu().numpy(), ref)
+    assert err <= 1e-2 and cos >= 0.9999, (err, cos)
