@@ -36,8 +36,12 @@ def _plain_inference(*tensors) -> bool:
             and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
 
 
+def _on_cuda(t: torch.Tensor) -> bool:
+    return t.is_cuda
+
+
 def _rows_ok(t: torch.Tensor, rows: int, *others) -> bool:
-    return t.is_cuda and t.dtype == torch.bfloat16 and rows > 0 and (rows <= MAX_ROWS or _plain_inference(t, *others))
+    return _on_cuda(t) and t.dtype == torch.bfloat16 and rows > 0 and (rows <= MAX_ROWS or _plain_inference(t, *others))
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
@@ -139,6 +143,13 @@ def _rope_layout_ok(x: torch.Tensor) -> bool:
     return x.stride(3) == 1 and (h == 1 or x.stride(1) == hd) and (B == 1 or T == 1 or x.stride(0) == T * x.stride(2))
 
 
+def _add_norm_ok(x: torch.Tensor, residual: torch.Tensor, norm) -> bool:
+    """`residual + x` and the LlamaRMSNorm `norm` behind it can be one launch.  Asked about the very tensors that go into it: a
+    module in front may have made one of them require a gradient although the layer's input does not."""
+    return (_rows_ok(x, x.numel() // x.shape[-1], residual, norm.weight) and residual.dtype == torch.bfloat16 and norm.weight.dtype == torch.bfloat16
+            and x.shape == residual.shape and x.stride(-1) == 1 and residual.stride(-1) == 1)
+
+
 def enable_fused_decode_ops(model) -> int:
     """Patch `model` (a transformers LLaMA-architecture causal LM) in place; returns the number of modules patched.
     The rotary embedding is a module-level function of transformers' LLaMA implementation, so that patch is
@@ -198,9 +209,10 @@ def enable_fused_decode_ops(model) -> int:
             mod._ade_orig_forward = mod.forward
 
             def mlp_forward(x, mod=mod):
-                if _rows_ok(x, x.numel() // x.shape[-1], *mod.parameters()):
+                if _rows_ok(x, x.numel() // x.shape[-1]):
                     g, u = mod.gate_proj(x), mod.up_proj(x)
-                    if g.dtype == torch.bfloat16 and g.stride(-1) == 1 and u.stride(-1) == 1:
+                    if (_rows_ok(g, g.numel() // g.shape[-1], u) and u.dtype == torch.bfloat16 and g.shape == u.shape and g.stride(-1) == 1
+                            and u.stride(-1) == 1):
                         return mod.down_proj(silu_mul(g, u))
                     return mod.down_proj(mod.act_fn(g) * u)
                 return mod._ade_orig_forward(x)
@@ -226,16 +238,21 @@ def enable_fused_decode_ops(model) -> int:
             def layer_forward(hidden_states, attention_mask=None, position_ids=None, past_key_values=None, use_cache=False,
                               position_embeddings=None, layer=layer, nxt=nxt, **kw):
                 post = layer.post_attention_layernorm
-                if not (_rows_ok(hidden_states, hidden_states.numel() // hidden_states.shape[-1], post.weight, nxt.weight) and hidden_states.is_contiguous()
-                        and post.weight.dtype == torch.bfloat16 and nxt.weight.dtype == torch.bfloat16 and not layer.training):
+                if not (_rows_ok(hidden_states, hidden_states.numel() // hidden_states.shape[-1]) and not layer.training):
                     return layer._ade_orig_forward(hidden_states, attention_mask=attention_mask, position_ids=position_ids,
                                                    past_key_values=past_key_values, use_cache=use_cache,
                                                    position_embeddings=position_embeddings, **kw)
                 h = layer.input_layernorm(hidden_states)
                 a, _ = layer.self_attn(hidden_states=h, attention_mask=attention_mask, position_ids=position_ids,
                                        past_key_values=past_key_values, use_cache=use_cache, position_embeddings=position_embeddings, **kw)
-                s1, h2 = add_rmsnorm(a, hidden_states, post.weight, post.variance_epsilon)
+                if _add_norm_ok(a, hidden_states, post):
+                    s1, h2 = add_rmsnorm(a, hidden_states, post.weight, post.variance_epsilon)
+                else:
+                    s1 = hidden_states + a
+                    h2 = post(s1)
                 m = layer.mlp(h2)
+                if not _add_norm_ok(m, s1, nxt):
+                    return s1 + m
                 s2, h3 = add_rmsnorm(m, s1, nxt.weight, nxt.variance_epsilon)
                 nxt._ade_pre = (s2, h3)
                 return s2

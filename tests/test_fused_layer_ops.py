@@ -1,0 +1,91 @@
+"""The patched decoder layer (`decode_ops.enable_fused_decode_ops`) against the unpatched one where something looks at, edits or
+differentiates through what lies between its modules.  600 token rows: above the limit up to which the kernels are unconditional.
+
+Every case runs on the GPU and, with torch stand-ins for the four launches (fresh tensors outside autograd, as a launch through raw
+pointers leaves them), on the CPU: what is tested is when a launch may take the place of the operations, not its arithmetic."""
+from __future__ import annotations
+
+import copy
+
+import pytest
+import torch
+
+from ade_b200 import decode_ops
+
+
+def _norm(x, weight, eps):
+    x32 = x.float()
+    return weight * (x32 * torch.rsqrt(x32.pow(2).mean(-1, keepdim=True) + eps)).to(x.dtype)
+
+
+def _rot(t):
+    return torch.cat((-t[..., t.shape[-1] // 2:], t[..., :t.shape[-1] // 2]), -1)
+
+
+STAND_INS = {
+    "rmsnorm": _norm,
+    "add_rmsnorm": lambda x, res, weight, eps: (res + x, _norm(res + x, weight, eps)),
+    "rope": lambda q, k, cos, sin: tuple(t * cos.unsqueeze(1) + _rot(t) * sin.unsqueeze(1) for t in (q, k)),
+    "silu_mul": lambda g, u: torch.nn.functional.silu(g) * u,
+}
+
+
+@pytest.fixture(params=["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def dev(request, monkeypatch):
+    """(device of the case, names of the launches or stand-ins that were taken)."""
+    launches = []
+    for name, stand_in in STAND_INS.items():
+        fn = torch.no_grad()(stand_in) if request.param == "cpu" else getattr(decode_ops, name)
+        monkeypatch.setattr(decode_ops, name, lambda *a, fn=fn, name=name: launches.append(name) or fn(*a))
+    if request.param == "cpu":
+        monkeypatch.setattr(decode_ops, "_on_cuda", lambda t: True)
+    return request.param, launches
+
+
+def _models(dev, seed=0):
+    """(patched, unpatched) frozen copies of one small LLaMA model in eval mode."""
+    from transformers import LlamaConfig, LlamaForCausalLM
+
+    cfg = LlamaConfig(hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=4, vocab_size=512,
+                      max_position_embeddings=1024)
+    torch.manual_seed(seed)
+    plain = LlamaForCausalLM(cfg).to(torch.bfloat16).eval().to(dev)
+    plain.requires_grad_(False)
+    patched = copy.deepcopy(plain)
+    decode_ops.enable_fused_decode_ops(patched)
+    return patched, plain
+
+
+def _ids(dev, seed=1):
+    return torch.randint(0, 512, (2, 300), generator=torch.Generator().manual_seed(seed)).to(dev)
+
+
+def _rel(a, b):
+    return float((a.float() - b.float()).norm() / b.float().norm())
+
+
+@pytest.mark.parametrize("name", ["self_attn.o_proj", "self_attn.q_proj", "mlp.up_proj", "mlp.gate_proj", "mlp.down_proj"])
+def test_gradient_of_one_trainable_module(dev, name):
+    """One trainable weight inside a layer: the layer's input requires no gradient, what its modules return does.  A unit in the last
+    place of bf16 is 2^-8 of a value and two layers of roundings lie between the weight and the result: 5 per cent."""
+    dev, _ = dev
+    grads = []
+    for model in _models(dev):
+        w = model.model.layers[0].get_submodule(name).weight
+        w.requires_grad_(True)
+        model(input_ids=_ids(dev), use_cache=False).logits.float().square().mean().backward()
+        grads.append(w.grad)
+    got, want = grads
+    assert got is not None and float(want.float().norm()) > 0 and _rel(got, want) < 5e-2
+
+
+def test_fused_where_nothing_differentiates(dev):
+    """The launches are taken on long inputs of a frozen model, with gradients enabled too."""
+    dev, launches = dev
+    patched, plain = _models(dev)
+    with torch.no_grad():
+        want = plain(input_ids=_ids(dev), use_cache=False).logits
+    launches.clear()
+    got = patched(input_ids=_ids(dev), use_cache=False).logits
+    assert launches.count("add_rmsnorm") == 4 and launches.count("silu_mul") == 2 and launches.count("rope") == 2
+    assert _rel(got, want) < 2e-2
