@@ -19,12 +19,15 @@ from __future__ import annotations
 import torch
 
 from . import _lib
+from .kernels import _on_device
 
 MAX_ROWS = 512          # token rows (batch * sequence) up to which the fused kernels are used unconditionally
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+def _launch(entry: str, dev: torch.device, *args) -> None:
+    """One call of the C entry `entry` on the current stream of `dev`, the device of the tensors (which need not be the current one)."""
+    with _on_device(dev):
+        _lib.check(getattr(_lib.load(), entry)(*args, torch.cuda.current_stream(dev).cuda_stream), entry)
 
 
 def _plain_inference(*tensors) -> bool:
@@ -41,7 +44,9 @@ def _on_cuda(t: torch.Tensor) -> bool:
 
 
 def _rows_ok(t: torch.Tensor, rows: int, *others) -> bool:
-    return _on_cuda(t) and t.dtype == torch.bfloat16 and rows > 0 and (rows <= MAX_ROWS or _plain_inference(t, *others))
+    """The kernels take `t` together with `others`: all on one device, and nothing records what is done with them."""
+    return (_on_cuda(t) and t.dtype == torch.bfloat16 and rows > 0 and all(o.device == t.device for o in others)
+            and (rows <= MAX_ROWS or _plain_inference(t, *others)))
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
@@ -51,8 +56,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     if x2.stride(1) != 1:
         x2 = x2.contiguous()
     out = torch.empty((x2.shape[0], H), dtype=torch.bfloat16, device=x.device)
-    _lib.check(_lib.load().ade_b200_rmsnorm(x2.data_ptr(), weight.data_ptr(), out.data_ptr(), x2.shape[0], H, x2.stride(0), float(eps),
-                                            _stream()), "ade_b200_rmsnorm")
+    _launch("ade_b200_rmsnorm", x.device, x2.data_ptr(), weight.data_ptr(), out.data_ptr(), x2.shape[0], H, x2.stride(0), float(eps))
     return out.view(x.shape)
 
 
@@ -67,8 +71,8 @@ def add_rmsnorm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, e
         r2 = r2.contiguous()
     total = torch.empty((x2.shape[0], H), dtype=torch.bfloat16, device=x.device)
     out = torch.empty_like(total)
-    _lib.check(_lib.load().ade_b200_add_rmsnorm(x2.data_ptr(), r2.data_ptr(), weight.data_ptr(), total.data_ptr(), out.data_ptr(), x2.shape[0], H,
-                                                x2.stride(0), r2.stride(0), float(eps), _stream()), "ade_b200_add_rmsnorm")
+    _launch("ade_b200_add_rmsnorm", x.device, x2.data_ptr(), r2.data_ptr(), weight.data_ptr(), total.data_ptr(), out.data_ptr(), x2.shape[0], H,
+            x2.stride(0), r2.stride(0), float(eps))
     return total.view(x.shape), out.view(x.shape)
 
 
@@ -83,8 +87,8 @@ def rope(q: torch.Tensor, k: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor)
     # distance between consecutive (batch, token) rows of the projection; a dimension of size 1 reports an arbitrary stride
     rq = q.stride(2) if T > 1 else q.stride(0)
     rk = k.stride(2) if T > 1 else k.stride(0)
-    _lib.check(_lib.load().ade_b200_rope(q.data_ptr(), k.data_ptr(), cos.data_ptr(), sin.data_ptr(), qo.data_ptr(), ko.data_ptr(), B, T, hq, hk,
-                                         hd, rq, rk, cs_stride, _stream()), "ade_b200_rope")
+    _launch("ade_b200_rope", q.device, q.data_ptr(), k.data_ptr(), cos.data_ptr(), sin.data_ptr(), qo.data_ptr(), ko.data_ptr(), B, T, hq, hk, hd,
+            rq, rk, cs_stride)
     return qo, ko
 
 
@@ -93,8 +97,7 @@ def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     cols = gate.shape[-1]
     g2, u2 = gate.reshape(-1, cols), up.reshape(-1, cols)
     out = torch.empty((g2.shape[0], cols), dtype=torch.bfloat16, device=gate.device)
-    _lib.check(_lib.load().ade_b200_silu_mul(g2.data_ptr(), u2.data_ptr(), out.data_ptr(), g2.shape[0], cols, g2.stride(0), u2.stride(0),
-                                             _stream()), "ade_b200_silu_mul")
+    _launch("ade_b200_silu_mul", gate.device, g2.data_ptr(), u2.data_ptr(), out.data_ptr(), g2.shape[0], cols, g2.stride(0), u2.stride(0))
     return out.view(*gate.shape[:-1], cols)
 
 
@@ -110,11 +113,10 @@ def attn_decode(q, k, v, cos, sin, mask, layer, scale: float) -> torch.Tensor:
     ticket = getattr(layer, "_ade_ticket", None)           # counter through which the launch advances the position itself
     if ticket is None or ticket.device != q.device:
         ticket = layer._ade_ticket = torch.zeros(1, dtype=torch.int32, device=q.device)
-    _lib.check(_lib.load().ade_b200_attn_decode(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), None if mask is None else mask.data_ptr(),
-        layer.keys.data_ptr(), layer.values.data_ptr(), layer.cumulative_length.data_ptr(), ticket.data_ptr(), out.data_ptr(), B, hq, hk, hd, L,
-        row(q), row(k), row(v), 0 if cos.shape[0] == 1 else hd, 0 if mask is None else mask.stride(0), float(scale), _stream()),
-        "ade_b200_attn_decode")
+    _launch("ade_b200_attn_decode", q.device,
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), None if mask is None else mask.data_ptr(),
+            layer.keys.data_ptr(), layer.values.data_ptr(), layer.cumulative_length.data_ptr(), ticket.data_ptr(), out.data_ptr(), B, hq, hk, hd, L,
+            row(q), row(k), row(v), 0 if cos.shape[0] == 1 else hd, 0 if mask is None else mask.stride(0), float(scale))
     return out
 
 
@@ -125,6 +127,8 @@ def _attn_decode_ok(mod, x, cos, mask, layer) -> bool:
         return False
     kc = layer.keys
     if not (kc.dtype == torch.bfloat16 and kc.is_contiguous() and layer.values.is_contiguous() and kc.shape[0] == x.shape[0]):
+        return False
+    if any(t.device != x.device for t in (cos, kc, layer.values, layer.cumulative_length)) or (mask is not None and mask.device != x.device):
         return False
     hd = kc.shape[3]
     if hd % 32 or hd > 256 or (7 * hd + kc.shape[2]) * 4 > 48 * 1024 or layer.cumulative_length.dtype != torch.int64:
@@ -152,8 +156,9 @@ def _add_norm_ok(x: torch.Tensor, residual: torch.Tensor, norm) -> bool:
 
 def enable_fused_decode_ops(model) -> int:
     """Patch `model` (a transformers LLaMA-architecture causal LM) in place; returns the number of modules patched.
-    The rotary embedding is a module-level function of transformers' LLaMA implementation, so that patch is
-    process-wide (it falls back to the original for anything but small bfloat16 CUDA inputs)."""
+    The rotary embedding is a module-level function of transformers' LLaMA implementation, so that patch is process-wide: LLaMA models
+    that were never patched take the launch too, for bfloat16 CUDA inputs with everything on one device (above ``MAX_ROWS`` token rows
+    where nothing differentiates or traces); anything else takes the original."""
     from transformers.models.llama import modeling_llama as ml
 
     if not getattr(ml, "_ade_rope_patched", False):
@@ -179,7 +184,8 @@ def enable_fused_decode_ops(model) -> int:
                 if (position_embeddings is not None and layer is not None
                         and _attn_decode_ok(mod, hidden_states, position_embeddings[0], attention_mask, layer)):
                     q, k, v = mod.q_proj(hidden_states), mod.k_proj(hidden_states), mod.v_proj(hidden_states)
-                    if all(t.dtype == torch.bfloat16 and t.stride(-1) == 1 for t in (q, k, v)) and position_embeddings[1].is_contiguous():
+                    if (all(t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.device == hidden_states.device for t in (q, k, v))
+                            and position_embeddings[1].is_contiguous() and position_embeddings[1].device == hidden_states.device):
                         ctx = attn_decode(q, k, v, position_embeddings[0], position_embeddings[1], attention_mask, layer, mod.scaling)
                         return mod.o_proj(ctx), None
                 return mod._ade_orig_forward(hidden_states, position_embeddings=position_embeddings, attention_mask=attention_mask,

@@ -89,3 +89,57 @@ def test_fused_where_nothing_differentiates(dev):
     got = patched(input_ids=_ids(dev), use_cache=False).logits
     assert launches.count("add_rmsnorm") == 4 and launches.count("silu_mul") == 2 and launches.count("rope") == 2
     assert _rel(got, want) < 2e-2
+
+
+def test_operands_on_another_device_are_left_to_torch(monkeypatch):
+    """A model spread over devices: a norm weight, a residual, cos / sin or a cache elsewhere cannot be passed to a launch as a pointer."""
+    monkeypatch.setattr(decode_ops, "_on_cuda", lambda t: True)
+    x = torch.zeros(2, 4, 8, dtype=torch.bfloat16)
+    away = torch.zeros(2, 4, 8, dtype=torch.bfloat16, device="meta")
+    norm = torch.nn.Module()
+    for weight, residual, ok in ((x[0, 0], x, True), (away[0, 0], x, False), (x[0, 0], away, False)):
+        norm.weight = torch.nn.Parameter(weight, requires_grad=False)
+        assert decode_ops._add_norm_ok(x, residual, norm) is ok
+    assert decode_ops._rows_ok(x, 8, x, x) and not decode_ops._rows_ok(x, 8, x, away)
+
+    class Layer:
+        is_initialized = True
+        keys = values = torch.zeros(2, 1, 16, 32, dtype=torch.bfloat16)
+        cumulative_length = torch.zeros(1, dtype=torch.int64)
+
+    Layer.__name__ = "StaticLayer"
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: True))
+    step, cos, mod = torch.zeros(2, 1, 32, dtype=torch.bfloat16), torch.zeros(1, 1, 32, dtype=torch.bfloat16), torch.nn.Module().eval()
+    assert decode_ops._attn_decode_ok(mod, step, cos, None, Layer())
+    assert not decode_ops._attn_decode_ok(mod, step, cos.to("meta"), None, Layer())
+
+
+def test_launches_go_to_the_device_of_the_tensors(monkeypatch):
+    """Every launch is made with the tensors' device current and on that device's current stream."""
+    import contextlib
+    import types
+
+    current, seen = [], []
+
+    @contextlib.contextmanager
+    def on_device(d):
+        current.append(d)
+        yield
+        current.pop()
+
+    class Lib:
+        def __getattr__(self, entry):
+            return lambda *a: seen.append((entry, list(current), a[-1])) or 0
+
+    monkeypatch.setattr(decode_ops, "_on_device", on_device)
+    monkeypatch.setattr(decode_ops._lib, "load", Lib)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: types.SimpleNamespace(cuda_stream=("stream of", d)))
+    x = torch.zeros(2, 4, 8, dtype=torch.bfloat16)
+    cache = types.SimpleNamespace(keys=torch.zeros(2, 1, 16, 8), values=torch.zeros(2, 1, 16, 8), cumulative_length=torch.zeros(1, dtype=torch.int64))
+    decode_ops.rmsnorm(x, x[0, 0], 1e-6)
+    decode_ops.add_rmsnorm(x, x, x[0, 0], 1e-6)
+    decode_ops.silu_mul(x, x)
+    decode_ops.rope(x.unsqueeze(1), x.unsqueeze(1), x[:1], x[:1])
+    decode_ops.attn_decode(x[:, :1], x[:, :1], x[:, :1], x[:1, :1], x[:1, :1], None, cache, 1.0)
+    assert [s[0] for s in seen] == [f"ade_b200_{n}" for n in ("rmsnorm", "add_rmsnorm", "silu_mul", "rope", "attn_decode")]
+    assert all(s[1] == [x.device] and s[2] == ("stream of", x.device) for s in seen)
