@@ -22,6 +22,7 @@ from . import _lib
 from .kernels import _on_device
 
 MAX_ROWS = 512          # token rows (batch * sequence) up to which the fused kernels are used unconditionally
+SILU_TYPES = ("SiLU", "SiLUActivation")
 
 
 def _launch(entry: str, dev: torch.device, *args) -> None:
@@ -47,6 +48,14 @@ def _rows_ok(t: torch.Tensor, rows: int, *others) -> bool:
     """The kernels take `t` together with `others`: all on one device, and nothing records what is done with them."""
     return (_on_cuda(t) and t.dtype == torch.bfloat16 and rows > 0 and all(o.device == t.device for o in others)
             and (rows <= MAX_ROWS or _plain_inference(t, *others)))
+
+
+def _passable(mod) -> bool:
+    """Nobody would notice that `mod` is not called: no hooks of its own or for all modules, and the forward it came (or was patched) with."""
+    m = torch.nn.modules.module
+    return not (mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks or m._global_forward_hooks
+                or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks
+                or mod.__dict__.get("forward") is not mod.__dict__.get("_ade_forward"))
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
@@ -208,17 +217,17 @@ def enable_fused_decode_ops(model) -> int:
                     return rmsnorm(x, mod.weight, mod.variance_epsilon)
                 return mod._ade_orig_forward(x)
 
-            mod.forward = norm_forward
+            mod.forward = mod._ade_forward = norm_forward
             n += 1
         elif (isinstance(mod, ml.LlamaMLP) and not hasattr(mod, "_ade_orig_forward")
-              and type(mod.act_fn).__name__ in ("SiLU", "SiLUActivation")):
+              and type(mod.act_fn).__name__ in SILU_TYPES):
             mod._ade_orig_forward = mod.forward
 
             def mlp_forward(x, mod=mod):
                 if _rows_ok(x, x.numel() // x.shape[-1]):
                     g, u = mod.gate_proj(x), mod.up_proj(x)
                     if (_rows_ok(g, g.numel() // g.shape[-1], u) and u.dtype == torch.bfloat16 and g.shape == u.shape and g.stride(-1) == 1
-                            and u.stride(-1) == 1):
+                            and u.stride(-1) == 1 and type(mod.act_fn).__name__ in SILU_TYPES and _passable(mod.act_fn)):
                         return mod.down_proj(silu_mul(g, u))
                     return mod.down_proj(mod.act_fn(g) * u)
                 return mod._ade_orig_forward(x)
@@ -251,7 +260,7 @@ def enable_fused_decode_ops(model) -> int:
                 h = layer.input_layernorm(hidden_states)
                 a, _ = layer.self_attn(hidden_states=h, attention_mask=attention_mask, position_ids=position_ids,
                                        past_key_values=past_key_values, use_cache=use_cache, position_embeddings=position_embeddings, **kw)
-                if _add_norm_ok(a, hidden_states, post):
+                if _add_norm_ok(a, hidden_states, post) and hasattr(post, "_ade_pre") and _passable(post):
                     s1, h2 = add_rmsnorm(a, hidden_states, post.weight, post.variance_epsilon)
                 else:
                     s1 = hidden_states + a

@@ -143,3 +143,32 @@ def test_launches_go_to_the_device_of_the_tensors(monkeypatch):
     decode_ops.attn_decode(x[:, :1], x[:, :1], x[:, :1], x[:1, :1], x[:1, :1], None, cache, 1.0)
     assert [s[0] for s in seen] == [f"ade_b200_{n}" for n in ("rmsnorm", "add_rmsnorm", "silu_mul", "rope", "attn_decode")]
     assert all(s[1] == [x.device] and s[2] == ("stream of", x.device) for s in seen)
+
+
+@pytest.mark.parametrize("name", ["post_attention_layernorm", "mlp.act_fn", "input_layernorm", "mlp"])
+@pytest.mark.parametrize("how", ["hook", "pre_hook", "global", "wrapped"])
+def test_modules_somebody_listens_to_are_called(dev, name, how):
+    """Hooks on a module of the layer, hooks for all modules, and a forward that was wrapped: they see as many calls as in the
+    unpatched model, and what a hook puts in place of an output arrives."""
+    dev, _ = dev
+    counts, logits = [], []
+    for model in _models(dev):
+        mod, seen, handle = model.model.layers[0].get_submodule(name), [], None
+        if how == "hook":
+            mod.register_forward_hook(lambda m, a, out: seen.append(1) or out * 1.5)
+        elif how == "pre_hook":
+            mod.register_forward_pre_hook(lambda m, a: seen.append(1))
+        elif how == "global":
+            handle = torch.nn.modules.module.register_module_forward_hook(lambda m, a, out: seen.append(1) if m is mod else None)
+        else:
+            inner = mod.forward
+            mod.forward = lambda *a, **k: seen.append(1) or inner(*a, **k)
+        try:
+            with torch.no_grad():
+                logits.append(model(input_ids=_ids(dev), use_cache=False).logits)
+        finally:
+            if handle is not None:
+                handle.remove()
+        counts.append(len(seen))
+    assert counts[0] == counts[1] == 1
+    assert _rel(*logits) < 2e-2
