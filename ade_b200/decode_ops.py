@@ -205,14 +205,14 @@ def enable_fused_decode_ops(model) -> int:
         elif isinstance(mod, ml.LlamaRMSNorm) and not hasattr(mod, "_ade_orig_forward"):
             mod._ade_orig_forward = mod.forward
 
-            mod._ade_pre = None                   # (input tensor, its normalisation) left by the layer in front, see below
+            mod._ade_pre = None                   # (input tensor, its version, its normalisation) left by the layer in front, see below
 
             def norm_forward(x, mod=mod):
                 pre = mod._ade_pre
                 if pre is not None:
                     mod._ade_pre = None
-                    if x is pre[0]:
-                        return pre[1]
+                    if x is pre[0] and x._version == pre[1]:
+                        return pre[2]
                 if _rows_ok(x, x.numel() // x.shape[-1], mod.weight) and x.stride(-1) == 1 and mod.weight.dtype == torch.bfloat16:
                     return rmsnorm(x, mod.weight, mod.variance_epsilon)
                 return mod._ade_orig_forward(x)
@@ -237,7 +237,8 @@ def enable_fused_decode_ops(model) -> int:
     # Residual connections: a decoder layer adds the attention output and the MLP output to its input, each time right in
     # front of an RMSNorm (its own post-attention norm; the next layer's input norm, or the model's final norm).  A
     # patched layer does add + norm in one launch each and leaves the second normalisation with the norm module that is
-    # about to be asked for it, which recognises the tensor by identity.
+    # about to be asked for it, which recognises the tensor by identity and by its version: a hook or wrapper in between may
+    # have edited it in place.
     for lm in model.modules():
         if not isinstance(lm, ml.LlamaModel):
             continue
@@ -266,10 +267,10 @@ def enable_fused_decode_ops(model) -> int:
                     s1 = hidden_states + a
                     h2 = post(s1)
                 m = layer.mlp(h2)
-                if not _add_norm_ok(m, s1, nxt):
+                if torch.is_inference_mode_enabled() or not _add_norm_ok(m, s1, nxt):     # inference tensors do not count their versions
                     return s1 + m
                 s2, h3 = add_rmsnorm(m, s1, nxt.weight, nxt.variance_epsilon)
-                nxt._ade_pre = (s2, h3)
+                nxt._ade_pre = (s2, s2._version, h3)
                 return s2
 
             layer.forward = layer_forward

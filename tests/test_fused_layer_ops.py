@@ -172,3 +172,18 @@ def test_modules_somebody_listens_to_are_called(dev, name, how):
         counts.append(len(seen))
     assert counts[0] == counts[1] == 1
     assert _rel(*logits) < 2e-2
+
+
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode])
+@pytest.mark.parametrize("rows", [(2, 300), (1, 20)])
+def test_hidden_state_edited_in_place_between_layers(dev, mode, rows):
+    """A forward hook that adds to a layer's output in place (steering vectors, features added at some layers) leaves the tensor's identity
+    as it is; the norm behind it normalises the edited values."""
+    dev, _ = dev
+    logits, g = [], torch.Generator().manual_seed(3)
+    ids, steer = torch.randint(0, 512, rows, generator=g).to(dev), torch.randn(256, generator=g).to(torch.bfloat16).to(dev)
+    for model in _models(dev):
+        model.model.layers[0].register_forward_hook(lambda m, a, out: (out.add_(steer), None)[1])
+        with mode():
+            logits.append(model(input_ids=ids, use_cache=False).logits.clone())
+    assert _rel(*logits) < 2e-2
