@@ -68,9 +68,15 @@ class ADEKernelLinear(nn.Module):
         self._x8 = None               # (uq pointer, (u8, v8)): expanded operands of the reconstruction, built on demand
         self._group = None            # (FusedADEGroup, index) once fuse_kernel_linears has grouped this module
 
+    def _tensor(self, name: str) -> torch.Tensor:
+        """self.<name> without the module's attribute lookup (0.2 us of every call) while it is a plain buffer; a caller may have made it a
+        parameter or parametrized it."""
+        t = self._buffers.get(name)
+        return getattr(self, name) if t is None else t
+
     def _stored_form(self) -> dict:
         """Stored form on the module's device (rebuilt after .to(device))."""
-        if self._p4 is None or self._p4["uq"].data_ptr() != self._buffers["p4_uq"].data_ptr():
+        if self._p4 is None or self._p4["uq"].data_ptr() != self._tensor("p4_uq").data_ptr():
             self._p4 = {k: getattr(self, f"p4_{k}") for k in STORED_KEYS}
             self._p4["M"], self._p4["N"], self._p4["r"] = self._dims
         return self._p4
@@ -100,7 +106,7 @@ class ADEKernelLinear(nn.Module):
         if T <= self.decode_max_tokens:
             y = self._group[0].apply(self._group[1], x, x2) if self._group is not None and T <= FUSED_MAX_TOKENS else None
             if y is None:
-                y = module_forward(x2, self._stored_form(), self._buffers["weight"])
+                y = module_forward(x2, self._stored_form(), self._tensor("weight"))
         else:
             y = F.linear(x2, self.merged_weight())
         return y if plain else y.reshape(*shape[:-1], self.out_features)
