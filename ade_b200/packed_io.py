@@ -177,6 +177,8 @@ class DeviceDeltaLoader:
             "M": M, "N": N, "r": r,
         }
         lib, check = self.lib, _lib.check
+        # The blocks came from the caller's stream: kernels queued there may still read what they held before.
+        self.stream.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.device(dev), torch.cuda.stream(self.stream):
             sp = self.stream.cuda_stream
             staged[:total].copy_(pinned[:total], non_blocking=True)
@@ -188,7 +190,7 @@ class DeviceDeltaLoader:
             out["vs"].view(torch.uint8).reshape(-1).copy_(staged[off["Vt_scale"][0]:off["Vt_scale"][0] + off["Vt_scale"][1]])
             ev = torch.cuda.Event()
             ev.record(self.stream)
-        for v in out.values():
+        for v in (staged, *out.values()):
             if torch.is_tensor(v):
                 v.record_stream(self.stream)
         self._free[t] = ev
