@@ -65,7 +65,7 @@ class ADEKernelLinear(nn.Module):
         for k in STORED_KEYS:
             self.register_buffer(f"p4_{k}", p4[k])
         self._p4 = None
-        self._x8 = None               # (uq pointer, (u8, v8)): expanded operands of the reconstruction, built on demand
+        self._x8 = None               # ([(tensor, version)], (u8, v8)): expanded operands and what they were made from, built on demand
         self._group = None            # (FusedADEGroup, index) once fuse_kernel_linears has grouped this module
 
     def _tensor(self, name: str) -> torch.Tensor:
@@ -82,11 +82,18 @@ class ADEKernelLinear(nn.Module):
         return self._p4
 
     def _expanded(self):
-        """8-bit operands of the reconstruction kernel, built on the first long input and kept ((d_o + d_i) * r bytes;
-        EXPAND_FOR_RECON = False keeps the packed codes only and unpacks inside the kernel on every call)."""
+        """8-bit operands of the reconstruction kernel, built on the first long input and kept ((d_o + d_i) * r bytes) until the codes
+        or zero-points they were made from are written to or replaced (load_state_dict).  EXPAND_FOR_RECON = False keeps the packed
+        codes only; every call then unpacks them, inside the kernel or, from rank 384, into a buffer of that size for the call."""
         p4 = self._stored_form()
-        if self._x8 is None or self._x8[0] != p4["uq"].data_ptr():
-            self._x8 = (p4["uq"].data_ptr(), expand_codes_f8(p4))
+        made_from = [p4[k] for k in ("uq", "uz", "vq", "vz")]
+        if any(t.is_inference() for t in made_from):
+            return None               # their contents can change unnoticed (no version counter): nothing is kept
+        if self._x8 is None or any(t is not old or t._version != v for t, (old, v) in zip(made_from, self._x8[0])):
+            new, kept = expand_codes_f8(p4), self._x8
+            if kept is not None and kept[1][0].device == new[0].device and not kept[1][0].is_inference():
+                new = tuple(old.copy_(t) for old, t in zip(kept[1], new))       # the addresses stay: a captured graph may hold them
+            self._x8 = ([(t, t._version) for t in made_from], new)
         return self._x8[1]
 
     def merged_weight(self) -> torch.Tensor:
