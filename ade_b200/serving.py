@@ -152,25 +152,16 @@ class FusedADEGroup:
         for m, lo, hi in zip(self.members, self.offsets[:-1], self.offsets[1:]):
             m._buffers["weight"] = W[lo:hi]
         self.weight = W
-        uq = torch.zeros(M, r // 2, dtype=torch.uint8, device=dev)
-        us = torch.zeros(M, ng, dtype=forms[0]["us"].dtype, device=dev)
-        uz = torch.zeros(M, ng, dtype=torch.uint8, device=dev)
-        k0 = 0
-        for f, lo, hi in zip(forms, self.offsets[:-1], self.offsets[1:]):
-            uq[lo:hi, k0 // 2:(k0 + f["r"]) // 2] = f["uq"]
-            us[lo:hi, k0 // GROUP:(k0 + f["r"]) // GROUP] = f["us"]
-            uz[lo:hi, k0 // GROUP:(k0 + f["r"]) // GROUP] = f["uz"]
-            k0 += f["r"]
+        blank = lambda rows, cols, like: torch.zeros(rows, cols, dtype=like.dtype, device=dev)
+        f0 = forms[0]
         self.p4 = {
-            "uq": uq, "us": us, "uz": uz,
-            "vq": torch.cat([f["vq"] for f in forms], dim=1).contiguous(),
-            "vt": torch.cat([f["vt"] for f in forms], dim=0).contiguous(),
-            "vs": torch.cat([f["vs"] for f in forms], dim=0).contiguous(),
-            "vz": torch.cat([f["vz"] for f in forms], dim=0).contiguous(),
+            "uq": blank(M, r // 2, f0["uq"]), "us": blank(M, ng, f0["us"]), "uz": blank(M, ng, f0["uz"]), "vq": blank(N, r // 2, f0["vq"]),
+            "vt": blank(r, N // 2, f0["vt"]), "vs": blank(ng, N, f0["vs"]), "vz": blank(ng, N, f0["vz"]),
             "M": M, "N": N, "r": r,
             # rows of member i use only its own rank groups: the kernel skips the zero blocks of U
             "blocks": [(self.offsets[i], sum(rs[:i]) // GROUP) for i in range(len(Ms) + 1)] if len(Ms) <= 4 else None,
         }
+        self._fill()
         self._x = None                # the input tensor the cached result belongs to (kept alive while cached)
         self._ver = -1
         self._y = None
@@ -178,24 +169,56 @@ class FusedADEGroup:
         for i, m in enumerate(self.members):
             m._group = (self, i)
 
+    def _fill(self):
+        """The members' stored forms into the group's, and what there is to tell when they change: the forms and the sum of their tensors'
+        versions, which only grow."""
+        p4, k0 = self.p4, 0
+        forms = [m._stored_form() for m in self.members]
+        for f, lo, hi in zip(forms, self.offsets[:-1], self.offsets[1:]):
+            k1 = k0 + f["r"]
+            for k, per in (("uq", 2), ("us", GROUP), ("uz", GROUP)):
+                p4[k][lo:hi, k0 // per:k1 // per].copy_(f[k])
+            p4["vq"][:, k0 // 2:k1 // 2].copy_(f["vq"])
+            for k, per in (("vt", 1), ("vs", GROUP), ("vz", GROUP)):
+                p4[k][k0 // per:k1 // per].copy_(f[k])
+            k0 = k1
+        self._forms = forms
+        self._copied = [f[k] for f in forms for k in STORED_KEYS]
+        self._versions = None if any(t.is_inference() for t in (*self._copied, p4["uq"])) else sum(t._version for t in self._copied)
+
+    def refresh(self) -> bool:
+        """Whether the group can serve its members as they are now.  A delta written into the members since (load_state_dict) is copied
+        over; a group whose members have moved, keep their weight elsewhere or cannot be watched (inference tensors) dissolves."""
+        if self.weight is None:
+            return False
+        w, row = self.weight, self.weight.shape[1] * self.weight.element_size()
+        if self._versions is None or any(m._tensor("weight").data_ptr() != w.data_ptr() + lo * row for m, lo in zip(self.members, self.offsets)):
+            self.release()
+        elif any(m._stored_form() is not f for m, f in zip(self.members, self._forms)) or sum(t._version for t in self._copied) != self._versions:
+            if any(f._tensor("p4_uq").device != w.device for f in self.members):
+                self.release()
+            else:
+                self._fill()
+        return self.weight is not None
+
     def release(self):
         """Dissolve the group: the members go back to their own launches and the fused buffers are dropped."""
         for m in self.members:
             if m._group is not None and m._group[0] is self:
                 m._group = None
-        self.weight = self.p4 = self._x = self._y = None
+        self.weight = self.p4 = self._x = self._y = self._forms = self._copied = None
 
     def apply(self, index: int, x, x2):
         """Output of member `index` for the input x (x2 = x as a contiguous (T, d_i) bfloat16 matrix), or None when
-        the group cannot serve it (the members moved to another device since the group was built; the group then
-        dissolves).  The first member asked about a given tensor launches for all; the others get their slices of
-        that result as long as they present the very same tensor object, unmodified: the group holds a reference to
-        it while a result is cached, so no other tensor can take its place in memory, and an in-place write bumps
-        its version."""
-        if self.weight is None or self.members[0].weight.data_ptr() != self.weight.data_ptr():
-            self.release()
+        the group cannot serve it (see `refresh`).  The first member asked about a given tensor launches for all; the
+        others get their slices of that result as long as they present the very same tensor object, unmodified: the
+        group holds a reference to it while a result is cached, so no other tensor can take its place in memory, and
+        an in-place write bumps its version."""
+        if self.weight is None:
             return None
         if self._y is None or x is not self._x or x._version != self._ver or index in self._used:
+            if not self.refresh():
+                return None
             self._y = module_forward(x2, self.p4, self.weight)
             self._x, self._ver = x, x._version
             self._used = set()
@@ -334,6 +357,7 @@ class GreedyGraphDecoder:
         self.model = model
         self.check_status = check_status
         self._graphs = {}          # (batch, max_len) -> (graph, cache, tok, pos, next)
+        self._fused = set()        # the fused groups the captured steps read
 
     def _step(self, cache, tok, pos):
         out = self.model(input_ids=tok, past_key_values=cache, cache_position=pos, use_cache=True)
@@ -373,6 +397,7 @@ class GreedyGraphDecoder:
             with torch.cuda.graph(graph):
                 nxt = self._step(cache, tok, pos)
             self._graphs[key] = (graph, cache, tok, pos, nxt)
+            self._fused |= {m._group[0] for m in self.model.modules() if isinstance(m, ADEKernelLinear) and m._group is not None}
         return self._graphs[key]
 
     @torch.no_grad()
@@ -387,6 +412,10 @@ class GreedyGraphDecoder:
         batch, prompt = input_ids.shape
         device = input_ids.device
         max_len = prompt + max_new_tokens + 1
+        # a captured step reads the groups' tensors without asking them: bring them up to date, or drop graphs whose groups are gone
+        if not all([g.refresh() for g in self._fused]):
+            self._graphs.clear()
+            self._fused = set()
         if use_graph:
             graph, cache, tok, pos, nxt = self._captured(batch, max_len, device)
         else:

@@ -90,3 +90,70 @@ def test_another_delta_in_place(how):
     _fields(other, mod, how)
     for x in xs:
         assert torch.equal(mod(x), other(x))
+
+
+def _group(seeds):
+    return serving.FusedADEGroup([_module(s) for s in seeds])
+
+
+@pytest.mark.parametrize("how", ["copy", "load", "assign"])
+@pytest.mark.parametrize("member", [0, 1])
+def test_group_follows_its_members(monkeypatch, how, member):
+    """A delta written into a member after the group was built is what the group's launch uses, at the same addresses."""
+    seen = []
+    monkeypatch.setattr(serving, "module_forward", lambda x, p4, w: seen.append((p4, w)) or torch.zeros(x.shape[0], w.shape[0], dtype=torch.bfloat16))
+    group, other, x = _group((0, 3)), _module(9), torch.zeros(4, N, dtype=torch.bfloat16)
+    other.weight.copy_(group.members[member].weight)
+    addresses = {k: group.p4[k].data_ptr() for k in serving.STORED_KEYS}
+    [m(x) for m in group.members]
+    assert len(seen) == 1 and seen[0][0] is group.p4
+    if how == "assign":
+        keep = group.members[member].weight
+        _fields(other, group.members[member], how)
+        group.members[member].weight = keep                       # the base weight stays a view of the group's
+    else:
+        _fields(other, group.members[member], how)
+    want = serving.FusedADEGroup([_module(9 if i == member else s) for i, s in enumerate((0, 3))]).p4
+    [m(x.clone()) for m in group.members[:1]]
+    assert seen[-1][0] is group.p4
+    for k in serving.STORED_KEYS:
+        assert torch.equal(group.p4[k], want[k]) and group.p4[k].data_ptr() == addresses[k], k
+
+
+@pytest.mark.parametrize("member", [0, 1])
+def test_group_dissolves_when_a_weight_is_kept_elsewhere(monkeypatch, member):
+    seen = []
+    monkeypatch.setattr(serving, "module_forward", lambda x, p4, w: seen.append(w) or torch.zeros(x.shape[0], w.shape[0], dtype=torch.bfloat16))
+    group, x = _group((0, 3)), torch.zeros(4, N, dtype=torch.bfloat16)
+    mods = group.members
+    mods[member].weight = nn.Parameter(mods[member].weight * 2, requires_grad=False)
+    for m in mods:
+        assert m(x).shape == (4, M)
+    assert not group.refresh() and all(m._group is None for m in mods)
+    assert [w.shape[0] for w in seen] == [M, M] and torch.equal(seen[member], mods[member].weight)
+
+
+@pytest.mark.gpu
+def test_captured_generation_follows_another_delta():
+    """Another delta written into the modules after a step was captured: the next generation, whose prompt is longer than a group serves,
+    gives the tokens of groups built from it."""
+    from ade_b200 import kernels
+
+    model = synth.synthetic_llama("tiny", layers=2, seed=1, vocab=512)[0]
+    ids = torch.randint(0, 512, (1, 30), generator=torch.Generator().manual_seed(4)).cuda()
+    dec = serving.GreedyGraphDecoder(model)
+    before = dec.generate(ids, 12)
+    mods = [m for m in model.modules() if isinstance(m, serving.ADEKernelLinear)]
+    for i, m in enumerate(mods):
+        packed = synth.random_packed(*m._dims, 50 + i)
+        packed["U_scale"] *= 20
+        for k, v in kernels.pack_int4(packed).items():
+            if k in serving.STORED_KEYS:
+                m.get_buffer(f"p4_{k}").copy_(v)
+    got = dec.generate(ids, 12)
+    for m in mods:
+        if m._group is not None:
+            m._group[0].release()
+    assert serving.fuse_kernel_linears(model) == 4
+    want = serving.GreedyGraphDecoder(model).generate(ids, 12, use_graph=False)
+    assert torch.equal(got, want) and not torch.equal(got, before)
