@@ -214,7 +214,7 @@ class FusedADEGroup:
         others get their slices of that result as long as they present the very same tensor object, unmodified: the
         group holds a reference to it while a result is cached, so no other tensor can take its place in memory, and
         an in-place write bumps its version."""
-        if self.weight is None:
+        if self.weight is None or x.is_inference():       # an inference tensor has no version to recognise it by
             return None
         if self._y is None or x is not self._x or x._version != self._ver or index in self._used:
             if not self.refresh():

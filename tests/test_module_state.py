@@ -157,3 +157,15 @@ def test_captured_generation_follows_another_delta():
     assert serving.fuse_kernel_linears(model) == 4
     want = serving.GreedyGraphDecoder(model).generate(ids, 12, use_graph=False)
     assert torch.equal(got, want) and not torch.equal(got, before)
+
+
+def test_group_members_serve_inference_tensors(monkeypatch):
+    """Under torch.inference_mode a tensor has no version counter: the members launch for themselves."""
+    seen = []
+    monkeypatch.setattr(serving, "module_forward", lambda x, p4, w: seen.append(w) or torch.zeros(x.shape[0], w.shape[0], dtype=torch.bfloat16))
+    group = _group((0, 3))
+    with torch.inference_mode():
+        x = torch.zeros(4, N, dtype=torch.bfloat16)
+        for m in group.members:
+            assert m(x).shape == (4, M)
+    assert [w.shape[0] for w in seen] == [M, M] and group.refresh()
