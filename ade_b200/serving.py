@@ -26,6 +26,25 @@ LINEAR_MODULE_NAMES = (
 )
 
 
+def _capturing(t: torch.Tensor) -> bool:
+    return t.is_cuda and torch.cuda.is_current_stream_capturing()
+
+
+def _mark(t: torch.Tensor):
+    """(stream, event) behind what was just launched to make `t`; for `_join`."""
+    if not t.is_cuda:
+        return None, None
+    stream, event = torch.cuda.current_stream(t.device), torch.cuda.Event()
+    event.record(stream)
+    return stream, event
+
+
+def _join(t: torch.Tensor, stream, event) -> None:
+    """Let the current stream wait for `event` unless it is the stream that recorded it."""
+    if stream is not None and torch.cuda.current_stream(t.device) != stream:
+        torch.cuda.current_stream(t.device).wait_event(event)
+
+
 class ADEKernelLinear(nn.Module):
     """Linear module W_b + U^ V^^T applied with the B200 kernels (bfloat16): factored application
     for T <= decode_max_tokens tokens, reconstructed application otherwise (src/serving.py:40-112)."""
@@ -65,8 +84,11 @@ class ADEKernelLinear(nn.Module):
         for k in STORED_KEYS:
             self.register_buffer(f"p4_{k}", p4[k])
         self._p4 = None
-        self._x8 = None               # ([(tensor, version)], (u8, v8)): expanded operands and what they were made from, built on demand
+        self._x8 = None               # ([(tensor, version)], (u8, v8), stream, event): expanded operands, what from, when; built on demand
         self._group = None            # (FusedADEGroup, index) once fuse_kernel_linears has grouped this module
+
+    def __getstate__(self):
+        return {**self.__dict__, "_x8": None}         # a copy or a saved module makes its own (streams and events do not travel)
 
     def _tensor(self, name: str) -> torch.Tensor:
         """self.<name> without the module's attribute lookup (0.2 us of every call) while it is a plain buffer; a caller may have made it a
@@ -91,9 +113,14 @@ class ADEKernelLinear(nn.Module):
             return None               # their contents can change unnoticed (no version counter): nothing is kept
         if self._x8 is None or any(t is not old or t._version != v for t, (old, v) in zip(made_from, self._x8[0])):
             new, kept = expand_codes_f8(p4), self._x8
+            if _capturing(new[0]):
+                return new            # they belong to the graph that is being captured and hold nothing before it runs
             if kept is not None and kept[1][0].device == new[0].device and not kept[1][0].is_inference():
+                _join(kept[1][0], *kept[2:])
                 new = tuple(old.copy_(t) for old, t in zip(kept[1], new))       # the addresses stay: a captured graph may hold them
-            self._x8 = ([(t, t._version) for t in made_from], new)
+            self._x8 = ([(t, t._version) for t in made_from], new, *_mark(new[0]))
+        elif not _capturing(self._x8[1][0]):                              # a capture begins behind everything that was launched
+            _join(self._x8[1][0], *self._x8[2:])
         return self._x8[1]
 
     def merged_weight(self) -> torch.Tensor:

@@ -1,6 +1,8 @@
 """State of a delta module that a program changes after it was built: tensors swapped, parametrized or written in place."""
 from __future__ import annotations
 
+import copy
+
 import pytest
 import torch
 from torch import nn
@@ -169,3 +171,34 @@ def test_group_members_serve_inference_tensors(monkeypatch):
         for m in group.members:
             assert m(x).shape == (4, M)
     assert [w.shape[0] for w in seen] == [M, M] and group.refresh()
+
+
+def test_expanded_operands_made_during_a_capture_are_not_kept(monkeypatch):
+    """What a capturing stream makes holds nothing before the graph runs, and its memory is the graph's."""
+    monkeypatch.setattr(serving, "expand_codes_f8", lambda p4: (p4["uq"].clone(), p4["vq"].clone()))
+    mod, capturing = _module(0), [True]
+    monkeypatch.setattr(serving, "_capturing", lambda t: capturing[0], raising=False)
+    first = mod._expanded()
+    assert mod._x8 is None and mod._expanded()[0] is not first[0]
+    capturing[0] = False
+    kept = mod._expanded()
+    capturing[0] = True
+    assert mod._expanded() is kept
+    twin = copy.deepcopy(mod)
+    assert twin._x8 is None and torch.equal(twin._expanded()[0], kept[0])
+
+
+@pytest.mark.gpu
+def test_expanded_operands_are_waited_for_on_another_stream():
+    """Two streams, the first use on one of them behind queued work: the other waits until the operands are there."""
+    mod = _module(0).cuda()
+    x = torch.randn(200, N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    want = _module(0).cuda()(x)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(100_000_000)
+    a = mod(x)
+    with torch.cuda.stream(side):
+        b = mod(x)
+    torch.cuda.synchronize()
+    assert torch.equal(a, want) and torch.equal(b, want)
