@@ -202,3 +202,18 @@ def test_expanded_operands_are_waited_for_on_another_stream():
         b = mod(x)
     torch.cuda.synchronize()
     assert torch.equal(a, want) and torch.equal(b, want)
+
+
+@pytest.mark.gpu
+def test_dimensions_of_a_stored_form_may_be_tensors():
+    """As a file's loader may leave them: one scratch buffer serves repeated calls."""
+    from ade_b200 import kernels
+
+    mod = _module(0).cuda()
+    p4 = {k: v if k in serving.STORED_KEYS else torch.tensor(v) for k, v in mod._stored_form().items()}
+    x = torch.randn(24, N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    want = mod(x)
+    buffers = len(kernels._scratch)
+    for _ in range(3):
+        assert torch.equal(kernels.module_forward(x, p4, mod.weight), want)
+    assert len(kernels._scratch) == buffers
