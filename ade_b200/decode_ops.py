@@ -33,8 +33,11 @@ def _launch(entry: str, dev: torch.device, *args) -> None:
 
 def _plain_inference(*tensors) -> bool:
     """Nothing records or transforms the operations on these tensors: no gradient, forward-mode or functorch level, no
-    tracing.  The reconstructed path of a long input is differentiable, so the operations around it have to stay so."""
+    tracing, no dispatch mode or tensor subclass (fake tensors, counters) that has to see them.  The reconstructed path of a
+    long input is differentiable, so the operations around it have to stay so."""
     if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return False
+    if torch._C._len_torch_dispatch_stack() or any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in tensors):
         return False
     return (torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
             and not torch.jit.is_tracing() and not torch.compiler.is_compiling())

@@ -187,3 +187,23 @@ def test_hidden_state_edited_in_place_between_layers(dev, mode, rows):
         with mode():
             logits.append(model(input_ids=ids, use_cache=False).logits.clone())
     assert _rel(*logits) < 2e-2
+
+
+def test_dispatch_modes_and_tensor_subclasses_see_the_operations(monkeypatch):
+    """Fake tensors, operation counters and wrapper tensors work through the operations a launch would hide."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Wrapped(torch.Tensor):
+        pass
+
+    monkeypatch.setattr(decode_ops, "_on_cuda", lambda t: True)
+    x, rows = torch.zeros(2, 400, 8, dtype=torch.bfloat16), 800
+    assert decode_ops._rows_ok(x, rows, x, torch.nn.Parameter(x, requires_grad=False))
+    assert not decode_ops._rows_ok(x, rows, x.as_subclass(Wrapped)) and not decode_ops._rows_ok(x.as_subclass(Wrapped), rows)
+    with Mode():
+        assert not decode_ops._rows_ok(x, rows, x)
+    assert decode_ops._rows_ok(x, rows, x)
