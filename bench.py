@@ -353,11 +353,11 @@ def sharded_recon_section(torch, dist, dev, rank, world, barrier):
         forms[i] = kernels.pack_int4(synth.random_packed(M, N, ranks[i], 5000 + i, dev, on_device=True), device=dev)
     outs = {shape: torch.empty(shape, dtype=torch.bfloat16, device=dev) for shape in uniq}
     status = torch.zeros(1, dtype=torch.int32, device=dev)
-    # one-shot reconstruction of a module: expand its codes to int8 operands in a work buffer shared by all modules
+    # one-shot reconstruction of a module: expand its codes to e4m3 operands in a work buffer shared by all modules
     # (two launches per module: the expansion is a few microseconds, the TMA-fed kernel saves more than that)
     small = [i for i in mine if ranks[i] <= 1024]
-    u8w = torch.empty(max([dims[i][0] * ranks[i] for i in small] + [16]), dtype=torch.int8, device=dev)
-    v8w = torch.empty(max([dims[i][1] * ranks[i] for i in small] + [16]), dtype=torch.int8, device=dev)
+    u8w = torch.empty(max([dims[i][0] * ranks[i] for i in small] + [16]), dtype=torch.uint8, device=dev)
+    v8w = torch.empty(max([dims[i][1] * ranks[i] for i in small] + [16]), dtype=torch.uint8, device=dev)
 
     def run_all():
         from ade_b200 import _lib
@@ -367,9 +367,9 @@ def sharded_recon_section(torch, dist, dev, rank, world, barrier):
         for i in mine:
             d = ctypes.byref(kernels._cdelta(forms[i]))
             if ranks[i] <= 1024:
-                _lib.check(lib.ade_b200_expand_codes(d, u8w.data_ptr(), v8w.data_ptr(), st), "ade_b200_expand_codes")
-                rc = lib.ade_b200_recon_expanded(d, u8w.data_ptr(), v8w.data_ptr(), bases[i].data_ptr(), outs[dims[i]].data_ptr(),
-                                                 None, status.data_ptr(), st)
+                _lib.check(lib.ade_b200_expand_codes_f8(d, u8w.data_ptr(), v8w.data_ptr(), st), "ade_b200_expand_codes_f8")
+                rc = lib.ade_b200_recon_expanded_f8(d, u8w.data_ptr(), v8w.data_ptr(), bases[i].data_ptr(), outs[dims[i]].data_ptr(),
+                                                    status.data_ptr(), st)
             else:
                 rc = lib.ade_b200_recon(d, bases[i].data_ptr(), outs[dims[i]].data_ptr(), None, status.data_ptr(), st)
             _lib.check(rc, "ade_b200_recon")
@@ -415,7 +415,7 @@ def sharded_recon_section(torch, dist, dev, rank, world, barrier):
     del forms, bases, outs, uniq
     torch.cuda.empty_cache()
     return {"workload": "llama-13b-shaped delta, 280 modules (5120/13824, ranks for alpha=1/16), W' = W_b + U^V^^T per module "
-                        "(codes expanded to int8 operands, then the TMA-fed kernel: two launches per module), "
+                        "(codes expanded to e4m3 operands, then the TMA-fed kernel: two launches per module), "
                         "modules split over ranks by cost d_o*d_i, no collective", "scaling": "strong",
             "ms_all_modules": ms, "modules_per_s": 280 / (ms * 1e-3), "gb_per_s_aggregate": total_bytes / (ms * 1e-3) / 1e9,
             "modules_on_slowest_rank": max(len(p) for p in plan), "rank0_bytes": nbytes,
@@ -489,7 +489,7 @@ def run_ade(args):
             if record:
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 e0.record()
-            W = m.merged_weight()             # the module's route: int8 operands expanded once at first use, kept
+            W = m.merged_weight()             # the module's route: e4m3 operands expanded once at first use, kept
             if record:
                 e1.record()
                 recon_ev.append((e0, e1))
@@ -551,7 +551,7 @@ def run_ade(args):
     t_wall1 = time.perf_counter()
     ms = s0.elapsed_time(s1)
     recon_ms = sum(a.elapsed_time(b) for a, b in recon_ev) / len(recon_ev)
-    # for the record: the same launches with the codes unpacked inside the kernel on every call (no kept int8 operands)
+    # for the record: the same modules without kept operands (rank 512: the codes are expanded on every call, two launches)
     pk = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
     for i in range(2 * len(mods) + 1):
         if i == len(mods):
@@ -560,21 +560,21 @@ def run_ade(args):
         kernels.recon_int4(m._stored_form(), m.weight)
     pk[1].record()
     torch.cuda.synchronize()
-    recon_packed_us = pk[0].elapsed_time(pk[1]) * 1e3 / (len(mods) + 1)
+    recon_one_shot_us = pk[0].elapsed_time(pk[1]) * 1e3 / (len(mods) + 1)
     # ... and the whole step that way (a few steps, for the record: the headline keeps the operands)
-    def step_unpacking():
+    def step_one_shot():
         for m, x in zip(mods, xs_dev):
             torch.nn.functional.linear(x, kernels.recon_int4(m._stored_form(), m.weight))
     for _ in range(2):
-        step_unpacking()
+        step_one_shot()
     pk2 = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
     n_alt = min(args.steps, 10)
     pk2[0].record()
     for _ in range(n_alt):
-        step_unpacking()
+        step_one_shot()
     pk2[1].record()
     torch.cuda.synchronize()
-    ms_step_unpacking = pk2[0].elapsed_time(pk2[1]) / n_alt
+    ms_step_one_shot = pk2[0].elapsed_time(pk2[1]) / n_alt
 
     # ---- end to end through the module API, host buffers in and out
     for i in range(4):
@@ -660,10 +660,10 @@ def run_ade(args):
             "gpu_launches": 3 * args.steps,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": RECON_TRAFFIC_BYTES, "traffic_source": "ncu capture of `bench.py --case recon`, not this run",
-                         "peak_kind": peak_kind, "kernel": "recon_strip_kernel (int8 operands expanded once per module and kept; "
+                         "peak_kind": peak_kind, "kernel": "recon_strip_kernel (e4m3 operands expanded once per module and kept; "
                          "algorithmic bytes count the packed codes)", "us_per_launch": recon_ms * 1e3,
-                         "us_per_launch_unpacking_in_kernel": recon_packed_us,
-                         "ms_per_step_unpacking_in_kernel": ms_step_unpacking,
+                         "us_without_kept_operands": recon_one_shot_us,
+                         "ms_per_step_without_kept_operands": ms_step_one_shot,
                          "int8_tops_kernel_only": (WORK_OPS / 3) / (recon_ms * 1e-3) / 1e12},
             "cpu_baseline": {"value": cpu_tops, "unit": UNIT, "cores": cpu_threads, "blas_threads": blas, "kind": "port",
                              "sample": f"{cpu_rows} of 11008 rows of gate_proj: reconstruct + base add + x W'^T, median of 5, {cpu_sec:.2f} s per pass"},
@@ -681,9 +681,10 @@ def run_case(argv):
     """One small fixed workload of a single kernel (seeded random packed fields, no SVD, well under 1 GB on the
     device), a handful of launches: what a profiler capture of two or three launches is taken on.
 
-        python bench.py --case recon [M N r [x]]      default 11008 4096 512 1 (Llama-2-7B gate_proj delta; x = 0: codes
-                                                      unpacked inside the kernel instead of int8 operands expanded beforehand)
+        python bench.py --case recon [M N r [x]]      default 11008 4096 512 1 (Llama-2-7B gate_proj delta; x = 0: without
+                                                      e4m3 operands expanded beforehand)
         python bench.py --case factored [T M N r]     default 16 4096 4096 256 (q_proj delta)
+        python bench.py --case delta [T M N r]        default 100 4096 11008 512 (down_proj delta behind a base term)
         python bench.py --case decode                 one graph replay of the 7B-architecture decode step (launch list)
     """
     import torch
@@ -697,12 +698,20 @@ def run_case(argv):
         p4 = kernels.pack_int4(synth.random_packed(M, N, r, 1), device=dev)
         W = synth.base_weight(M, N, 5).to(dev)
         status = torch.zeros(1, dtype=torch.int32, device=dev)
-        x8 = kernels.expand_codes(p4) if expanded else None
+        x8 = kernels.expand_codes_f8(p4) if expanded else None
         for _ in range(4):
             kernels.recon_int4(p4, W, status=status, expanded=x8)
         torch.cuda.synchronize()
-        print(f"recon {M}x{N} r={r} ({'int8 operands' if expanded else 'codes unpacked in the kernel'}): 4 launches, "
+        print(f"recon {M}x{N} r={r} ({'e4m3 operands' if expanded else 'no kept operands'}): 4 launches, "
               f"device status {int(status.item())}")
+    elif what == "delta":
+        T, M, N, r = nums if len(nums) == 4 else (100, 4096, 11008, 512)
+        p4 = kernels.pack_int4(synth.random_packed(M, N, r, 1), device=dev)
+        x, y = synth.activations(T, N, 6).to(dev), synth.activations(T, M, 7).to(dev)
+        for _ in range(4):
+            kernels.decode_forward_packed(x, y, p4)
+        torch.cuda.synchronize()
+        print(f"delta {M}x{N} r={r} T={T}: 4 launches, status {kernels.factored_status(dev, T, r)}")
     elif what == "factored":
         T, M, N, r = nums if len(nums) == 4 else (16, 4096, 4096, 256)
         p4 = kernels.pack_int4(synth.random_packed(M, N, r, 1), device=dev)
