@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(CQ_THREADS) compress_rows_kernel(const float* 
     const int ng = r >> 7, pitch = r + 4;
     __nv_bfloat16* stile = reinterpret_cast<__nv_bfloat16*>(cq_smem + static_cast<size_t>(pitch) * CQ_ROWS);   // [2 ng][CQ_ROWS]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float norm = ROT ? rsqrtf(static_cast<float>(r)) : 1.0f;     // exact for r = 4^k, else one rounding (as 1 / sqrt(r))
+    const float norm = ROT ? rsqrtf(static_cast<float>(r)) : 1.0f;     // exact for r = 4^k, else within rsqrtf's 2 ulp of 1 / sqrt(r)
     const int m0 = blockIdx.x * CQ_ROWS;
     const int nrows = min(CQ_ROWS, rows - m0);
     const int parts = ROT ? 1 : ng;                                     // pieces a row is taken in

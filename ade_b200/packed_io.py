@@ -8,8 +8,8 @@ What differs is how a file becomes something the kernels can read.  The referenc
 CPU, and each module constructor then packs nibbles and builds side tables with int64 torch ops on the CPU
 (src/kernels.py:145-188 called from src/serving.py:174-190): O(d r) host work per module, 224-280 modules per
 model.  Here ``PackedDeltaFile`` memory-maps the file, and ``DeviceDeltaLoader`` streams it module by module
-through a pinned staging buffer to the GPU, where the packing kernels of the C ABI (``ade_b200_pack_codes`` /
-``ade_b200_pack_zeros``) write ``uq / vq / vt / uz / vz`` straight into their final buffers on a side stream:
+through a pinned staging buffer to the GPU, where one launch per module (``ade_b200_pack_delta`` of the C ABI)
+writes ``uq / vq / vt / uz / vz`` straight into their final buffers on a side stream:
 the host only copies bytes, and the copy of module i+1 overlaps the packing of module i.
 """
 from __future__ import annotations
@@ -111,8 +111,8 @@ class DeviceDeltaLoader:
     """Builds device stored forms (the dict ``kernels.pack_int4`` returns) from packed modules in one pass.
 
     Per module: the six fields are copied into one pinned staging block (two blocks alternate), sent to the GPU
-    with one asynchronous copy on a side stream, and packed there by one launch of ``ade_b200_pack_delta``; scales are already in their final form.  The staging
-    blocks are sized for the largest module seen and reused.  ``finish()`` joins the side stream.
+    with one asynchronous copy on a side stream, and packed there by one launch of ``ade_b200_pack_delta``; scales are
+    already in their final form.  The side stream waits for the caller's before it writes.  The staging blocks are sized for the largest module seen and reused.  ``finish()`` joins the side stream.
     """
 
     def __init__(self, device="cuda"):

@@ -108,7 +108,7 @@ def compress_module(U, S, V, bits: int = 4, group_size: int = 128, generator=Non
 def compress_module_cuda(U, S, V, generator=None) -> dict:
     """compress_module on the GPU through ``ade_b200_compress_rows``: per factor one kernel that scales by sqrt(S),
     rotates (fast Walsh-Hadamard transform for a power-of-two rank; for other ranks the seeded random orthogonal H is
-    applied here with one dense matmul, as the reference does) and quantises the groups in shared memory.  4 bits,
+    applied here with one dense matmul, as the reference does) and quantises the groups in registers.  4 bits,
     groups of 128.  Returns the packed dict on the device of U."""
     from . import _lib
 
