@@ -66,3 +66,42 @@ def test_f8_operands_and_dump_are_exclusive():
     acc = torch.empty(1, 128, 128, dtype=torch.int32, device=DEV)
     with pytest.raises((RuntimeError, _lib.AdeKernelError)):
         kernels.recon_int4(p4, W, dbg_acc=acc, expanded=kernels.expand_codes_f8(p4))
+
+
+# both configurations and the unrolled one; 446 strips of one tile: every CTA walks three strips or more, so each us table is used a third time
+@pytest.mark.parametrize("r", [256, 512, 640])
+def test_three_strips_of_one_tile_per_cta(r):
+    M, N = 57000, 128
+    tp, W = synth.random_packed(M, N, r, r), synth.base_weight(M, N, 3)
+    p4, Wd = kernels.pack_int4(tp, device=DEV), W.to(DEV)
+    out = kernels.recon_int4(p4, Wd, expanded=kernels.expand_codes_f8(p4))
+    torch.cuda.synchronize()
+    _, merged = O.reconstruct(O.packed_from_torch(tp), base_bits=W.view(torch.uint16).numpy())
+    assert np.array_equal(out.cpu().view(torch.uint16).numpy(), merged)
+
+
+@pytest.mark.parametrize("pattern", ["uniform", "extremes", "one sign"])
+@pytest.mark.parametrize("r,group", [(128, 0), (384, 1), (512, 3), (1024, 0), (1024, 7)])
+def test_accumulators_are_exact_in_every_group(r, group, pattern):
+    """As above with one group of several looked at (the others have scale 0): codes and zero-points over their whole range, products of 0
+    and plus and minus 225, and products of one sign."""
+    M, N, ng = 200, 256, r // 128
+    g = torch.Generator().manual_seed(r + group)
+    uz, vz = torch.randint(0, 16, (M, ng), generator=g), torch.randint(0, 16, (ng, N), generator=g)
+    uc, vc = torch.randint(0, 16, (M, r), generator=g), torch.randint(0, 16, (r, N), generator=g)
+    if pattern == "extremes":
+        uz, vz = torch.randint(0, 2, (M, ng), generator=g) * 15, torch.randint(0, 2, (ng, N), generator=g) * 15
+        uc, vc = 15 - uz.repeat_interleave(128, 1), torch.randint(0, 2, (r, N), generator=g) * 15
+    elif pattern == "one sign":
+        uz, vz = torch.zeros(M, ng), torch.zeros(ng, N)
+        uc, vc = torch.randint(11, 16, (M, r), generator=g), torch.randint(11, 16, (r, N), generator=g)
+    us, vs = torch.zeros(M, ng), torch.zeros(ng, N)
+    us[:, group], vs[group] = 1, 1
+    tp = {"U_codes": uc.to(torch.uint8), "Vt_codes": vc.to(torch.uint8), "U_scale": us.to(torch.bfloat16), "Vt_scale": vs.to(torch.bfloat16),
+          "U_zero": uz.to(torch.bfloat16), "Vt_zero": vz.to(torch.bfloat16)}
+    k = slice(128 * group, 128 * group + 128)
+    P = (uc[:, k].double() - uz[:, group:group + 1].double()) @ (vc[k].double() - vz[group:group + 1].double())
+    W = (-P).to(torch.bfloat16)                         # 8 of at most 15 bits: the other 7 are what the result shows
+    p4 = kernels.pack_int4(tp, device=DEV)
+    out = kernels.recon_int4(p4, W.to(DEV), expanded=kernels.expand_codes_f8(p4)).cpu()
+    assert torch.equal(out.double(), W.double() + P)
