@@ -269,7 +269,7 @@ def _launch(op, x, p4, weight, y_dense):
     if not x.is_cuda or x.dim() != 2 or (weight is None) == (y_dense is None):
         _check_module_args(x, p4, weight, y_dense)
     dev = x.device
-    M, N, r, T = int(p4["M"]), int(p4["N"]), int(p4["r"]), x.shape[0]       # r is part of the scratch buffer's key: a number, not a tensor
+    r, T = int(p4["r"]), x.shape[0]                      # part of the scratch buffer's key: numbers, not tensors
     with _on_device(dev):
         stream = torch._C._cuda_getCurrentRawStream(dev.index)
         scratch = _scratch.get((dev.index, stream, T, r))
@@ -277,7 +277,7 @@ def _launch(op, x, p4, weight, y_dense):
             _check_module_args(x, p4, weight, y_dense)
             scratch = _scratch_for(dev, stream, T, r, _lib.load().ade_b200_factored_scratch_bytes(T, r))
         try:
-            return op(x, weight, y_dense, p4["uq"], p4["vq"], p4["vt"], p4["us"], p4["uz"], p4["vs"], p4["vz"], M, N, r,
+            return op(x, weight, y_dense, p4["uq"], p4["vq"], p4["vt"], p4["us"], p4["uz"], p4["vs"], p4["vz"], p4["M"], p4["N"], r,
                       _flat_blocks(p4), scratch)
         except RuntimeError as e:
             _check_module_args(x, p4, weight, y_dense)

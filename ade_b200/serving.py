@@ -31,18 +31,18 @@ def _capturing(t: torch.Tensor) -> bool:
 
 
 def _mark(t: torch.Tensor):
-    """(stream, event) behind what was just launched to make `t`; for `_join`."""
+    """(raw stream, event) behind what was just launched to make `t`; for `_join`."""
     if not t.is_cuda:
-        return None, None
+        return None
     stream, event = torch.cuda.current_stream(t.device), torch.cuda.Event()
     event.record(stream)
-    return stream, event
+    return stream.cuda_stream, event
 
 
-def _join(t: torch.Tensor, stream, event) -> None:
-    """Let the current stream wait for `event` unless it is the stream that recorded it."""
-    if stream is not None and torch.cuda.current_stream(t.device) != stream:
-        torch.cuda.current_stream(t.device).wait_event(event)
+def _join(t: torch.Tensor, mark) -> None:
+    """Let the current stream wait for `mark` unless it is the stream that made it.  A capture begins behind everything that was launched."""
+    if mark is not None and torch._C._cuda_getCurrentRawStream(t.device.index) != mark[0] and not _capturing(t):
+        torch.cuda.current_stream(t.device).wait_event(mark[1])
 
 
 class ADEKernelLinear(nn.Module):
@@ -84,44 +84,45 @@ class ADEKernelLinear(nn.Module):
         for k in STORED_KEYS:
             self.register_buffer(f"p4_{k}", p4[k])
         self._p4 = None
-        self._x8 = None               # ([(tensor, version)], (u8, v8), stream, event): expanded operands, what from, when; built on demand
+        self._x8 = None               # (stored form, (u8, v8), sum of versions, mark): expanded operands, built on demand
         self._group = None            # (FusedADEGroup, index) once fuse_kernel_linears has grouped this module
 
     def __getstate__(self):
         return {**self.__dict__, "_x8": None}         # a copy or a saved module makes its own (streams and events do not travel)
 
     def _tensor(self, name: str) -> torch.Tensor:
-        """self.<name> without the module's attribute lookup (0.2 us of every call) while it is a plain buffer; a caller may have made it a
-        parameter or parametrized it."""
+        """self.<name> without the module's attribute lookup while it is a plain buffer; a caller may have made it a parameter or
+        parametrized it."""
         t = self._buffers.get(name)
         return getattr(self, name) if t is None else t
 
     def _stored_form(self) -> dict:
         """Stored form on the module's device (rebuilt after .to(device))."""
-        if self._p4 is None or self._p4["uq"].data_ptr() != self._tensor("p4_uq").data_ptr():
-            self._p4 = {k: getattr(self, f"p4_{k}") for k in STORED_KEYS}
-            self._p4["M"], self._p4["N"], self._p4["r"] = self._dims
-        return self._p4
+        p4 = self._p4
+        if p4 is None or p4["uq"] is not self._tensor("p4_uq"):
+            p4 = self._p4 = {k: getattr(self, f"p4_{k}") for k in STORED_KEYS}
+            p4["M"], p4["N"], p4["r"] = self._dims
+        return p4
 
     def _expanded(self):
         """8-bit operands of the reconstruction kernel, built on the first long input and kept ((d_o + d_i) * r bytes) until the codes
         or zero-points they were made from are written to or replaced (load_state_dict).  EXPAND_FOR_RECON = False keeps the packed
         codes only; every call then unpacks them, inside the kernel or, from rank 384, into a buffer of that size for the call."""
-        p4 = self._stored_form()
+        p4, kept = self._stored_form(), self._x8
+        if kept is not None and kept[0] is p4 and kept[2] == p4["uq"]._version + p4["uz"]._version + p4["vq"]._version + p4["vz"]._version:
+            _join(kept[1][0], kept[3])
+            return kept[1]
         made_from = [p4[k] for k in ("uq", "uz", "vq", "vz")]
         if any(t.is_inference() for t in made_from):
             return None               # their contents can change unnoticed (no version counter): nothing is kept
-        if self._x8 is None or any(t is not old or t._version != v for t, (old, v) in zip(made_from, self._x8[0])):
-            new, kept = expand_codes_f8(p4), self._x8
-            if _capturing(new[0]):
-                return new            # they belong to the graph that is being captured and hold nothing before it runs
-            if kept is not None and kept[1][0].device == new[0].device and not kept[1][0].is_inference():
-                _join(kept[1][0], *kept[2:])
-                new = tuple(old.copy_(t) for old, t in zip(kept[1], new))       # the addresses stay: a captured graph may hold them
-            self._x8 = ([(t, t._version) for t in made_from], new, *_mark(new[0]))
-        elif not _capturing(self._x8[1][0]):                              # a capture begins behind everything that was launched
-            _join(self._x8[1][0], *self._x8[2:])
-        return self._x8[1]
+        new = expand_codes_f8(p4)
+        if _capturing(new[0]):
+            return new                # they belong to the graph that is being captured and hold nothing before it runs
+        if kept is not None and kept[1][0].device == new[0].device and not kept[1][0].is_inference():
+            _join(kept[1][0], kept[3])
+            new = tuple(old.copy_(t) for old, t in zip(kept[1], new))           # the addresses stay: a captured graph may hold them
+        self._x8 = (p4, new, sum(t._version for t in made_from), _mark(new[0]))
+        return new
 
     def merged_weight(self) -> torch.Tensor:
         """bf16(W_b + U^ V^^T), one launch of the reconstruction kernel."""
@@ -140,7 +141,8 @@ class ADEKernelLinear(nn.Module):
         if T <= self.decode_max_tokens:
             y = self._group[0].apply(self._group[1], x, x2) if self._group is not None and T <= FUSED_MAX_TOKENS else None
             if y is None:
-                y = module_forward(x2, self._stored_form(), self._tensor("weight"))
+                w = self._buffers.get("weight")
+                y = module_forward(x2, self._stored_form(), self.weight if w is None else w)
         else:
             y = F.linear(x2, self.merged_weight())
         return y if plain else y.reshape(*shape[:-1], self.out_features)
