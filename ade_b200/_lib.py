@@ -43,7 +43,7 @@ EXPORTS = (
     "ade_b200_device_status", "ade_b200_version", "ade_b200_last_cuda_error",
     "ade_b200_pack_codes", "ade_b200_pack_zeros", "ade_b200_pack_delta", "ade_b200_compress_rows",
     "ade_b200_factored_scratch_bytes", "ade_b200_factored_sync_offset", "ade_b200_factored",
-    "ade_b200_linear", "ade_b200_linear_workspace_bytes", "ade_b200_linear_preferred",
+    "ade_b200_linear", "ade_b200_linear_workspace_bytes", "ade_b200_linear_preferred", "ade_b200_linear_faster",
     "ade_b200_factored_static", "ade_b200_factored_static_status", "ade_b200_recon", "ade_b200_expand_codes",
     "ade_b200_recon_expanded", "ade_b200_expand_codes_f8", "ade_b200_recon_expanded_f8", "ade_b200_set_option",
     "ade_b200_rmsnorm", "ade_b200_add_rmsnorm", "ade_b200_rope", "ade_b200_silu_mul", "ade_b200_attn_decode",
@@ -103,6 +103,8 @@ def load() -> ctypes.CDLL:
     lib.ade_b200_linear.restype = ci
     lib.ade_b200_linear_preferred.argtypes = [ci, ci, ci]
     lib.ade_b200_linear_preferred.restype = ci
+    lib.ade_b200_linear_faster.argtypes = [ci] * 5
+    lib.ade_b200_linear_faster.restype = ci
     lib.ade_b200_recon.argtypes = [ctypes.POINTER(AdeDelta), vp, vp, vp, vp, vp]
     lib.ade_b200_expand_codes.argtypes = [ctypes.POINTER(AdeDelta), vp, vp, vp]
     lib.ade_b200_expand_codes_f8.argtypes = [ctypes.POINTER(AdeDelta), vp, vp, vp]

@@ -200,6 +200,16 @@ int launch_small(Kernel kernel, int grid, int threads, size_t smem, void* stream
     return cuda_ok(cudaGetLastError()) ? ADE_OK : ADE_ERR_CUDA;
 }
 
+// Stages of the warp-MMA kernel's W_b FIFO: what shared memory has left beside `smem` bytes of other buffers; 0 = register prefetch.
+// Up to 8 tokens, or up to 16 with a long stream per CTA, W_b goes through a shared-memory FIFO (deeper than registers allow).  At
+// 9-16 tokens a short stream (a 4096 x 4096 module is 227 KB per CTA) is as fast with the register prefetch: the deep FIFO raises
+// the loaded memory latency, which the h hand-over pays several times.
+int fifo_stages(int NT, size_t smem, long long M, long long N, int grid) {
+    if (!ade::fa_side(NT) || !(NT == 1 || static_cast<size_t>(M * N * 2 / grid) >= kFifoMinStream)) return 0;
+    const size_t room = (static_cast<size_t>(kMaxSmem) - smem) / ade::fa_fifo_item(NT);
+    return room >= 2 ? static_cast<int>(room < static_cast<size_t>(ade::FA_FIFO_MAX) ? room : ade::FA_FIFO_MAX) : 0;
+}
+
 template <int NT, bool FUSE>
 int launch_factored_one(ade::FactoredParams p, int grid, cudaStream_t st) {
     size_t smem = ade::factored_smem_bytes(NT, p.rows_cap, p.T, p.r);
@@ -207,13 +217,8 @@ int launch_factored_one(ade::FactoredParams p, int grid, cudaStream_t st) {
     p.upf = 0;
     p.spin_limit = g_wait_limit;
     p.drop_arrivals = g_drop_signals;
-    // Up to 8 tokens, or up to 16 with a long stream per CTA: W_b goes through a shared-memory FIFO (deeper than
-    // registers allow).  At 9-16 tokens a short stream (a 4096 x 4096 module is 227 KB per CTA) is as fast with the
-    // register prefetch: the deep FIFO raises the loaded memory latency, which the h hand-over pays several times.
-    const size_t stream_bytes = static_cast<size_t>(p.M) * p.N * 2 / static_cast<size_t>(grid);
-    if (FUSE && ade::fa_side(NT) && (NT == 1 || stream_bytes >= kFifoMinStream)) {
-        const size_t room = (static_cast<size_t>(kMaxSmem) - smem) / ade::fa_fifo_item(NT);
-        p.stages = room >= 2 ? static_cast<int>(room < static_cast<size_t>(ade::FA_FIFO_MAX) ? room : ade::FA_FIFO_MAX) : 0;
+    if (FUSE) {
+        p.stages = fifo_stages(NT, smem, p.M, p.N, grid);
         smem += static_cast<size_t>(p.stages) * ade::fa_fifo_item(NT);
     }
     p.hstage = 0;
@@ -473,13 +478,41 @@ int ade_b200_factored(const ade_delta_t* d, const void* x, const void* y_dense, 
     return launch_factored<16>(p, grid, st);
 }
 
-// With y_dense, the tensor-core kernel against the warp-MMA kernel, per call with the library GEMM of the base term in front, in us:
-// 4096 x 4096 r = 512 T = 32 27.6 / 23.3, T = 40 29.5 / 27.3, T = 65 32.8 / 36.5, T = 128 37.5 / 40.1; 5000 x 5120 r = 896 T = 32 38.0 / 35.4,
-// T = 40 38.7 / 45.9, T = 128 49.5 / 109; 11008 x 4096 r = 512 T = 32 39.5 / 38.7, T = 40 42.7 / 48.7, T = 128 46.8 / 73.1; 4096 x 11008 T = 40
-// 43.6 / 41.8, T = 100 50.6 / 63.9.  The warp-MMA kernel slows down with M r (its U^ h) whenever the tokens pass a power of two.
-int ade_b200_linear_preferred(int T, int M, int r) {
-    return T > 64 || (T > 32 && static_cast<long long>(M) * r >= 4000000);
+// Which of the two kernels is faster, per call in a graph over rotated weights (with y_dense: the library GEMM of the base term in front),
+// warp-MMA / tensor-core in us.  The warp-MMA kernel is priced by its steps: row blocks of 32 per SM, token tiles of 8 doubled at 17,
+// 33 and 65, and what shared memory has room for; the tensor-core kernel by the hand-overs of h and 64 ranks of U^ h at a time.
+int ade_b200_linear_faster(int T, int M, int N, int r, int with_base) {
+    const DeviceInfo* di = nullptr;
+    if (T < 1 || T > ADE_B200_MAX_TOKENS || M < 1 || N < 1 || r < ADE_B200_GROUP || device_info(&di)) return 0;
+    const int rows = (M + di->sms - 1) / di->sms, rows_cap = (rows + 1 + 31) / 32 * 32;
+    if (rows > ade::LT_MAX_SEG * ade::LT_TILE) return 0;
+    if (with_base) {
+        // From 9 tokens the warp-MMA kernel no longer hides U^ h under its stream (22016 x 4096 r = 512 T = 8 36.9 / 48.3, T = 12 44.2 / 40.6);
+        // it shows where the stream is long: 12288 x 4096 (q/k/v) T = 16 41.7 / 42.7.  The tensor-core kernel hides U^ h only while there
+        // are about six columns per rank: 22016 x 4096 r = 768 T = 12 45.3 / 43.1 but 18944 rows 37.4 / 39.6; 22016 x 1024 r = 512 24.3 / 25.1.
+        // (Up to rank 256 there is too little of it to matter: 22016 x 1024 24.1 / 20.5.)
+        if (T <= 8 || T > 16 || M < 16384) return 0;
+        if (r <= 256 || 6ll * r <= N) return 1;
+        // Where h leaves the warp-MMA kernel's FIFO two stages it loses a quarter at once: 22016 x 4096 r = 1024 T = 15 47.8 / 46.4, T = 16
+        // 60.8 / 46.6.  Not worth it with two columns per rank and less: 22016 x 4096 r = 2048 T = 12 65.0 / 65.8, x 3072 54.0 / 62.4.
+        return N > 2 * r && fifo_stages(2, ade::factored_smem_bytes(2, rows_cap, T, r), M, N, di->sms) == 2;
+    }
+    // Up to 32 tokens the warp-MMA kernel is ahead (4096 x 4096 r = 512 T = 32 23.4 / 27.4, 13824 x 4096 42.0 / 43.8; at the next token 26.5 / 29.3
+    // and 41.9 / 37.4), up to 64 with little of U^ h (8192 x 1024 r = 256 T = 48 23.2 / 23.6, r = 512 27.1 / 26.2).
+    if (T <= 32 || (T <= 64 && static_cast<long long>(M) * r < 4000000)) return 0;
+    // A second row block per SM: 4736 x 4096 r = 512 T = 65 35.9 / 34.7, 4800 rows 45.1 / 35.8; r = 896 T = 48 34.8 / 36.5, 42.8 / 37.6.
+    if (rows > 32) return 1;
+    // h no longer fits beside the rows: 2048 x 2048 r = 896 T = 88 38.4 / 38.6, T = 104 57.9 / 39.9.
+    const int nt = T <= 64 ? 8 : 16;
+    if (ade::factored_smem_bytes(nt, rows_cap, T, r) + ade::fa_side_region(T, r) > static_cast<size_t>(kMaxSmem)) return 1;
+    // One row block and h in shared memory is the warp-MMA kernel's best ground.  It loses it with V^T x, which grows with N.
+    // 4096 rows, r = 1024 T = 40: x 6144 38.7 / 40.3, x 11008 53.1 / 51.3; r = 1280 x 4096 37.7 / 40.3, x 6144 45.6 / 44.4.
+    if (T <= 64) return N >= 8192 || (N >= 6144 && r >= 1280);
+    // T = 72: x 1536 r = 768 36.2 / 35.1, r = 1024 38.9 / 40.6; r = 1024 x 4096 47.3 / 47.0.  T = 80: x 1024 r = 256 24.0 / 23.6, r = 512 27.4 / 29.1.
+    return r <= 256 || (N >= 1152 && r <= 768) || N >= 4096;
 }
+
+int ade_b200_linear_preferred(int T, int M, int r) { return ade_b200_linear_faster(T, M, 13824, r, 0); }
 
 size_t ade_b200_linear_workspace_bytes(int T, int M, int r) {
     const DeviceInfo* di = nullptr;
@@ -585,7 +618,7 @@ int ade_b200_factored_static(const ade_delta_t* d, const void* x, const void* y_
     // the array keeps whatever the previous call left: the four sync words must start at zero (the status word
     // behind them is sticky until ade_b200_factored_static_status clears it)
     if (!cuda_ok(cudaMemsetAsync(base, 0, 16, st))) return ADE_ERR_CUDA;
-    if (y_dense && ade_b200_linear_preferred(T, d->M, d->r) && di->sms <= kStaticGrid) {
+    if (y_dense && ade_b200_linear_faster(T, d->M, d->N, d->r, 0) && di->sms <= kStaticGrid) {
         unsigned int* sync = reinterpret_cast<unsigned int*>(base);
         return launch_linear(d, x, y_dense, nullptr, out, reinterpret_cast<__nv_bfloat16*>(base + 256), sync, sync + 4,
                              base + ADE_B200_STATIC_SCRATCH_BYTES, kStaticWorkspace, T, stream);

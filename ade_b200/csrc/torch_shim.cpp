@@ -69,8 +69,8 @@ ade_delta_t make_delta(const at::Tensor& uq, const at::Tensor& vq, const at::Ten
     return d;
 }
 
-// TC: the tensor-core kernel (ade_b200_linear) in any case, else where it is preferred for a call with y_dense; its workspace comes from torch's caching allocator (stream-ordered, so calls on other
-// streams and graph captures get memory of their own).
+// TC: the tensor-core kernel (ade_b200_linear) in any case, else where it is the faster one for a call with y_dense; its workspace comes from
+// torch's caching allocator (stream-ordered, so calls on other streams and graph captures get memory of their own).
 template <bool TC>
 at::Tensor factored(const at::Tensor& x, const c10::optional<at::Tensor>& weight, const c10::optional<at::Tensor>& y_dense,
                     const at::Tensor& uq, const at::Tensor& vq, const at::Tensor& vt, const at::Tensor& us, const at::Tensor& uz,
@@ -96,7 +96,7 @@ at::Tensor factored(const at::Tensor& x, const c10::optional<at::Tensor>& weight
     const void* wb = weight.has_value() ? weight->data_ptr() : nullptr;
     void* stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
     int rc;
-    if (TC || (yd && ade_b200_linear_preferred(static_cast<int>(T), d.M, d.r))) {
+    if (TC || (yd && ade_b200_linear_faster(static_cast<int>(T), d.M, d.N, d.r, 0))) {
         const size_t wbytes = ade_b200_linear_workspace_bytes(static_cast<int>(T), d.M, d.r);
         const at::Tensor work = at::empty({static_cast<int64_t>(wbytes)}, x.options().dtype(at::kByte));
         rc = ade_b200_linear(&d, x.data_ptr(), yd, wb, out.data_ptr(), scratch.data_ptr(), static_cast<size_t>(scratch.nbytes()), work.data_ptr(),

@@ -288,7 +288,7 @@ def factored_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor | None = No
                      y_dense: torch.Tensor | None = None) -> torch.Tensor:
     """out = base + U^(V^T x) for T <= 128 tokens; base = x W_b^T computed in-kernel when `weight`
     is given, else the supplied `y_dense`.  One launch: ``ade_b200_factored``, or with `y_dense` ``ade_b200_linear`` where
-    ``ade_b200_linear_preferred`` says so."""
+    ``ade_b200_linear_faster`` says so."""
     return _launch(_lib.ops().factored, x, p4, weight, y_dense)
 
 
@@ -300,10 +300,9 @@ def linear_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor) -> torch.Ten
     return _launch(_lib.ops().linear, x, p4, weight, None)
 
 
-# Up to this many tokens the base GEMM runs in the launch of the delta: the warp-MMA kernel (`ade_b200_factored`), or for modules of
-# TALL_ROWS rows and more (the fused gate/up groups) above 8 tokens the tensor-core kernel (`ade_b200_linear`), because the former no
-# longer hides U^ h under its stream there.  Per call on B200 in a graph over rotated weights, former / latter in us: 22016 x 4096 T = 8
-# 36.9 / 48.3, T = 16 62.5 / 49.1; 27648 x 5120 T = 16 86.2 / 59.9; 12288 x 4096 (q/k/v) T = 16 41.7 / 42.7; 4096 x 4096 T = 16 13.9 / 18.3.
+# Up to this many tokens the base GEMM runs in the launch of the delta: the warp-MMA kernel (`ade_b200_factored`), or the tensor-core kernel
+# (`ade_b200_linear`) where `ade_b200_linear_faster` says so, which is asked above 8 tokens for modules of TALL_ROWS rows and more (the
+# fused gate/up groups) only: it says no everywhere else.
 FUSED_MAX_TOKENS = 16
 TALL_ROWS = 16384
 TALL_FACTORED_MAX_TOKENS = 8
@@ -315,7 +314,7 @@ def module_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor) -> torch.Ten
     T = x.shape[0]
     if T > FUSED_MAX_TOKENS:
         return decode_forward_packed(x, torch.nn.functional.linear(x, weight), p4)
-    if T > TALL_FACTORED_MAX_TOKENS and weight.shape[0] >= TALL_ROWS:
+    if T > TALL_FACTORED_MAX_TOKENS and weight.shape[0] >= TALL_ROWS and _lib.load().ade_b200_linear_faster(T, *weight.shape, int(p4["r"]), 1):
         return linear_forward(x, p4, weight)
     return factored_forward(x, p4, weight=weight)
 

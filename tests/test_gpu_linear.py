@@ -118,3 +118,62 @@ def test_module_dispatch_edges(M, T):
     ref = O.factored_apply(x.view(torch.uint16).numpy(), W.view(torch.uint16).numpy(), O.packed_from_torch(tp))
     err, cos = O.parity(y.float().cpu().numpy(), ref)
     assert err <= 1e-2 and cos >= 0.9999, (err, cos)
+
+
+def _direct(entry, x, p4, y=None, W=None):
+    """One of the two kernels by its C entry, whatever the dispatch says."""
+    import ctypes
+
+    lib, (T, M, r) = _lib.load(), (x.shape[0], p4["M"], p4["r"])
+    out = torch.empty(T, M, dtype=torch.bfloat16, device=DEV)
+    scratch = torch.zeros(lib.ade_b200_factored_scratch_bytes(T, r), dtype=torch.uint8, device=DEV)
+    args = [ctypes.byref(kernels._cdelta(p4)), x.data_ptr(), None if y is None else y.data_ptr(), None if W is None else W.data_ptr(),
+            out.data_ptr(), scratch.data_ptr(), scratch.numel()]
+    work = torch.empty(lib.ade_b200_linear_workspace_bytes(T, M, r), dtype=torch.uint8, device=DEV)
+    if entry == "linear":
+        args += [work.data_ptr(), work.numel()]
+    assert getattr(lib, f"ade_b200_{entry}")(*args, T, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    return out
+
+
+# both sides of every line of the rule for calls with y_dense: tokens, rows times rank, rows per SM, h in shared memory, columns and rank
+@pytest.mark.parametrize("M,N,r,T,linear", [(31250, 128, 128, 32, 0), (31250, 128, 128, 33, 1), (31249, 128, 128, 33, 0), (31249, 128, 128, 65, 1),
+                                            (4736, 384, 384, 65, 0), (4737, 384, 384, 65, 1), (4736, 128, 256, 128, 1), (600, 384, 1024, 87, 0),
+                                            (600, 384, 1024, 90, 1), (500, 1152, 768, 80, 1), (500, 1024, 768, 80, 0), (500, 1152, 896, 80, 0),
+                                            (300, 4096, 896, 66, 1), (4000, 8192, 1024, 40, 1), (4000, 8064, 1024, 40, 0), (3200, 6144, 1280, 34, 1)])
+def test_supplied_base_term_takes_the_kernel_of_the_rule(M, N, r, T, linear):
+    assert _lib.load().ade_b200_linear_faster(T, M, N, r, 0) == linear
+    p4 = kernels.pack_int4(synth.random_packed(M, N, r, M + T, DEV, on_device=True))
+    x, y = synth.activations(T, N, 1).to(DEV), synth.activations(T, M, 2).to(DEV)
+    by = {e: _direct(e, x, p4, y) for e in ("factored", "linear")}
+    assert torch.equal(kernels.decode_forward_packed(x, y, p4), by["linear" if linear else "factored"])
+    err, cos = O.parity(by["linear"].float().cpu().numpy(), by["factored"].float().cpu().numpy())
+    assert err <= 1e-2 and cos >= 0.9999, (err, cos)
+
+
+# the rule for calls with the base weight: rows, tokens, rank against columns, and where h takes the third FIFO stage (with two columns per rank)
+@pytest.mark.parametrize("M,N,r,T,linear", [(16383, 128, 128, 9, 0), (16384, 128, 256, 8, 0), (16384, 128, 256, 9, 1), (16384, 128, 384, 9, 0),
+                                            (16384, 2304, 384, 16, 1), (16384, 2176, 384, 16, 0), (22016, 2176, 1024, 15, 0), (22016, 2176, 1024, 16, 1),
+                                            (22016, 2048, 1024, 16, 0)])
+def test_module_takes_the_kernel_of_the_rule(M, N, r, T, linear):
+    assert (_lib.load().ade_b200_linear_faster(T, M, N, r, 1) == 1) == bool(linear)
+    p4 = kernels.pack_int4(synth.random_packed(M, N, r, M + T, DEV, on_device=True))
+    x, W = synth.activations(T, N, 1).to(DEV), synth.base_weight(M, N, 2).to(DEV)
+    by = {e: _direct(e, x, p4, W=W) for e in ("factored", "linear")}
+    assert torch.equal(kernels.module_forward(x, p4, W), by["linear" if linear else "factored"])
+    err, cos = O.parity(by["linear"].float().cpu().numpy(), by["factored"].float().cpu().numpy())
+    assert err <= 1e-2 and cos >= 0.9999, (err, cos)
+
+
+# the form with y_dense on both ways U^ h is prepared (64 / 65 tokens), one to three slices per SM, ragged rows, the highest rank, fewer rows
+# than SMs, whatever the dispatch would take
+@pytest.mark.parametrize("M,N,r,T", [(5000, 256, 896, 17), (4097, 384, 1024, 47), (129, 128, 256, 64), (129, 128, 256, 65), (300, 1024, 2048, 100),
+                                     (19000, 128, 256, 40), (38000, 128, 128, 128), (1, 128, 128, 1)])
+def test_supplied_base_term_by_its_entry(M, N, r, T):
+    tp, W, x = _case(M, N, r, T)
+    p4, xd = kernels.pack_int4(tp, device=DEV), x.to(DEV)
+    y = _direct("linear", xd, p4, torch.nn.functional.linear(xd, W.to(DEV)))
+    ref = O.factored_apply(x.view(torch.uint16).numpy(), W.view(torch.uint16).numpy(), O.packed_from_torch(tp))
+    err, cos = O.parity(y.float().cpu().numpy(), ref)
+    assert err <= 1e-2 and cos >= 0.9999, (err, cos)
