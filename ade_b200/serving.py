@@ -31,18 +31,21 @@ def _capturing(t: torch.Tensor) -> bool:
 
 
 def _mark(t: torch.Tensor):
-    """(raw stream, event) behind what was just launched to make `t`; for `_join`."""
+    """The stream that was just given the launch that makes `t`, and the raw streams that need not wait for it; for `_join`."""
     if not t.is_cuda:
         return None
-    stream, event = torch.cuda.current_stream(t.device), torch.cuda.Event()
-    event.record(stream)
-    return stream.cuda_stream, event
+    stream = torch.cuda.current_stream(t.device)
+    return stream, {stream.cuda_stream}
 
 
 def _join(t: torch.Tensor, mark) -> None:
-    """Let the current stream wait for `mark` unless it is the stream that made it.  A capture begins behind everything that was launched."""
-    if mark is not None and torch._C._cuda_getCurrentRawStream(t.device.index) != mark[0] and not _capturing(t):
-        torch.cuda.current_stream(t.device).wait_event(mark[1])
+    """Let the current stream wait for the stream of `mark`, once.  A capture begins behind everything that was launched."""
+    if mark is None:
+        return
+    raw = torch._C._cuda_getCurrentRawStream(t.device.index)
+    if raw not in mark[1] and not _capturing(t):
+        torch.cuda.current_stream(t.device).wait_stream(mark[0])
+        mark[1].add(raw)
 
 
 class ADEKernelLinear(nn.Module):
