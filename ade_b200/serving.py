@@ -35,14 +35,14 @@ def _mark(t: torch.Tensor):
     if not t.is_cuda:
         return None
     stream = torch.cuda.current_stream(t.device)
-    return stream, {stream.cuda_stream}
+    return stream, {stream.cuda_stream}, t.device.index
 
 
 def _join(t: torch.Tensor, mark) -> None:
     """Let the current stream wait for the stream of `mark`, once.  A capture begins behind everything that was launched."""
     if mark is None:
         return
-    raw = torch._C._cuda_getCurrentRawStream(t.device.index)
+    raw = torch._C._cuda_getCurrentRawStream(mark[2])
     if raw not in mark[1] and not _capturing(t):
         torch.cuda.current_stream(t.device).wait_stream(mark[0])
         mark[1].add(raw)
@@ -107,11 +107,11 @@ class ADEKernelLinear(nn.Module):
             p4["M"], p4["N"], p4["r"] = self._dims
         return p4
 
-    def _expanded(self):
+    def _expanded(self, p4: dict | None = None):
         """8-bit operands of the reconstruction kernel, built on the first long input and kept ((d_o + d_i) * r bytes) until the codes
         or zero-points they were made from are written to or replaced (load_state_dict).  EXPAND_FOR_RECON = False keeps the packed
         codes only; every call then unpacks them, inside the kernel or, from rank 384, into a buffer of that size for the call."""
-        p4, kept = self._stored_form(), self._x8
+        p4, kept = p4 or self._stored_form(), self._x8
         if kept is not None and kept[0] is p4 and kept[2] == p4["uq"]._version + p4["uz"]._version + p4["vq"]._version + p4["vz"]._version:
             _join(kept[1][0], kept[3])
             return kept[1]
@@ -130,8 +130,8 @@ class ADEKernelLinear(nn.Module):
     def merged_weight(self) -> torch.Tensor:
         """bf16(W_b + U^ V^^T), one launch of the reconstruction kernel."""
         p4 = self._stored_form()
-        expanded = self._expanded() if EXPAND_FOR_RECON and p4["r"] <= 1024 else None
-        return recon_int4(p4, self.weight, self.group_size, expanded=expanded)
+        expanded = self._expanded(p4) if EXPAND_FOR_RECON and p4["r"] <= 1024 else None
+        return recon_int4(p4, self._tensor("weight"), self.group_size, expanded=expanded)
 
     def forward(self, x):
         """x (..., d_i) -> (..., d_o) in bfloat16."""
