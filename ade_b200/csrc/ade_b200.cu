@@ -44,9 +44,6 @@ long long g_wait_limit = ade::RC_SPIN_LIMIT;   // clock cycles a device-side wai
 int g_cooperative = 1;                         // factored kernel launched cooperatively (co-residency guaranteed)
 int g_drop_signals = 0;                        // diagnostic: producers inside the kernels stay silent
 int g_attn_single_pass = 1;                    // attention step: the single-pass kernel where the head dimension allows it
-#ifdef ADE_TRACE
-unsigned long long* g_trace = nullptr;         // development builds: device buffer for event stamps (option 100)
-#endif
 
 template <int NT>
 bool optin_factored();
@@ -316,7 +313,7 @@ int set_blocks(Params& p, const ade_delta_t* d) {
 // code this name is only a handle for cudaGetSymbolAddress.
 // Behind it the workspace of the tensor-core kernel, which serves the calls with y_dense that it is preferred for.
 constexpr int kStaticGrid = 160;
-constexpr size_t kStaticWorkspace = static_cast<size_t>(kStaticGrid) * (ADE_B200_MAX_TOKENS * 128 * sizeof(float) + sizeof(unsigned int));
+constexpr size_t kStaticWorkspace = static_cast<size_t>(kStaticGrid) * ADE_B200_MAX_TOKENS * 128 * sizeof(float);
 static_assert(ADE_B200_STATIC_SCRATCH_BYTES % 256 == 0, "the workspace behind the scratch array keeps its alignment");
 __device__ __align__(256) unsigned char g_static_scratch[ADE_B200_STATIC_SCRATCH_BYTES + kStaticWorkspace];
 void* g_static_scratch_addr[kMaxDevices] = {};
@@ -531,10 +528,9 @@ static int launch_linear(const ade_delta_t* d, const void* x, const void* y_dens
     ade::LinearParams p = {};
     p.tpad = (T + 15) / 16 * 16;
     ade::LinearSplit split;
-    if (!ade::linear_split(d->M, d->N, T, p.tpad, grid, w_b != nullptr, split)) return ADE_ERR_SHAPE;
+    if (!ade::linear_split(d->M, T, p.tpad, grid, split)) return ADE_ERR_SHAPE;
     p.slices = split.slices;
     p.segs = split.segs;
-    p.ksplit = split.ksplit;
     p.rows = split.rows;
     p.stages = split.stages;
     p.u_start = split.u_start;
@@ -550,7 +546,6 @@ static int launch_linear(const ade_delta_t* d, const void* x, const void* y_dens
     p.status = status;
     p.y_dense = static_cast<const __nv_bfloat16*>(y_dense);
     p.part = static_cast<float*>(workspace);
-    p.slice_count = reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + ade::linear_part_bytes(T, grid));
     p.out = static_cast<__nv_bfloat16*>(out);
     p.T = T;
     p.M = d->M;
@@ -567,9 +562,6 @@ static int launch_linear(const ade_delta_t* d, const void* x, const void* y_dens
     if (rc) return rc;
     p.spin_limit = g_wait_limit;
     p.drop_arrivals = g_drop_signals;
-#ifdef ADE_TRACE
-    p.trace = g_trace;
-#endif
     if (!load_encode_tiled()) return ADE_ERR_CUDA;
     ade::LinearMaps maps;
     const uint64_t N = static_cast<uint64_t>(d->N);
@@ -775,11 +767,6 @@ int ade_b200_set_option(int option, long long value) {
         case ADE_OPT_ATTN_SINGLE_PASS:
             g_attn_single_pass = value != 0;
             return ADE_OK;
-#ifdef ADE_TRACE
-        case 100:
-            g_trace = reinterpret_cast<unsigned long long*>(static_cast<uintptr_t>(value));
-            return ADE_OK;
-#endif
         default:
             return ADE_ERR_SHAPE;
     }
@@ -858,10 +845,6 @@ static int recon_impl(const ade_delta_t* d, const void* u8, const void* v8, bool
     p.one = 1.0f;
     p.spin_limit = g_wait_limit;
     p.drop_loads = g_drop_signals;
-    p.trace = nullptr;
-#ifdef ADE_TRACE
-    p.trace = g_trace;
-#endif
     const int ng = d->r / ADE_B200_GROUP;
     const int ntiles = ((d->M + ade::RC_TILE - 1) / ade::RC_TILE) * (d->N / ade::RC_TILE);
     const int grid = ntiles < di->sms ? ntiles : di->sms;

@@ -1,32 +1,31 @@
-// One delta linear module  out = x W_b^T + U^ (V^T x)  for up to 128 token rows, one launch, every contraction on the
-// 5th-generation tensor cores.
+// One delta linear module  out = base + U^ (V^T x)  for up to 128 token rows, one launch, every contraction on the 5th-generation
+// tensor cores.  The base term is either supplied (y_dense: what modules of 33-128 tokens take behind the library GEMM, in place of the
+// reference's kernels A and B, src/kernels.py:486-886) or x W_b^T, streamed here (w_b: tall fused groups at 9-16 tokens).  Which calls come
+// here is decided by ade_b200_linear_faster.
 //
-// Replaces, per call, the library GEMM of the base term and the reference's kernels A and B behind it
-// (src/kernels.py:486-886, src/serving.py:106-111).  The weights are the 128-row operand of tcgen05.mma (K-major, bf16), the
-// token rows the N operand (padded to a multiple of 16), the accumulators stay in tensor memory for the whole launch.
-//
-// What bounds it: the stream of W_b from HBM, and for short streams the two grid-wide hand-overs of h.  Rows are cut into
-// equal slices, so every SM streams the same number of bytes.  With one slice per SM (ksplit = 1) nothing has to be combined
-// afterwards, but every SM reads all of x (from L2); when x would cost more than the weights do, slices are ksplit times as
-// tall and ksplit SMs share one, each taking a part of the columns and exchanging float32 partial sums through global scratch
-// in a fixed order (the rule is linear_split below).
+// The weights are the 128-row operand of tcgen05.mma (K-major, bf16), the token rows the N operand (padded to a multiple of 16), the
+// accumulators stay in tensor memory for the whole launch.  Rows are cut into equal slices, one to three per SM, so that every SM streams
+// and multiplies the same; every SM reads all of x (from L2).
 //
 // Everything a CTA multiplies goes through ONE ring of shared-memory stages (A part: up to 128 rows x 128 columns,
 // B part: the token rows of the same columns), in this order:
 //   A items   h = V^T x: the (rank group, 128-column block) pairs are dealt to all CTAs.  A = (code - zero) * scale, one bf16
 //             rounding, written by the eight unpack warps; B = x by TMA.  The float32 partial sums of h go to scratch; when
 //             all have arrived every CTA adds its share of the T x r elements, rounds to bf16 once and publishes it.
-//   W items   the CTA's part of W_b: A and B by TMA.  While the tensor core works through them, the unpack warps do the h
+//   W items   the CTA's slices of W_b: A and B by TMA.  While the tensor core works through them, the unpack warps do the h
 //             exchange above: the hand-overs are hidden under the stream as far as it is long enough.
 //             (With a base term from the caller there are no W items; its values are added at the end.)
 //   U items   U^ h on top of the same accumulators, 64 ranks at a time, spread over the end of the stream.  The scale of a (row, group) belongs to
 //             the row, so it is multiplied into the A operand; scale (8 significant bits) times code - zero (4) is 12 bits,
 //             which is exactly the sum of two bf16 values hi + lo: two MMA passes share one B tile of h and the product is
 //             exact, as when the scale was applied to the float32 sums.
-// Measured (us per call in a graph over rotated weights, library GEMM + warp-MMA delta launch before): 4096 x 4096 r = 512 T = 40 27.8 -> 19.4
-// (its bytes take 5.4; the stream has ended after 9, h is there after 11.5, U^ h after 14, the exchange of partial sums takes 4);
-// 4096 x 11008 T = 100 63.6 -> 28.9; 11008 x 4096 T = 128 73.3 -> 35.5; 5000 x 5120 r = 896 T = 40 45.3 -> 25.8; 22016 x 4096 (a fused
-// group) T = 32 49.8.  One 64-column block per ring item took 36 and 70 us on the two tall ones: the issuing warp bound them.
+//
+// What bounds it: with y_dense the chain of the two grid-wide hand-overs of h (partial sums visible, sums published: 3-5 us each under a
+// loaded memory system) and of the U items behind them; with w_b the stream of W_b beside that chain.
+// Measured (us per launch in a graph over rotated weights, warp-MMA kernel / this one).  Behind a given base term: 5000 x 5120 r = 896 T = 40
+// 32.8 / 25.2, 4096 x 11008 r = 512 T = 100 42.4 / 26.6, 11008 x 4096 T = 128 52.9 / 25.7, 13824 x 5120 r = 640 T = 64 36.4 / 26.3, but 4096 x 4096
+// r = 256 T = 64 16.0 / 16.1.  Base inside: 22016 x 4096 r = 1024 T = 16 60.5 / 45.8, r = 512 T = 12 44.4 / 40.0, 27648 x 5120 r = 1024 T = 16 86.2 / 59.5.
+// One 64-column block per ring item took half as long again on tall slices (22016 x 4096 70): the issuing warp bound them.
 #pragma once
 #include <cuda.h>
 
@@ -49,7 +48,7 @@ constexpr int LT_A_BYTES = 2 * LT_A_BLOCK;
 constexpr int LT_MAX_STAGES = 12;
 constexpr int LT_MAX_SEG = 3;                      // slices per CTA (accumulators in tensor memory beside that of h)
 constexpr int LT_MAX_BLOCKS = LT_MAX_SEG * 2 * 16;  // 64-rank blocks of a CTA at the highest rank
-constexpr int LT_SMEM_FIXED = 1024 /* alignment */ + 8 * (2 * LT_MAX_STAGES + LT_MAX_BLOCKS + 4) + 32;
+constexpr int LT_SMEM_FIXED = 1024 /* alignment */ + 8 * (2 * LT_MAX_STAGES + LT_MAX_BLOCKS + 3) + 32;
 
 struct LinearParams {
     const uint8_t* uq;             // [M][r/2]
@@ -61,17 +60,16 @@ struct LinearParams {
     __nv_bfloat16* h;              // scratch: bf16 [T][r]
     unsigned int* sync;            // scratch: [0] partial sums of h written, [1] CTAs past their waits, [3] shares of h published
     unsigned int* status;          // an expired wait records 1
-    float* part;                   // workspace: [CTA][T][128] partial sums of h, later of the output
-    unsigned int* slice_count;     // workspace: arrivals per slice (zeroed by the kernel before use)
+    float* part;                   // workspace: [CTA][T][128] partial sums of h
     const __nv_bfloat16* y_dense;  // [T][M]: base term supplied by the caller, nothing of W_b is streamed; or nullptr
     __nv_bfloat16* out;            // [T][M]
     int T, tpad, M, N, r;
-    int slices, segs, ksplit;      // row slices; slices per CTA (ksplit = 1), or CTAs per slice (segs = 1)
+    int slices, segs;              // row slices, and how many of them a CTA takes
     int rows;                      // tallest slice
     int hparts;                    // CTAs per rank group in the computation of h
     int stages;
     int u_start;                   // W items a CTA streams before its first U item (h is there by then)
-    uint32_t ring_bytes;           // the ring's area; reused for the exchange of partial sums once it has drained
+    uint32_t ring_bytes;
     uint32_t idesc;
     uint32_t tmem_cols;
     int n_blocks;                  // block-diagonal U^ as in FactoredParams
@@ -79,13 +77,7 @@ struct LinearParams {
     int block_groups[5];
     long long spin_limit;
     int drop_arrivals;
-    unsigned long long* trace;     // development builds (ADE_TRACE) only
 };
-#ifdef ADE_TRACE
-#define LT_STAMP(i) do { if (p.trace && (threadIdx.x & 31) == 0) p.trace[(blockIdx.x * 10 + (threadIdx.x >> 5)) * 16 + (i)] = clock64(); } while (0)
-#else
-#define LT_STAMP(i) do { } while (0)
-#endif
 
 struct LinearMaps {
     CUtensorMap w;                 // (M, N) bf16, box `rows` rows x 64, 128-byte swizzle
@@ -109,8 +101,6 @@ __device__ __forceinline__ uint32_t bf2_fma(uint32_t a, uint32_t b, uint32_t c) 
     return d;
 }
 __device__ __forceinline__ void unpack_sync() { asm volatile("bar.sync 1, %0;" ::"n"(LT_UNPACK_THREADS) : "memory"); }
-// other CTAs' generic-proxy writes (made visible by an acquire) -> this thread's bulk copies
-__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
 // Grid-wide wait of one thread for a counter (bounded; an expired wait is recorded and the launch carries on to its end).
 __device__ __forceinline__ void lt_wait_count(const unsigned int* c, unsigned int want, const LinearParams& p, volatile int* abort_flag) {
@@ -134,14 +124,13 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
     const uint32_t stage_bytes = LT_A_BYTES + 2 * x_bytes;
     const uint32_t bars = ring + p.ring_bytes;
     const uint32_t bar_full = bars, bar_empty = bars + 8 * S, bar_slot = bars + 16 * S, bar_h = bar_slot + 8 * LT_MAX_BLOCKS, bar_done = bar_h + 8,
-                   bar_pass = bar_h + 16, bar_fix = bar_h + 24;
-    uint8_t* gen = lt_smem + (bar_fix + 8 - raw0);
+                   bar_pass = bar_h + 16;
+    uint8_t* gen = lt_smem + (bar_pass + 8 - raw0);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 4);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
     const int G = gridDim.x, c = blockIdx.x;
-    LT_STAMP(0);
     const int T = p.T, N = p.N, M = p.M, r = p.r, ng = r >> 7;
     const int kbs = N / LT_ITEM;                                 // items along the columns
     // A items: CTA c computes part c % hparts of rank group c / hparts
@@ -179,7 +168,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
         mbar_init(bar_h, 1);
         mbar_init(bar_done, 1);
         mbar_init(bar_pass, 1);
-        mbar_init(bar_fix, 1);
         *abort_flag = 0;
         fence_mbar_init();
         prefetch_tensormap(&maps.w);
@@ -193,16 +181,13 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    LT_STAMP(1);
     const WaitCtx wctx{abort_flag, reinterpret_cast<int*>(p.status), p.spin_limit};
 
-    // W items: slices [slice0, slice0 + nseg), columns [k0, k1) in blocks
-    const int kpart = p.ksplit > 1 ? c % p.ksplit : 0;
-    const int slice0 = p.ksplit > 1 ? c / p.ksplit : c * p.segs;
+    // W items: slices [slice0, slice0 + nseg)
+    const int slice0 = c * p.segs;
     const int nseg = max(0, min(p.segs, p.slices - slice0));
-    const int k0 = kpart * kbs / p.ksplit, k1 = (kpart + 1) * kbs / p.ksplit;
     auto slice_row = [&](int s) { return static_cast<int>(static_cast<long long>(s) * M / p.slices); };
-    // U items of segment s: this CTA's share of the 64-rank blocks the slice's rows can touch
+    // U items of segment s: the 64-rank blocks the slice's rows can touch
     auto u_range = [&](int s, int& u0, int& u1) {
         int lo = 0, hi = ng;
         if (p.n_blocks > 0) {
@@ -218,14 +203,13 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                 hi = h;
             }
         }
-        const int nu = 2 * (hi - lo);
-        u0 = 2 * lo + kpart * nu / p.ksplit;
-        u1 = 2 * lo + (kpart + 1) * nu / p.ksplit;
+        u0 = 2 * lo;
+        u1 = 2 * hi;
     };
     // The U items (one per 64-rank block) are spread evenly over the part of the W items that comes after u_start, so that their
     // preparation runs under the stream; a block of segment s comes after the segment's first W item, which starts the
     // accumulator.  Every role walks the same order: `u_before(j)` W items come before U block j.
-    const int wtotal = p.y_dense ? 0 : nseg * (k1 - k0);
+    const int wtotal = p.y_dense ? 0 : nseg * kbs;
     int ucum[LT_MAX_SEG + 1] = {0, 0, 0, 0}, ufirst[LT_MAX_SEG] = {0, 0, 0};
 #pragma unroll
     for (int s = 0; s < LT_MAX_SEG; ++s) {
@@ -238,7 +222,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
     const int u_start = min(p.u_start, wtotal);
     auto u_seg = [&](int j) { return (j >= ucum[1]) + (j >= ucum[2]); };
     auto u_block = [&](int j) { return j < ucum[1] ? ufirst[0] + j : (j < ucum[2] ? ufirst[1] + j - ucum[1] : ufirst[2] + j - ucum[2]); };
-    auto u_before = [&](int j) { return min(max(u_start + (j + 1) * (wtotal - u_start) / ucount, u_seg(j) * (k1 - k0) + 1), wtotal); };
+    auto u_before = [&](int j) { return min(max(u_start + (j + 1) * (wtotal - u_start) / ucount, u_seg(j) * kbs + 1), wtotal); };
 
     if (warp == LT_LOAD_WARP) {
         // ------------------------------------------------------------------ TMA producer
@@ -261,7 +245,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                 load_x(kb, bar_full + 8 * st);
             }
             const uint32_t w_bytes = static_cast<uint32_t>(p.rows) * 128u;
-            int s = 0, kb = k0, m0 = slice_row(slice0), i = 0;
+            int s = 0, kb = 0, m0 = slice_row(slice0), i = 0;
             for (int j = 0; j <= ucount; ++j) {
                 const int stop = j < ucount ? u_before(j) : wtotal;
                 for (; i < stop; ++i, next()) {
@@ -272,8 +256,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                     tma_load_2d(sa, &maps.w, kb * LT_ITEM, m0, full);
                     tma_load_2d(sa + LT_A_BLOCK, &maps.w, kb * LT_ITEM + LT_KB, m0, full);
                     load_x(kb, full);
-                    if (++kb == k1) {
-                        kb = k0;
+                    if (++kb == kbs) {
+                        kb = 0;
                         m0 = slice_row(slice0 + ++s);
                     }
                 }
@@ -325,23 +309,21 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
             }
             __syncwarp();
         }
-        LT_STAMP(2);
         {
             uint32_t d = tmem_base + p.tpad;
-            int kb = k0, i = 0;
+            int kb = 0, i = 0;
             for (int j = 0; j <= ucount; ++j) {
                 const int stop = j < ucount ? u_before(j) : wtotal;
                 for (; i < stop; ++i, next()) {
                     wait_bounded(bar_full + 8 * st, ph, wctx, 1);
                     tc_fence_after();
-                    if (elect_one()) item(d, x_bytes, kb == k0);
+                    if (elect_one()) item(d, x_bytes, kb == 0);
                     __syncwarp();
-                    if (++kb == k1) {
-                        kb = k0;
+                    if (++kb == kbs) {
+                        kb = 0;
                         d += p.tpad;
                     }
                 }
-                if (i == wtotal && j == 0) LT_STAMP(3);
                 if (j < ucount) {
                     wait_bounded(bar_full + 8 * st, ph, wctx, 1);
                     tc_fence_after();
@@ -352,15 +334,10 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                 }
             }
         }
-        LT_STAMP(4);
         if (elect_one()) tc_commit(bar_done);
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ unpack, h exchange, epilogue
-        // counters of the slices, used after the second hand-over only
-        if (p.ksplit > 1)
-            for (int t = c * LT_UNPACK_THREADS + tid; t < p.slices; t += G * LT_UNPACK_THREADS) p.slice_count[t] = 0u;
-
         {
             int st = 0;
             uint32_t ph = 1;
@@ -391,7 +368,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                 }
             }
         }
-        LT_STAMP(2);
 
         // ---- partial sums of h: tensor memory -> scratch, [part][token][rank]
         const int q = warp & 3, hcol = warp >> 2;                // tensor-memory lane quarter, column half
@@ -409,7 +385,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                     if (c0 + i < T) __stcg(part + static_cast<size_t>(c0 + i) * 128, __uint_as_float(v[i]));
             }
         }
-        LT_STAMP(3);
 
         // Operands of the U blocks, one block ahead of their use: 32 codes of one row per thread, and 16-byte pieces of h.
         struct UOp {
@@ -436,7 +411,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
         if (!by_warp && ucount > 0) fetch_u(u, 0);                           // after the release: the fence in it would wait for these loads too
         if (tid == 0) lt_wait_count(p.sync, static_cast<unsigned int>(ng * p.hparts), p, abort_flag);
         unpack_sync();
-        LT_STAMP(4);
         // ---- this CTA's share of h: four lanes per four ranks, each adds every fourth part, fixed order
         {
             const int quads = (T * r) >> 2;
@@ -477,7 +451,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                 }
             }
         }
-        LT_STAMP(5);
         unpack_sync();
         if (tid == 0) {
             red_release_gpu_add(p.sync + 3, 1u);
@@ -485,7 +458,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
             mbar_arrive(bar_pass);                               // the load warp checks out for this CTA
         }
         unpack_sync();
-        LT_STAMP(6);
 
         // ---- U items.  The load warp, which follows the ring item by item, says when a block's stage is free (one barrier per block: a
         // wait of this role's own on bar_empty could take an older phase of the same parity for the right one).
@@ -550,7 +522,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
             // All eight warps on each block, operands one block ahead.
             uint4 hc[4], hn[4];
             if (ucount > 0) fetch_h(hc, 0);
-            LT_STAMP(7);
             for (int j = 0; j < ucount; ++j) {
                 if (j + 1 < ucount) {
                     fetch_u(un, j + 1);
@@ -590,96 +561,40 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
                 for (int i = 0; i < 4; ++i) hc[i] = hn[i];
             }
         }
-        LT_STAMP(8);
 
         // ---- epilogue
-        if (p.ksplit == 1) {
-            for (int s = 0; s < nseg; ++s) {
-                const int m = slice_row(slice0 + s) + rr;
-                const bool live = m < slice_row(slice0 + s + 1);
-                uint32_t y[4][16];                               // base term, requested before the last products are waited for
-                if (p.y_dense) {
+        for (int s = 0; s < nseg; ++s) {
+            const int m = slice_row(slice0 + s) + rr;
+            const bool live = m < slice_row(slice0 + s + 1);
+            uint32_t y[4][16];                               // base term, requested before the last products are waited for
+            if (p.y_dense) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const int t = hcol * 16 + 32 * k + i;
-                            y[k][i] = live && t < T ? static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(p.y_dense) + static_cast<size_t>(t) * M + m)) : 0u;
-                        }
-                }
-                if (s == 0) {
-                    wait_bounded(bar_done, 0, wctx, 1);
-                    tc_fence_after();
-                    LT_STAMP(9);
-                }
-                if (q * 32 >= p.rows) continue;                  // uniform in the warp
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int c0 = hcol * 16 + 32 * k;
-                    if (c0 >= p.tpad) break;
-                    uint32_t v[16];
-                    tmem_ld16_sync(lane_addr + static_cast<uint32_t>(p.tpad) * (1 + s) + c0, v);
+                for (int k = 0; k < 4; ++k)
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        float o = __uint_as_float(v[i]);
-                        if (p.y_dense) o += __uint_as_float(y[k][i] << 16);
-                        if (live && c0 + i < T) p.out[static_cast<size_t>(c0 + i) * M + m] = __float2bfloat16_rn(o);
+                        const int t = hcol * 16 + 32 * k + i;
+                        y[k][i] = live && t < T ? static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(p.y_dense) + static_cast<size_t>(t) * M + m)) : 0u;
                     }
-                }
             }
-        } else if (nseg > 0) {
-            // ksplit CTAs hold partial sums of the slice: each finishes an equal share of the tokens, [t0, t1)
-            wait_bounded(bar_done, 0, wctx, 1);
-            tc_fence_after();
-            LT_STAMP(9);
-            const int n = p.ksplit, t0 = kpart * T / n, t1 = (kpart + 1) * T / n;
-            const uint32_t piece = static_cast<uint32_t>(t1 - t0) * 512u, acc = lane_addr + p.tpad;
-            for (int c0 = hcol * 16; c0 < p.tpad; c0 += 32) {
+            if (s == 0) {
+                wait_bounded(bar_done, 0, wctx, 1);
+                tc_fence_after();
+            }
+            if (q * 32 >= p.rows) continue;                  // uniform in the warp
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int c0 = hcol * 16 + 32 * k;
+                if (c0 >= p.tpad) break;
                 uint32_t v[16];
-                tmem_ld16_sync(acc + c0, v);
+                tmem_ld16_sync(lane_addr + static_cast<uint32_t>(p.tpad) * (1 + s) + c0, v);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const int t = c0 + i;
-                    if (t < T) {
-                        if (t < t0 || t >= t1) __stcg(part + static_cast<size_t>(t) * 128, __uint_as_float(v[i]));
-                        else sts4(ring + kpart * piece + (t - t0) * 512 + rr * 4, v[i]);
-                    }
-                }
-            }
-            fence_proxy_async_all();
-            unpack_sync();
-            LT_STAMP(10);
-            if (tid == 0) {
-                red_release_gpu_add(p.slice_count + slice0, 1u);
-                if (piece > 0) {
-                    // the others' sums of this CTA's tokens are one contiguous piece each: all in flight together
-                    lt_wait_count(p.slice_count + slice0, static_cast<unsigned int>(n), p, abort_flag);
-                    fence_proxy_async_all();
-                    mbar_arrive_expect_tx(bar_fix, piece * static_cast<uint32_t>(n - 1));
-                    for (int j = 0; j < n; ++j)
-                        if (j != kpart) bulk_g2s(ring + j * piece, p.part + (static_cast<size_t>(c - kpart + j) * T + t0) * 128, piece, bar_fix);
-                }
-            }
-            __syncwarp();
-            LT_STAMP(11);
-            if (piece > 0) {
-                wait_bounded(bar_fix, 0, wctx, 1);
-                // a warp per token, consecutive rows per lane: contributors added in their order, one rounding
-                const int m0 = slice_row(slice0), rows = slice_row(slice0 + 1) - m0;
-                for (int t = t0 + warp; t < t1; t += LT_UNPACK_WARPS) {
-                    const uint32_t src = ring + static_cast<uint32_t>(t - t0) * 512u + lane * 4;
-                    float v[4] = {0.f, 0.f, 0.f, 0.f};
-                    for (int j = 0; j < n; ++j) {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) v[k] += __uint_as_float(lds4(src + j * piece + k * 128));
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (lane + 32 * k < rows) p.out[static_cast<size_t>(t) * M + m0 + lane + 32 * k] = __float2bfloat16_rn(v[k]);
+                    float o = __uint_as_float(v[i]);
+                    if (p.y_dense) o += __uint_as_float(y[k][i] << 16);
+                    if (live && c0 + i < T) p.out[static_cast<size_t>(c0 + i) * M + m] = __float2bfloat16_rn(o);
                 }
             }
         }
-        LT_STAMP(12);
     }
 
     drain_after_abort(abort_flag);
@@ -688,43 +603,18 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_tc_kernel(const LinearPa
     if (warp == LT_MMA_WARP) tmem_dealloc(tmem_base, p.tmem_cols);
 }
 
-// How a launch is cut: see the note at the top.
+// How a launch is cut: equal row slices, `segs` of them per CTA.
 struct LinearSplit {
-    int slices, segs, ksplit, rows, stages, u_start;
+    int slices, segs, rows, stages, u_start;
     uint32_t ring_bytes;
 };
 constexpr int kLtRingMax = 232448 - LT_SMEM_FIXED;
 
-// Cost in microseconds of `ksplit` CTAs per slice, as far as the choice depends on it: the bytes an SM takes in (its weights
-// once, x for its columns; 83 GB/s per SM measured with all SMs streaming), the MMAs (a 64-column block takes about 0.17 us
-// whatever the height of the slice: the tensor core reads 128 rows) and the exchange of partial sums.
-inline double linear_split_cost(int M, int N, int T, int grid, int ksplit) {
-    const int slices = grid / ksplit;
-    const double rows = (M + slices - 1) / slices;
-    const double ingest = (rows + T) * 2.0 * N / ksplit / 83e3;
-    const double mma = 0.17 * N / LT_KB / ksplit;
-    return (ingest > mma ? ingest : mma) + (ksplit > 1 ? 3.0 + 2.0 * T * rows * 4.0 / 83e3 : 0.0);
-}
-// `stream`: W_b is streamed; without it there is nothing to split over the columns.
-inline bool linear_split(int M, int N, int T, int tpad, int grid, bool stream, LinearSplit& out) {
-    const int kbs = N / LT_ITEM;
+inline bool linear_split(int M, int T, int tpad, int grid, LinearSplit& out) {
     LinearSplit s = {};
-    s.ksplit = 1;
     s.segs = (M + LT_TILE * grid - 1) / (LT_TILE * grid);
     if (s.segs > LT_MAX_SEG) return false;
-    if (s.segs == 1 && stream) {
-        double best = linear_split_cost(M, N, T, grid, 1);
-        for (int k = 2; k <= kbs && k <= grid; ++k) {
-            const int slices = grid / k;
-            if ((M + slices - 1) / slices > LT_TILE) break;
-            const double cost = linear_split_cost(M, N, T, grid, k);
-            if (cost < best) {
-                best = cost;
-                s.ksplit = k;
-            }
-        }
-    }
-    s.slices = grid / s.ksplit * s.segs;
+    s.slices = grid * s.segs;
     if (s.slices > M) s.slices = M;
     s.rows = (M + s.slices - 1) / s.slices;
     const int stage = LT_A_BYTES + 2 * tpad * 128;
@@ -734,17 +624,13 @@ inline bool linear_split(int M, int N, int T, int tpad, int grid, bool stream, L
     // (its share of 6.4 TB/s, or 0.34 us each).  U items that come up earlier would hold the stream up.
     const double item = s.rows * 256.0 * grid / 6.4e6 > 0.34 ? s.rows * 256.0 * grid / 6.4e6 : 0.34;
     s.u_start = static_cast<int>((10.0 + 0.04 * T) / item) + 1;
-    int ring = s.stages * stage;
-    const int fix = s.ksplit > 1 ? 512 * (T + s.ksplit) : 0;      // n pieces of ceil(T / n) token rows at most
-    if (ring < fix) ring = (fix + 1023) & ~1023;
-    s.ring_bytes = static_cast<uint32_t>(ring);
-    if (s.stages < 2 || ring > kLtRingMax) return false;
+    s.ring_bytes = static_cast<uint32_t>(s.stages * stage);
+    if (s.stages < 2) return false;
     out = s;
     return true;
 }
 
-// Workspace: partial sums (of h, then of the output) and the slice counters behind them.
-inline size_t linear_part_bytes(int T, int grid) { return static_cast<size_t>(grid) * T * 128 * sizeof(float); }
-inline size_t linear_workspace_bytes(int T, int grid) { return linear_part_bytes(T, grid) + static_cast<size_t>(grid) * sizeof(unsigned int); }
+// Workspace: partial sums of h.
+inline size_t linear_workspace_bytes(int T, int grid) { return static_cast<size_t>(grid) * T * 128 * sizeof(float); }
 
 }  // namespace ade

@@ -272,18 +272,9 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
         bool tf_ready = false;                            // per-group barriers: the coming group's accumulator was seen complete
         int j = 0, sm = strip0, nt = nt0;
         uint32_t sct_u = scf;                             // us table of the current strip
-#ifdef ADE_TRACE
-        int tcn = 0;
-        const int ttrack = warp == 0 ? 0 : 1;
-        const bool tr = (warp == 0 || warp == 9) && lane == 0;
-#define EPI_STAMP(code) do { if (tr) ADE_TRACE_STAMP(p, tcn, ttrack, code); } while (0)
-#else
-#define EPI_STAMP(code) do { } while (0)
-#endif
         for (int tile = t_begin; tile < t_end; ++tile, ++j) {
             const int m0 = sm << 7, n0 = nt << 7;
             const int m = m0 + row;
-            EPI_STAMP(0x0100 | (j & 255));
             const bool live = m < p.M;
             const uint32_t b = j & 1, jph = (j >> 1) & 1;
             const uint32_t wbb = C::WB_BUFS == 2 ? b : 0, wph = C::WB_BUFS == 2 ? jph : static_cast<uint32_t>(j & 1);
@@ -310,7 +301,6 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                 if (!ok_wb) wait_bounded(wbar, wph, wctx, 6);
             }
             if (C::PER_TILE) tc_fence_after();
-            EPI_STAMP(0x0200 | (j & 255));
             const uint32_t sct = F8 ? scf + (2 + b) * (ng * 512) : scf + b * (ng * RS_SC_BYTES);     // the tile's vs, or both its tables
 
             uint64_t acc[16];
@@ -329,7 +319,6 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                     if (!tf_ready) wait_bounded(bar(C::BAR_TFULL + a), aph, wctx, 3);
                     tc_fence_after();
                 }
-                EPI_STAMP(0x0300 | g);
                 const float u = __uint_as_float(lds4((F8 ? sct_u + g * 512 : sct + g * RS_SC_BYTES) + row * 4));
                 const uint64_t uu = f2_pack(u, u);
                 const float um = __fmul_rn(u, -12582912.0f);            // -m us, exact (m = 1.5 * 2^23)
@@ -397,19 +386,16 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                         tf_ready = mbar_test(bar(C::BAR_TFULL + a1), ph1);
                     }
                     tmem_ld16_sync(tbase + ch * 16, vc);
-                    EPI_STAMP(0x0400 | (g << 1) | ch);
                     tmem_st16_fill(tbase + ch * 16, magic4);    // re-arm, completes under the arithmetic
                     rescale16(vc, ch);
                 }
                 }
-                EPI_STAMP(0x0500 | g);
                 if (!F8) {
                     tmem_st_wait();                      // accumulator stage re-armed: hand it back
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar(C::BAR_TEMPTY + a));
                 }
-                EPI_STAMP(0x0600 | g);
                 if (C::WB_BUFS == 2 && g == 0 && lane == 0 && tile + 1 < t_end) {
                     // base box of the next tile into the other buffer; the store that last read it was issued a tile ago
                     const bool wrap = nt + 1 == tiles_n;
@@ -422,9 +408,7 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(C::BAR_SC_EMPTY + b));             // this warp is done with the scale tables
-            EPI_STAMP(0x0700 | (j & 255));
             if (C::WB_BUFS == 1) wait_bounded(wbar, wph, wctx, 6);
-            EPI_STAMP(0x0800 | (j & 255));
             uint4 wv4[4];                                // 8 columns per 16-byte chunk
 #pragma unroll
             for (int c = 0; c < 4; ++c) wv4[c] = lds16(box + own + ((c ^ swz) << 4));
@@ -448,7 +432,6 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                 tma_store_2d(&maps.out, n0 + hh * 32, m0 + q * 32, box);
                 bulk_commit_group();
             }
-            EPI_STAMP(0x0900 | (j & 255));
             if (++nt == tiles_n) {
                 nt = 0;
                 ++sm;
@@ -462,12 +445,6 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
         const int c = pt & 3, rbase = pt >> 2;
         uint32_t ri = 0, bi = 0, sk = 0;
         int cur_strip = -1;
-#ifdef ADE_TRACE
-        int tcn = 0;
-#define UNP_STAMP(code) do { if (pt == 0) ADE_TRACE_STAMP(p, tcn, 2, code); } while (0)
-#else
-#define UNP_STAMP(code) do { } while (0)
-#endif
         uint64_t za_pack[4] = {0, 0, 0, 0};               // zero-points of this thread's four U rows, one byte per group
         int sm = strip0, nt = nt0;
         for (int tile = t_begin; tile < t_end; ++tile) {
@@ -508,9 +485,7 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
             }
             for (int g = 0; g < ng; ++g, ++ri, ++bi) {
                 const uint32_t slot = ri % C::RAW_DEPTH, ph = (ri / C::RAW_DEPTH) & 1;
-                UNP_STAMP(0x1000 | g);
                 wait_bounded(bar(C::BAR_RAW_FULL + slot), ph, wctx, 8);
-                UNP_STAMP(0x1100 | g);
                 const uint32_t rs = rawr + slot * RS_RAW_SLOT;
                 uint4 qb[4];
                 uint32_t zb[4];
@@ -523,13 +498,11 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                 if (lane == 0) mbar_arrive(bar(C::BAR_RAW_EMPTY + slot));
                 const uint32_t s = bi % C::B_STAGES, bph = (bi / C::B_STAGES) & 1;
                 wait_bounded(bar(C::BAR_B_EMPTY + s), bph ^ 1, wctx, 2);
-                UNP_STAMP(0x1200 | g);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) unpack_store_s(b_st + s * RS_OPER_BYTES, rbase + 32 * i, c, qb[i], zb[i]);
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(C::BAR_B_FULL + s));
-                UNP_STAMP(0x1300 | g);
             }
         }
     } else {
@@ -542,12 +515,6 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
         // (two issuing threads taking alternate groups were tried with the expanded operands: no faster)
         if (EXP || lane == 0) {
             uint32_t it = 0, k = 0, s = 0, bph = 0;
-#ifdef ADE_TRACE
-            int tcn = 0;
-#define MMA_STAMP(code) do { if (lane == 0) ADE_TRACE_STAMP(p, tcn, 3, code); } while (0)
-#else
-#define MMA_STAMP(code) do { } while (0)
-#endif
             int nt = nt0;
             uint32_t jt = 0;
             for (int tile = t_begin; tile < t_end; ++tile, ++jt) {
@@ -556,14 +523,11 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                 if (++nt == tiles_n) nt = 0;
                 for (int g = 0; g < ng; ++g, ++it) {
                     const uint32_t a = it % RS_ACC_STAGES, aph = (it / RS_ACC_STAGES) & 1;
-                    MMA_STAMP(0x2000 | g);
                     {
                         const bool ok_e = mbar_test(bar(C::BAR_TEMPTY + a), aph), ok_b = mbar_test(bar(C::BAR_B_FULL + s), bph);
                         if (!ok_e) wait_bounded(bar(C::BAR_TEMPTY + a), aph, wctx, 4);
-                        MMA_STAMP(0x2100 | g);
                         if (!ok_b) wait_bounded(bar(C::BAR_B_FULL + s), bph, wctx, 1);
                     }
-                    MMA_STAMP(0x2200 | g);
                     if (first) wait_bounded(bar(C::BAR_A_FULL + g), k & 1, wctx, 9);
                     tc_fence_after();
                     const uint64_t ad = smem_desc_k_sw128(a_res + g * RS_OPER_BYTES);
@@ -580,7 +544,6 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                         if (last && g == ng - 1) tc_commit(bar(C::BAR_A_FREE));    // the strip of U may be overwritten
                     }
                     if (EXP) __syncwarp();
-                    MMA_STAMP(0x2300 | g);
                     if (++s == C::B_STAGES) {
                         s = 0;
                         bph ^= 1;
@@ -629,9 +592,6 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
             prefetch_tensormap(&maps.vq);
             uint32_t ri = 0;
             int cur_strip = -1;
-#ifdef ADE_TRACE
-            int tcn = 0;
-#endif
             int sm = strip0, nt = nt0;
             for (int tile = t_begin; tile < t_end; ++tile) {
                 const int strip = sm, n0 = nt << 7;
@@ -651,7 +611,6 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                 for (int g = 0; g < ng; ++g, ++ri) {
                     const uint32_t slot = ri % C::RAW_DEPTH, ph = (ri / C::RAW_DEPTH) & 1;
                     wait_bounded(bar(C::BAR_RAW_EMPTY + slot), ph ^ 1, wctx, 10);
-                    ADE_TRACE_STAMP(p, tcn, 4, 0x3000 | g);
                     mbar_arrive_expect_tx(bar(C::BAR_RAW_FULL + slot), RS_RAW_CODES + 128);
                     tma_load_2d(rawr + slot * RS_RAW_SLOT, &maps.vq, g * 64, n0, bar(C::BAR_RAW_FULL + slot));
                     bulk_g2s(rawr + slot * RS_RAW_SLOT + RS_RAW_CODES, p.vz + static_cast<size_t>(g) * p.N + n0, 128,

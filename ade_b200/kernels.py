@@ -295,8 +295,8 @@ def factored_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor | None = No
 def linear_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor) -> torch.Tensor:
     """out = x W_b^T + U^(V^T x) for T <= 128 tokens with every contraction on the tensor cores in one launch of ``ade_b200_linear``.
     Modules use it for tall groups at 9-16 tokens only: above 16 their result is defined by the reference's split, whose base
-    term is rounded to bfloat16 by the library GEMM.  This one keeps the base term in float32 and is faster (4096 x 4096 r = 512
-    T = 40 19.9 us against 27.3 for the split, 4096 x 11008 T = 100 29.8 / 50.6)."""
+    term is rounded to bfloat16 by the library GEMM.  This one keeps the base term in float32 (us per call, split / this: 11008 x 4096
+    r = 512 T = 128 48.6 / 36.7, 13824 x 5120 r = 640 T = 64 53.6 / 35.9, 4096 x 4096 r = 512 T = 100 36.0 / 31.1, 4096 x 11008 51.3 / 53.7)."""
     return _launch(_lib.ops().linear, x, p4, weight, None)
 
 

@@ -17,8 +17,8 @@ def _case(M, N, r, T):
     return tp, W, x
 
 
-# one row, one slice per SM and fewer rows than SMs; ragged token counts around the multiples of 16; ksplit > 1 with ragged slices
-# (4096 x 2048 at 100 tokens, 1000 x 4096); the highest rank; two and three slices per SM (19000 and 38000 rows); the widest token range
+# one row, one slice per SM and fewer rows than SMs; ragged token counts around the multiples of 16; ragged slices; the highest rank;
+# two and three slices per SM (19000 and 38000 rows); the widest token range
 @pytest.mark.parametrize("M,N,r,T", [(1, 128, 128, 1), (100, 256, 512, 17), (129, 128, 256, 128), (500, 1024, 128, 33), (1000, 4096, 384, 20),
                                      (4096, 2048, 640, 100), (301, 4096, 1024, 64), (256, 384, 2048, 47), (19000, 128, 256, 40),
                                      (38000, 128, 128, 128), (2050, 1152, 896, 16)])
