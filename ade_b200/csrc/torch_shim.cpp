@@ -111,8 +111,9 @@ at::Tensor factored(const at::Tensor& x, const c10::optional<at::Tensor>& weight
 }
 
 // A merge without kept operands expands the codes into a work buffer first and takes the float8 kernel: two launches, but the kernel
-// that unpacks codes inside is slower by more than the expansion from rank 384 up (4096 x 4096 r = 256 22.5 / 22.2 us;
-// 11008 x 4096 r = 512 72 / 50 us; 13824 x 5120 r = 1024 189 / 126 us; unpacking inside / both launches).
+// that unpacks codes inside is slower by more than the expansion from rank 384 up, on every shape measured (M 500-13824, N 1024-11008).
+// Unpacking inside / both launches in us: r = 256 4096 x 4096 22.2 / 19.3, 8192 x 4096 38.0 / 36.8, 500 x 11008 12.9 / 13.2; r = 384 27.0 / 21.9,
+// 45.5 / 38.3, 15.1 / 14.6; r = 512 11008 x 4096 72 / 50; r = 1024 13824 x 5120 189 / 126.  At rank 256 the gain is not worth the buffer.
 constexpr int kExpandFirst = 384;
 
 at::Tensor recon(const at::Tensor& base, const at::Tensor& uq, const at::Tensor& vq, const at::Tensor& vt, const at::Tensor& us,
