@@ -148,7 +148,7 @@ def _attn_decode_ok(mod, x, cos, mask, layer) -> bool:
     hd = kc.shape[3]
     if hd % 32 or hd > 256 or (7 * hd + kc.shape[2]) * 4 > 48 * 1024 or layer.cumulative_length.dtype != torch.int64:
         return False
-    if not (cos.dtype == torch.bfloat16 and cos.dim() == 3 and cos.shape[1] == 1 and cos.is_contiguous() and cos.shape[0] in (1, x.shape[0])):
+    if not (cos.dtype == torch.bfloat16 and cos.dim() == 3 and cos.shape[1:] == (1, hd) and cos.is_contiguous() and cos.shape[0] in (1, x.shape[0])):
         return False
     if mask is not None and not (mask.dtype == torch.bool and mask.dim() == 4 and mask.shape[1] == 1 and mask.shape[2] == 1
                                  and mask.shape[3] == kc.shape[2] and mask.stride(3) == 1 and mask.shape[0] == x.shape[0]):
@@ -162,11 +162,23 @@ def _rope_layout_ok(x: torch.Tensor) -> bool:
     return x.stride(3) == 1 and (h == 1 or x.stride(1) == hd) and (B == 1 or T == 1 or x.stride(0) == T * x.stride(2))
 
 
+def _rope_ok(q: torch.Tensor, k: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> bool:
+    """The launch reads a full table row for every (batch, token): what torch would broadcast is left to it."""
+    return (q.dim() == 4 and k.dim() == 4 and _rows_ok(q, q.shape[0] * q.shape[2], k, cos, sin) and k.dtype == torch.bfloat16
+            and k.shape[0] == q.shape[0] and k.shape[2:] == q.shape[2:] and q.shape[3] % 2 == 0
+            and cos.dtype == sin.dtype == torch.bfloat16 and cos.dim() == 3 and cos.shape == sin.shape and cos.shape[1:] == q.shape[2:]
+            and cos.is_contiguous() and sin.is_contiguous() and cos.shape[0] in (1, q.shape[0]) and _rope_layout_ok(q) and _rope_layout_ok(k))
+
+
+def _norm_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    return weight.dtype == torch.bfloat16 and weight.shape == x.shape[-1:] and weight.is_contiguous() and x.stride(-1) == 1
+
+
 def _add_norm_ok(x: torch.Tensor, residual: torch.Tensor, norm) -> bool:
     """`residual + x` and the LlamaRMSNorm `norm` behind it can be one launch.  Asked about the very tensors that go into it: a
     module in front may have made one of them require a gradient although the layer's input does not."""
-    return (_rows_ok(x, x.numel() // x.shape[-1], residual, norm.weight) and residual.dtype == torch.bfloat16 and norm.weight.dtype == torch.bfloat16
-            and x.shape == residual.shape and x.stride(-1) == 1 and residual.stride(-1) == 1)
+    return (_rows_ok(x, x.numel() // x.shape[-1], residual, norm.weight) and residual.dtype == torch.bfloat16 and x.shape == residual.shape
+            and _norm_ok(x, norm.weight) and residual.stride(-1) == 1)
 
 
 def enable_fused_decode_ops(model) -> int:
@@ -180,9 +192,7 @@ def enable_fused_decode_ops(model) -> int:
         original = ml.apply_rotary_pos_emb
 
         def apply_rotary_pos_emb(q, k, cos, sin, unsqueeze_dim=1):
-            if (unsqueeze_dim == 1 and q.dim() == 4 and _rows_ok(q, q.shape[0] * q.shape[2], k, cos, sin) and k.dtype == torch.bfloat16
-                    and cos.dtype == torch.bfloat16 and cos.dim() == 3 and cos.is_contiguous() and sin.is_contiguous()
-                    and cos.shape[0] in (1, q.shape[0]) and _rope_layout_ok(q) and _rope_layout_ok(k)):
+            if unsqueeze_dim == 1 and _rope_ok(q, k, cos, sin):
                 return rope(q, k, cos, sin)
             return original(q, k, cos, sin, unsqueeze_dim)
 
@@ -199,9 +209,12 @@ def enable_fused_decode_ops(model) -> int:
                 if (position_embeddings is not None and layer is not None
                         and _attn_decode_ok(mod, hidden_states, position_embeddings[0], attention_mask, layer)):
                     q, k, v = mod.q_proj(hidden_states), mod.k_proj(hidden_states), mod.v_proj(hidden_states)
+                    kc, cos, sin = layer.keys, *position_embeddings
                     if (all(t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.device == hidden_states.device for t in (q, k, v))
-                            and position_embeddings[1].is_contiguous() and position_embeddings[1].device == hidden_states.device):
-                        ctx = attn_decode(q, k, v, position_embeddings[0], position_embeddings[1], attention_mask, layer, mod.scaling)
+                            and q.shape[-1] % kc.shape[3] == 0 and k.shape[-1] == v.shape[-1] == kc.shape[1] * kc.shape[3]
+                            and layer.values.shape == kc.shape and sin.shape == cos.shape and sin.dtype == cos.dtype and sin.is_contiguous()
+                            and sin.device == hidden_states.device):
+                        ctx = attn_decode(q, k, v, cos, sin, attention_mask, layer, mod.scaling)
                         return mod.o_proj(ctx), None
                 return mod._ade_orig_forward(hidden_states, position_embeddings=position_embeddings, attention_mask=attention_mask,
                                              past_key_values=past_key_values, **kw)
@@ -219,7 +232,7 @@ def enable_fused_decode_ops(model) -> int:
                     mod._ade_pre = None
                     if x is pre[0] and x._version == pre[1]:
                         return pre[2]
-                if _rows_ok(x, x.numel() // x.shape[-1], mod.weight) and x.stride(-1) == 1 and mod.weight.dtype == torch.bfloat16:
+                if _rows_ok(x, x.numel() // x.shape[-1], mod.weight) and _norm_ok(x, mod.weight):
                     return rmsnorm(x, mod.weight, mod.variance_epsilon)
                 return mod._ade_orig_forward(x)
 

@@ -207,3 +207,29 @@ def test_dispatch_modes_and_tensor_subclasses_see_the_operations(monkeypatch):
     with Mode():
         assert not decode_ops._rows_ok(x, rows, x)
     assert decode_ops._rows_ok(x, rows, x)
+
+
+def test_operands_a_launch_would_read_past_are_left_to_torch(monkeypatch):
+    """Tables and weights that torch broadcasts or refuses: a launch would read a full row of them through a pointer."""
+    launches = []
+    monkeypatch.setattr(decode_ops, "_on_cuda", lambda t: True)
+    for name in STAND_INS:
+        monkeypatch.setattr(decode_ops, name, lambda *a, name=name: launches.append(name) or STAND_INS[name](*a))
+    patched, _ = _models("cpu")
+    from transformers.models.llama import modeling_llama as ml
+
+    B, T, hd = 2, 300, 64
+    q = torch.randn(B, T, 4, hd).to(torch.bfloat16).transpose(1, 2)
+    cos, sin = torch.randn(1, T, hd).to(torch.bfloat16), torch.randn(1, T, hd).to(torch.bfloat16)
+    ml.apply_rotary_pos_emb(q, q, cos, sin)
+    assert launches == ["rope"]
+    for c, s in ((cos[:, :1], sin[:, :1]), (cos, sin[:, :1]), (cos[..., :1], sin[..., :1]), (cos, sin.float())):
+        out = ml.apply_rotary_pos_emb(q, q, c.contiguous(), s.contiguous())
+        assert out[0].shape == q.shape and launches == ["rope"]
+    norm, x = patched.model.norm, torch.randn(B, T, 256).to(torch.bfloat16)
+    launches.clear()
+    norm(x)
+    assert launches == ["rmsnorm"] and decode_ops._add_norm_ok(x, x, norm)
+    for w in (torch.ones(1), torch.ones(1).expand(256)):
+        norm.weight = torch.nn.Parameter(w.to(torch.bfloat16) if w.is_contiguous() else torch.ones(1, dtype=torch.bfloat16).expand(256), requires_grad=False)
+        assert norm(x).shape == x.shape and launches == ["rmsnorm"] and not decode_ops._add_norm_ok(x, x, norm)
