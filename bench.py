@@ -76,9 +76,9 @@ def factored_bytes(M, N, r, T, fused):
 
 WORK_OPS = sum(delta_ops(M, N, RANK) for _, M, N in MODULES)
 # dram__bytes_read.sum + dram__bytes_write.sum of one reconstruction launch on gate_proj, taken from an ncu capture
-# of `--case recon` with expanded operands (not measured in this run; 101.3 MB read + 53.4 MB written); part of W' is
+# of `--case recon` with e4m3 operands (not measured in this run; 100.8 MB read + 51.4 MB written); part of W' is
 # still in L2 when the kernel ends
-RECON_TRAFFIC_BYTES = 154.7e6
+RECON_TRAFFIC_BYTES = 152.2e6
 
 
 def measured_peaks():
