@@ -181,8 +181,9 @@ class FusedADEGroup:
         self.offsets = [sum(Ms[:i]) for i in range(len(Ms) + 1)]
         # base weights: one buffer, the members keep views of it
         W = torch.cat([m.weight for m in self.members], dim=0)
-        for m, lo, hi in zip(self.members, self.offsets[:-1], self.offsets[1:]):
-            m._buffers["weight"] = W[lo:hi]
+        self._views = [W[lo:hi] for lo, hi in zip(self.offsets[:-1], self.offsets[1:])]
+        for m, view in zip(self.members, self._views):
+            m._buffers["weight"] = view
         self.weight = W
         blank = lambda rows, cols, like: torch.zeros(rows, cols, dtype=like.dtype, device=dev)
         f0 = forms[0]
@@ -202,8 +203,8 @@ class FusedADEGroup:
             m._group = (self, i)
 
     def _fill(self):
-        """The members' stored forms into the group's, and what there is to tell when they change: the forms and the sum of their tensors'
-        versions, which only grow."""
+        """The members' stored forms into the group's, and what there is to tell when they change: the tensors themselves and the sum of
+        their versions, which only grow."""
         p4, k0 = self.p4, 0
         forms = [m._stored_form() for m in self.members]
         for f, lo, hi in zip(forms, self.offsets[:-1], self.offsets[1:]):
@@ -214,8 +215,8 @@ class FusedADEGroup:
             for k, per in (("vt", 1), ("vs", GROUP), ("vz", GROUP)):
                 p4[k][k0 // per:k1 // per].copy_(f[k])
             k0 = k1
-        self._forms = forms
         self._copied = [f[k] for f in forms for k in STORED_KEYS]
+        self._watch = [(m._buffers, view, f["uq"]) for m, view, f in zip(self.members, self._views, forms)]
         self._versions = None if any(t.is_inference() for t in (*self._copied, p4["uq"])) else sum(t._version for t in self._copied)
 
     def refresh(self) -> bool:
@@ -223,11 +224,16 @@ class FusedADEGroup:
         over; a group whose members have moved, keep their weight elsewhere or cannot be watched (inference tensors) dissolves."""
         if self.weight is None:
             return False
-        w, row = self.weight, self.weight.shape[1] * self.weight.element_size()
-        if self._versions is None or any(m._tensor("weight").data_ptr() != w.data_ptr() + lo * row for m, lo in zip(self.members, self.offsets)):
+        same = True
+        for buffers, view, uq in self._watch:
+            if buffers.get("weight") is not view:
+                self.release()
+                return False
+            same &= buffers.get("p4_uq") is uq
+        if self._versions is None:
             self.release()
-        elif any(m._stored_form() is not f for m, f in zip(self.members, self._forms)) or sum(t._version for t in self._copied) != self._versions:
-            if any(f._tensor("p4_uq").device != w.device for f in self.members):
+        elif not same or sum([t._version for t in self._copied]) != self._versions:
+            if any(m._tensor("p4_uq").device != self.weight.device for m in self.members):
                 self.release()
             else:
                 self._fill()
@@ -238,7 +244,7 @@ class FusedADEGroup:
         for m in self.members:
             if m._group is not None and m._group[0] is self:
                 m._group = None
-        self.weight = self.p4 = self._x = self._y = self._forms = self._copied = None
+        self.weight = self.p4 = self._x = self._y = self._views = self._copied = self._watch = None
 
     def apply(self, index: int, x, x2):
         """Output of member `index` for the input x (x2 = x as a contiguous (T, d_i) bfloat16 matrix), or None when
