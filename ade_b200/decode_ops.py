@@ -31,7 +31,7 @@ SILU_TYPES = ("SiLU", "SiLUActivation")
 def _launch(entry: str, dev: torch.device, *args) -> None:
     """One call of the C entry `entry` on the current stream of `dev`, the device of the tensors (which need not be the current one)."""
     with _on_device(dev):
-        _lib.check(getattr(_lib.load(), entry)(*args, torch.cuda.current_stream(dev).cuda_stream), entry)
+        _lib.check(getattr(_lib.load(), entry)(*args, torch._C._cuda_getCurrentRawStream(dev.index)), entry)
 
 
 def _plain_inference(*tensors) -> bool:

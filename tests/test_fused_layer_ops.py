@@ -133,7 +133,7 @@ def test_launches_go_to_the_device_of_the_tensors(monkeypatch):
 
     monkeypatch.setattr(decode_ops, "_on_device", on_device)
     monkeypatch.setattr(decode_ops._lib, "load", Lib)
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: types.SimpleNamespace(cuda_stream=("stream of", d)))
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: ("stream of", index), raising=False)
     x = torch.zeros(2, 4, 8, dtype=torch.bfloat16)
     cache = types.SimpleNamespace(keys=torch.zeros(2, 1, 16, 8), values=torch.zeros(2, 1, 16, 8), cumulative_length=torch.zeros(1, dtype=torch.int64))
     decode_ops.rmsnorm(x, x[0, 0], 1e-6)
@@ -142,7 +142,7 @@ def test_launches_go_to_the_device_of_the_tensors(monkeypatch):
     decode_ops.rope(x.unsqueeze(1), x.unsqueeze(1), x[:1], x[:1])
     decode_ops.attn_decode(x[:, :1], x[:, :1], x[:, :1], x[:1, :1], x[:1, :1], None, cache, 1.0)
     assert [s[0] for s in seen] == [f"ade_b200_{n}" for n in ("rmsnorm", "add_rmsnorm", "silu_mul", "rope", "attn_decode")]
-    assert all(s[1] == [x.device] and s[2] == ("stream of", x.device) for s in seen)
+    assert all(s[1] == [x.device] and s[2] == ("stream of", x.device.index) for s in seen)
 
 
 @pytest.mark.parametrize("name", ["post_attention_layernorm", "mlp.act_fn", "input_layernorm", "mlp"])
