@@ -478,21 +478,24 @@ int ade_b200_factored(const ade_delta_t* d, const void* x, const void* y_dense, 
 // Which of the two kernels is faster, per call in a graph over rotated weights (with y_dense: the library GEMM of the base term in front),
 // warp-MMA / tensor-core in us.  The warp-MMA kernel is priced by its steps: row blocks of 32 per SM, token tiles of 8 doubled at 17,
 // 33 and 65, and what shared memory has room for; the tensor-core kernel by the hand-overs of h and 64 ranks of U^ h at a time.
-int ade_b200_linear_faster(int T, int M, int N, int r, int with_base) {
+int ade_b200_linear_faster(int T, int M, int N, int r, int base_blocks) {
     const DeviceInfo* di = nullptr;
     if (T < 1 || T > ADE_B200_MAX_TOKENS || M < 1 || N < 1 || r < ADE_B200_GROUP || device_info(&di)) return 0;
     const int rows = (M + di->sms - 1) / di->sms, rows_cap = (rows + 1 + 31) / 32 * 32;
     if (rows > ade::LT_MAX_SEG * ade::LT_TILE) return 0;
-    if (with_base) {
-        // From 9 tokens the warp-MMA kernel no longer hides U^ h under its stream (22016 x 4096 r = 512 T = 8 36.9 / 48.3, T = 12 44.2 / 40.6);
-        // it shows where the stream is long: 12288 x 4096 (q/k/v) T = 16 41.7 / 42.7.  The tensor-core kernel hides U^ h only while there
-        // are about six columns per rank: 22016 x 4096 r = 768 T = 12 45.3 / 43.1 but 18944 rows 37.4 / 39.6; 22016 x 1024 r = 512 24.3 / 25.1.
-        // (Up to rank 256 there is too little of it to matter: 22016 x 1024 24.1 / 20.5.)
+    if (base_blocks > 0) {
+        // From 9 tokens the warp-MMA kernel no longer hides U^ h under its stream (gate/up, two blocks: 22016 x 4096 r = 512 T = 8 36.9 / 48.3,
+        // T = 12 44.2 / 40.6); it shows where the stream is long: 12288 x 4096 (q/k/v) T = 16 41.7 / 42.7.  The tensor-core kernel hides U^ h
+        // only while there are about twelve columns for each rank of a row (r / blocks): 22016 x 4096 r = 768 T = 12 45.3 / 43.1 but 18944 rows
+        // 37.4 / 39.6; 22016 x 1024 r = 512 24.3 / 25.1; dense 18943 x 4096 r = 512 T = 12 36.9 / 38.3, r = 256 35.7 / 34.6.  (Up to 128 ranks there is
+        // too little of it to matter: 22016 x 1024 r = 256 24.1 / 20.5.)
         if (T <= 8 || T > 16 || M < 16384) return 0;
-        if (r <= 256 || 6ll * r <= N) return 1;
+        const int row_rank = r / base_blocks;
+        if (row_rank <= 128 || 12ll * row_rank <= N) return 1;
         // Where h leaves the warp-MMA kernel's FIFO two stages it loses a quarter at once: 22016 x 4096 r = 1024 T = 15 47.8 / 46.4, T = 16
-        // 60.8 / 46.6.  Not worth it with two columns per rank and less: 22016 x 4096 r = 2048 T = 12 65.0 / 65.8, x 3072 54.0 / 62.4.
-        return N > 2 * r && fifo_stages(2, ade::factored_smem_bytes(2, rows_cap, T, r), M, N, di->sms) == 2;
+        // 60.8 / 46.6.  Not worth it with four columns for each rank of a row and less: 22016 x 4096 r = 2048 T = 12 65.0 / 65.8, x 3072
+        // 54.0 / 62.4; dense 22015 x 5120 r = 2048 85.8 / 103.
+        return N > 4 * row_rank && fifo_stages(2, ade::factored_smem_bytes(2, rows_cap, T, r), M, N, di->sms) == 2;
     }
     // Up to 32 tokens the warp-MMA kernel is ahead (4096 x 4096 r = 512 T = 32 23.4 / 27.4, 13824 x 4096 42.0 / 43.8; at the next token 26.5 / 29.3
     // and 41.9 / 37.4), up to 64 with little of U^ h (8192 x 1024 r = 256 T = 48 23.2 / 23.6, r = 512 27.1 / 26.2).
@@ -506,7 +509,10 @@ int ade_b200_linear_faster(int T, int M, int N, int r, int with_base) {
     // 4096 rows, r = 1024 T = 40: x 6144 38.7 / 40.3, x 11008 53.1 / 51.3; r = 1280 x 4096 37.7 / 40.3, x 6144 45.6 / 44.4.
     if (T <= 64) return N >= 8192 || (N >= 6144 && r >= 1280);
     // T = 72: x 1536 r = 768 36.2 / 35.1, r = 1024 38.9 / 40.6; r = 1024 x 4096 47.3 / 47.0.  T = 80: x 1024 r = 256 24.0 / 23.6, r = 512 27.4 / 29.1.
-    return r <= 256 || (N >= 1152 && r <= 768) || N >= 4096;
+    // With little of either the two are close, and behind a long GEMM the warp-MMA kernel's start is the lighter one: r = 256 T = 101
+    // 4727 x 10496 187.2 / 191.0 (a GEMM of odd rows), 2047 x 10496 0.97 of it, 4096 x 8192 T = 112 1.01.
+    if (r <= 256) return N < 8192 || M <= 2048;
+    return (N >= 1152 && r <= 768) || N >= 4096;
 }
 
 int ade_b200_linear_preferred(int T, int M, int r) { return ade_b200_linear_faster(T, M, 13824, r, 0); }

@@ -314,8 +314,10 @@ def module_forward(x: torch.Tensor, p4: dict, weight: torch.Tensor) -> torch.Ten
     T = x.shape[0]
     if T > FUSED_MAX_TOKENS:
         return decode_forward_packed(x, torch.nn.functional.linear(x, weight), p4)
-    if T > TALL_FACTORED_MAX_TOKENS and weight.shape[0] >= TALL_ROWS and _lib.load().ade_b200_linear_faster(T, *weight.shape, int(p4["r"]), 1):
-        return linear_forward(x, p4, weight)
+    if T > TALL_FACTORED_MAX_TOKENS and weight.shape[0] >= TALL_ROWS:
+        blocks = max(1, len(p4.get("blocks") or ()) - 1)
+        if _lib.load().ade_b200_linear_faster(T, *weight.shape, int(p4["r"]), blocks):
+            return linear_forward(x, p4, weight)
     return factored_forward(x, p4, weight=weight)
 
 

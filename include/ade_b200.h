@@ -180,9 +180,9 @@ int ade_b200_factored(const ade_delta_t* d, const void* x, const void* y_dense, 
  * d->M up to 384 rows per SM of the device (56832 on 148 SMs).  The launch is cooperative, one CTA per SM.
  */
 size_t ade_b200_linear_workspace_bytes(int T, int M, int r);
-/* 1 where ade_b200_linear is the faster of the two kernels, else 0: with_base == 0 for calls with y_dense (what the torch binding
- * and ade_b200_factored_static go by), != 0 for calls with w_b. */
-int ade_b200_linear_faster(int T, int M, int N, int r, int with_base);
+/* 1 where ade_b200_linear is the faster of the two kernels, else 0.  base_blocks == 0: calls with y_dense (what the torch binding and
+ * ade_b200_factored_static go by); n > 0: calls with w_b whose U^ has n diagonal blocks (1 = dense). */
+int ade_b200_linear_faster(int T, int M, int N, int r, int base_blocks);
 /* The same for calls with y_dense where N is not known: 1 where ade_b200_linear is the faster one at the longest rows in use. */
 int ade_b200_linear_preferred(int T, int M, int r);
 int ade_b200_linear(const ade_delta_t* d, const void* x, const void* y_dense, const void* w_b, void* out, void* scratch, size_t scratch_bytes,

@@ -141,7 +141,7 @@ def _direct(entry, x, p4, y=None, W=None):
 @pytest.mark.parametrize("M,N,r,T,linear", [(31250, 128, 128, 32, 0), (31250, 128, 128, 33, 1), (31249, 128, 128, 33, 0), (31249, 128, 128, 65, 1),
                                             (4736, 384, 384, 65, 0), (4737, 384, 384, 65, 1), (4736, 128, 256, 128, 1), (600, 384, 1024, 87, 0),
                                             (600, 384, 1024, 90, 1), (500, 1152, 768, 80, 1), (500, 1024, 768, 80, 0), (500, 1152, 896, 80, 0),
-                                            (300, 4096, 896, 66, 1), (4000, 8192, 1024, 40, 1), (4000, 8064, 1024, 40, 0), (3200, 6144, 1280, 34, 1)])
+                                            (300, 4096, 896, 66, 1), (2048, 8192, 128, 65, 1), (2049, 8192, 128, 65, 0), (4000, 8192, 1024, 40, 1), (4000, 8064, 1024, 40, 0), (3200, 6144, 1280, 34, 1)])
 def test_supplied_base_term_takes_the_kernel_of_the_rule(M, N, r, T, linear):
     assert _lib.load().ade_b200_linear_faster(T, M, N, r, 0) == linear
     p4 = kernels.pack_int4(synth.random_packed(M, N, r, M + T, DEV, on_device=True))
@@ -152,13 +152,18 @@ def test_supplied_base_term_takes_the_kernel_of_the_rule(M, N, r, T, linear):
     assert err <= 1e-2 and cos >= 0.9999, (err, cos)
 
 
-# the rule for calls with the base weight: rows, tokens, rank against columns, and where h takes the third FIFO stage (with two columns per rank)
-@pytest.mark.parametrize("M,N,r,T,linear", [(16383, 128, 128, 9, 0), (16384, 128, 256, 8, 0), (16384, 128, 256, 9, 1), (16384, 128, 384, 9, 0),
-                                            (16384, 2304, 384, 16, 1), (16384, 2176, 384, 16, 0), (22016, 2176, 1024, 15, 0), (22016, 2176, 1024, 16, 1),
-                                            (22016, 2048, 1024, 16, 0)])
-def test_module_takes_the_kernel_of_the_rule(M, N, r, T, linear):
-    assert (_lib.load().ade_b200_linear_faster(T, M, N, r, 1) == 1) == bool(linear)
+# the rule for calls with the base weight, one block and two: rows, tokens, ranks of a row against columns, and where h takes the third FIFO
+# stage (with four columns for each rank of a row)
+@pytest.mark.parametrize("M,N,r,T,blocks,linear", [(16383, 128, 128, 9, 1, 0), (16384, 128, 128, 8, 1, 0), (16384, 128, 128, 9, 1, 1), (16384, 128, 256, 9, 2, 1),
+                                                   (16384, 128, 256, 9, 1, 0), (16384, 3072, 256, 16, 1, 1), (16384, 2944, 256, 16, 1, 0),
+                                                   (16384, 3072, 512, 16, 2, 1), (22016, 2176, 1024, 15, 2, 0), (22016, 2176, 1024, 16, 2, 1),
+                                                   (22016, 2176, 1024, 16, 1, 0), (22016, 2048, 1024, 16, 2, 0)])
+def test_module_takes_the_kernel_of_the_rule(M, N, r, T, blocks, linear):
+    assert _lib.load().ade_b200_linear_faster(T, M, N, r, blocks) == linear
     p4 = kernels.pack_int4(synth.random_packed(M, N, r, M + T, DEV, on_device=True))
+    if blocks == 2:
+        p4["blocks"] = [(0, 0), (M // 2, r // 256), (M, r // 128)]
+        p4["us"][:M // 2, r // 256:], p4["us"][M // 2:, :r // 256] = 0, 0
     x, W = synth.activations(T, N, 1).to(DEV), synth.base_weight(M, N, 2).to(DEV)
     by = {e: _direct(e, x, p4, W=W) for e in ("factored", "linear")}
     assert torch.equal(kernels.module_forward(x, p4, W), by["linear" if linear else "factored"])
