@@ -441,6 +441,9 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
         if (lane == 0) bulk_wait_group_read<0>();    // shared memory may go once the last store has read it
     } else if (!EXP && warp < MMA_WARP) {
         // ------------------------------------------------------------------ unpack
+        // A raw slot is handed back behind the stores of what was read from it: they need the loaded registers, so the reads are over, and
+        // the proxy fence stands between them and the copy that refills the slot.  Handed back right behind the loads, the refill could
+        // overtake a load still in flight (one tile column in some 10^6 items had the codes of the slot's next item).
         const int pt = threadIdx.x - RS_EPI_WARPS * 32;
         const int c = pt & 3, rbase = pt >> 2;
         uint32_t ri = 0, bi = 0, sk = 0;
@@ -472,14 +475,15 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                     uint4 qa[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) qa[i] = lds16(rs + (rbase + 32 * i) * 64 + c * 16);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(C::BAR_RAW_EMPTY + slot));
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         unpack_store_s(a_res + g * RS_OPER_BYTES, rbase + 32 * i, c, qa[i], static_cast<uint32_t>(za_pack[i] >> (8 * g)) & 0xFFu);
                     fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(C::BAR_A_FULL + g));
+                    if (lane == 0) {
+                        mbar_arrive(bar(C::BAR_A_FULL + g));
+                        mbar_arrive(bar(C::BAR_RAW_EMPTY + slot));
+                    }
                 }
                 ++sk;
             }
@@ -494,15 +498,16 @@ __global__ void __launch_bounds__(EXP ? RS_THREADS_EXP : RS_THREADS, 1) recon_st
                     qb[i] = lds16(rs + (rbase + 32 * i) * 64 + c * 16);
                     zb[i] = lds1(rs + RS_RAW_CODES + rbase + 32 * i);
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(C::BAR_RAW_EMPTY + slot));
                 const uint32_t s = bi % C::B_STAGES, bph = (bi / C::B_STAGES) & 1;
                 wait_bounded(bar(C::BAR_B_EMPTY + s), bph ^ 1, wctx, 2);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) unpack_store_s(b_st + s * RS_OPER_BYTES, rbase + 32 * i, c, qb[i], zb[i]);
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar(C::BAR_B_FULL + s));
+                if (lane == 0) {
+                    mbar_arrive(bar(C::BAR_B_FULL + s));
+                    mbar_arrive(bar(C::BAR_RAW_EMPTY + slot));
+                }
             }
         }
     } else {
